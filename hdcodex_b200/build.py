@@ -24,6 +24,13 @@ INCLUDE = os.path.join(ROOT, "include")
 SOURCES = [
     "bvh_build.cu",
     "integrator.cu",
+    "shade_plain_groups.cu",
+    "shade_plain_singles.cu",
+    "shade_full_groups.cu",
+    "shade_full_singles_lit.cu",
+    "shade_full_singles_unlit.cu",
+    "shade_full_replays_lit.cu",
+    "shade_full_replays_unlit.cu",
     "nrc.cu",
     "render_static.cu",
     "scene_pack.cpp",

@@ -99,6 +99,7 @@ struct TexDesc {
     const float4* mips;
     uint32_t levels;
     uint32_t pad;
+    const float* bytes;  // 8-bit formats: 256 linear values of the sRGB bytes, then the 256 values n / 255
 };
 
 // 8-wide BVH node with quantised child boxes (80 bytes). The layout is the
@@ -258,6 +259,7 @@ HDCX_D float glog(float x) { return hdcx_fp_log(x); }
 HDCX_D float gpow(float x, float y) { return hdcx_fp_pow(x, y); }
 HDCX_D float gsin(float x) { return hdcx_fp_sin(x); }
 HDCX_D float gcos(float x) { return hdcx_fp_cos(x); }
+HDCX_D void gsincos(float x, float& sine, float& cosine) { hdcx_fp_sincos(x, &sine, &cosine); }
 HDCX_D float gacos(float x) { return hdcx_fp_acos(x); }
 HDCX_D float gatan2(float y, float x) { return hdcx_fp_atan2(y, x); }
 

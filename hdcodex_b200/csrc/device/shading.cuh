@@ -1,27 +1,30 @@
 // shading.cuh - device restatement of the reference integrator's shading
 // functions (src/gpu/vulkan_path_tracer.cpp:115-1186), one function per GLSL
 // function with the GLSL names. Lane-replicated vec3 values are scalars here
-// (see common.cuh); vectors that really vary per component (directions, RGB
-// inputs before spectral conversion) stay float3.
+// (see common.cuh), or Lanes3 where one thread shades the lanes of a sample
+// together (lanes.cuh; the type V of the templates here); vectors that really
+// vary per component (directions, RGB inputs before spectral conversion) stay
+// float3.
 #pragma once
 
 #include "common.cuh"
+#include "lanes.cuh"
 
 namespace hdcx {
-
-__constant__ float cSrgbToLinear[256];
 
 // ---------------------------------------------------------------------------
 // Per-lane spectral constants. reconstructRgb's Gaussian basis and the Planck
 // factor of illuminantSpectrum depend only on the wavelength, so each path
 // computes them once (the same binary32 values the GLSL recomputes per call).
 // ---------------------------------------------------------------------------
-struct Spectrum {
-    float wavelength;
-    float br, bg, bb;   // basis (vulkan_path_tracer.cpp:120-123)
-    float denominator;  // max(dot(vec3(1), basis), 1e-5)
-    float planck;       // illuminantSpectrum's Planck ratio (:137-142)
+template <class V>
+struct SpectrumOf {
+    V wavelength;
+    V br, bg, bb;   // basis (vulkan_path_tracer.cpp:120-123)
+    V denominator;  // max(dot(vec3(1), basis), 1e-5)
+    V planck;       // illuminantSpectrum's Planck ratio (:137-142)
 };
+using Spectrum = SpectrumOf<float>;
 
 HDCX_D Spectrum makeSpectrum(float wavelength)
 {
@@ -52,19 +55,30 @@ HDCX_D Spectrum spectrumFromBasis(float wavelength, float4 packed)
     return s;
 }
 
-HDCX_D float reconstructRgb(float3 rgb, const Spectrum& s)
+template <class V>
+HDCX_D V reconstructRgb(float3 rgb, const SpectrumOf<V>& s)
 {
     // :118-126
-    const float num = gmax(rgb.x, 0.0f) * s.br + gmax(rgb.y, 0.0f) * s.bg + gmax(rgb.z, 0.0f) * s.bb;
+    const V num = V(gmax(rgb.x, 0.0f)) * s.br + V(gmax(rgb.y, 0.0f)) * s.bg + V(gmax(rgb.z, 0.0f)) * s.bb;
     return num / s.denominator;
 }
-HDCX_D float reflectanceSpectrum(float3 rgb, const Spectrum& s)
+// reconstructRgb of a colour that is often white: there the sum equals the
+// denominator and the quotient is one.
+template <class V>
+HDCX_D V reconstructLikelyWhite(float3 rgb, const SpectrumOf<V>& s)
+{
+    const V num = V(gmax(rgb.x, 0.0f)) * s.br + V(gmax(rgb.y, 0.0f)) * s.bg + V(gmax(rgb.z, 0.0f)) * s.bb;
+    return ratioLikelyOne(num, s.denominator);
+}
+template <class V>
+HDCX_D V reflectanceSpectrum(float3 rgb, const SpectrumOf<V>& s)
 {
     return clampf(reconstructRgb(rgb, s), 0.0f, 1.0f);
 }
-HDCX_D float illuminantSpectrum(float3 rgb, const Spectrum& s)
+template <class V>
+HDCX_D V illuminantSpectrum(float3 rgb, const SpectrumOf<V>& s)
 {
-    return gmax(reconstructRgb(rgb, s) * s.planck, 0.0f);
+    return gmax(reconstructRgb(rgb, s) * s.planck, V(0.0f));
 }
 
 HDCX_D float3 cieXyz(float wavelength)
@@ -102,10 +116,9 @@ HDCX_D float4 texelFetch(const TexDesc& t, int x, int y)
     if (t.format == 2u) return __ldg(reinterpret_cast<const float4*>(t.texels) + i);
     const uint32_t p = __ldg(reinterpret_cast<const uint32_t*>(t.texels) + i);
     const uint32_t r = p & 0xffu, g = (p >> 8) & 0xffu, b = (p >> 16) & 0xffu, a = p >> 24;
-    if (t.format == 1u) {
-        return make_float4(cSrgbToLinear[r], cSrgbToLinear[g], cSrgbToLinear[b], u2f(a) / 255.0f);
-    }
-    return make_float4(u2f(r) / 255.0f, u2f(g) / 255.0f, u2f(b) / 255.0f, u2f(a) / 255.0f);
+    // Tables of the 256 values (TexDesc::bytes): linear from sRGB, then n / 255.
+    const float* color = t.bytes + (t.format == 1u ? 0 : 256);
+    return make_float4(__ldg(color + r), __ldg(color + g), __ldg(color + b), __ldg(t.bytes + 256 + a));
 }
 
 HDCX_D int wrapIndex(int i, int n)
@@ -120,8 +133,10 @@ HDCX_D float texelCoordinate(float uv, uint32_t size)
     return fabsf(x) < 16777216.0f ? x : 0.0f;
 }
 
-HDCX_D float4 sampleBilinear(const TexDesc& t, float2 uv)
+// Not inlined: every texture lookup of a kernel shares the copy.
+HDCX_NOINLINE float4 sampleBilinear(const TexDesc* desc, float2 uv)
 {
+    const TexDesc t = *desc;
     const float x = texelCoordinate(uv.x, t.width);
     const float y = texelCoordinate(uv.y, t.height);
     const float fx = floorf(x), fy = floorf(y);
@@ -144,8 +159,7 @@ HDCX_D float4 sampleBilinear(const TexDesc& t, float2 uv)
 HDCX_D float4 textureSample(const DeviceScene& s, uint32_t index, float2 uv)
 {
     if (index >= s.textureCount) return make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    const TexDesc t = s.textures[index];
-    return sampleBilinear(t, uv);
+    return sampleBilinear(s.textures + index, uv);
 }
 
 // Texture LOD (not in the reference, whose sampler has one mip level): the
@@ -178,25 +192,26 @@ HDCX_D float4 sampleMipBilinear(const TexDesc& t, uint32_t level, float2 uv)
 // cones: lodBase holds the hit's texture-independent terms), trilinear
 // between the two nearest levels; lodBase = -inf samples level 0 exactly as
 // textureSample does.
-HDCX_D float4 textureSampleLod(const DeviceScene& s, uint32_t index, float2 uv, float lodBase)
+HDCX_D float4 textureSampleLod(const TexDesc* textures, uint32_t index, float2 uv, float lodBase)
 {
-    if (index >= s.textureCount) return make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    const TexDesc t = s.textures[index];
-    if (!(lodBase > -1e30f) || t.levels <= 1u || t.mips == nullptr) return sampleBilinear(t, uv);
+    const TexDesc t = textures[index];
+    if (!(lodBase > -1e30f) || t.levels <= 1u || t.mips == nullptr) return sampleBilinear(textures + index, uv);
     const float lod = fminf(fmaxf(lodBase + 0.5f * log2f(u2f(t.width) * u2f(t.height)), 0.0f), u2f(t.levels - 1u));
     const uint32_t l0 = static_cast<uint32_t>(lod);
     const float f = lod - u2f(l0);
-    const float4 a = l0 == 0u ? sampleBilinear(t, uv) : sampleMipBilinear(t, l0, uv);
+    const float4 a = l0 == 0u ? sampleBilinear(textures + index, uv) : sampleMipBilinear(t, l0, uv);
     if (f <= 0.0f || l0 + 1u >= t.levels) return a;
     const float4 b = sampleMipBilinear(t, l0 + 1u, uv);
     return make_float4(a.x + (b.x - a.x) * f, a.y + (b.y - a.y) * f, a.z + (b.z - a.z) * f, a.w + (b.w - a.w) * f);
 }
 
-HDCX_D float4 sampleMaterialTexture(const DeviceScene& s, uint32_t textureIndex, float2 uv, float4 fallbackValue,
-                                    float lodBase = -INFINITY)
+// A bound material texture. Not inlined: the full shade kernels look up some
+// twenty slots, and one shared copy of the UDIM, filter and mip code keeps
+// their instruction footprint within the instruction caches. The arguments
+// are scalars, so that the scene record stays in constant memory.
+HDCX_NOINLINE float4 sampleBoundTexture(const TexDesc* textures, uint32_t textureCount, uint32_t textureIndex, float2 uv,
+                                        float4 fallbackValue, float lodBase)
 {
-    // :760-775
-    if (textureIndex == kMissingTexture) return fallbackValue;
     if ((textureIndex & 0x80000000u) != 0u) {
         const float fu = floorf(uv.x), fv = floorf(uv.y);
         if (!(fabsf(fu) < 1e6f) || !(fabsf(fv) < 1e6f)) return fallbackValue;
@@ -205,12 +220,19 @@ HDCX_D float4 sampleMaterialTexture(const DeviceScene& s, uint32_t textureIndex,
         const uint32_t presentTiles = (textureIndex >> 8u) & 0x7fffffu;
         const uint32_t tileBit = 1u << static_cast<uint32_t>(tileOffset);
         if ((presentTiles & tileBit) == 0u) return fallbackValue;
-        const uint32_t descriptorIndex = (textureIndex & 0xffu) + static_cast<uint32_t>(__popc(presentTiles & (tileBit - 1u)));
-        if (descriptorIndex >= s.textureCount) return fallbackValue;
-        return textureSampleLod(s, descriptorIndex, make_float2(fract(uv.x), fract(uv.y)), lodBase);
+        textureIndex = (textureIndex & 0xffu) + static_cast<uint32_t>(__popc(presentTiles & (tileBit - 1u)));
+        uv = make_float2(fract(uv.x), fract(uv.y));
     }
-    if (textureIndex >= s.textureCount) return fallbackValue;
-    return textureSampleLod(s, textureIndex, uv, lodBase);
+    if (textureIndex >= textureCount) return fallbackValue;
+    return textureSampleLod(textures, textureIndex, uv, lodBase);
+}
+
+HDCX_D float4 sampleMaterialTexture(const DeviceScene& s, uint32_t textureIndex, float2 uv, float4 fallbackValue,
+                                    float lodBase = -INFINITY)
+{
+    // :760-775
+    if (textureIndex == kMissingTexture) return fallbackValue;
+    return sampleBoundTexture(s.textures, s.textureCount, textureIndex, uv, fallbackValue, lodBase);
 }
 
 HDCX_D float4 f4(float v) { return make_float4(v, v, v, v); }
@@ -263,13 +285,16 @@ HDCX_D float3 cosineHemisphere(float3 normal, uint32_t& state)
     const float r2s = sqrtf(r2);
     const float3 tangent = tangentFrameAxis(normal);
     const float3 bitangent = cross(normal, tangent);
-    return normalize(tangent * gcos(r1) * r2s + bitangent * gsin(r1) * r2s + normal * sqrtf(1.0f - r2));
+    float sine, cosine;
+    gsincos(r1, sine, cosine);
+    return normalize(tangent * cosine * r2s + bitangent * sine * r2s + normal * sqrtf(1.0f - r2));
 }
 
-HDCX_D float fresnelSchlick(float cosTheta, float f0)
+template <class V>
+HDCX_D V fresnelSchlick(float cosTheta, V f0)
 {
     // :202-205
-    return f0 + (1.0f - f0) * gpow5(1.0f - clampf(cosTheta, 0.0f, 1.0f));
+    return f0 + (V(1.0f) - f0) * V(gpow5(1.0f - clampf(cosTheta, 0.0f, 1.0f)));
 }
 
 HDCX_D float3 orthogonalTangent(float3 normal, float3 tangent)
@@ -287,93 +312,130 @@ HDCX_D float2 clampRoughness(float2 roughness)
     return make_float2(clampf(roughness.x * roughness.x, 0.001f, 1.0f), clampf(roughness.y * roughness.y, 0.001f, 1.0f));
 }
 
-HDCX_D float distributionGGXAnisotropic(float3 halfway, float3 normal, float3 tangent, float2 roughness)
+// What the lobes of a shading point share for every light and sampled
+// direction: the anisotropy axes (orthogonalTangent and its cross product,
+// which the reference's functions each derive again), squared roughness and
+// the view direction's masking.
+struct ShadingFrame {
+    float3 normal, axisX, axisY, view;
+    float nDotV;        // max(dot(normal, view), 0)
+    float2 alpha, coatAlpha;
+    float maskView, maskViewCoat;
+    bool coated;        // the coat lobe's pdf is needed
+};
+
+// What the lobes need of one direction, computed once for evaluation, pdf and
+// sample weight alike.
+struct LobeTerms {
+    float signedNdotL, nDotL;
+    float cosine;        // nDotL / pi
+    float vDotH, nDotH;  // of the half vector; the normal takes its place where nDotL <= 0
+    float d, dCoat;      // GGX distributions (zero where the view or the direction is below the surface)
+};
+
+HDCX_D float distributionGGXAnisotropic(float3 halfway, const ShadingFrame& f, float2 alpha)
 {
     // :287-300
-    const float3 axisX = orthogonalTangent(normal, tangent);
-    const float3 axisY = cross(normal, axisX);
-    const float2 alpha = clampRoughness(roughness);
-    const float lx = dot(halfway, axisX), ly = dot(halfway, axisY), lz = gmax(dot(halfway, normal), 0.0f);
+    const float lx = dot(halfway, f.axisX), ly = dot(halfway, f.axisY), lz = gmax(dot(halfway, f.normal), 0.0f);
     const float denominator = lx * lx / (alpha.x * alpha.x) + ly * ly / (alpha.y * alpha.y) + lz * lz;
     return 1.0f / gmax(kPi * alpha.x * alpha.y * denominator * denominator, 1e-6f);
 }
 
-HDCX_D float geometryGGXAnisotropic(float3 direction, float3 normal, float3 tangent, float2 roughness)
+HDCX_D float geometryGGXAnisotropic(float3 direction, float nDotDirection, const ShadingFrame& f, float2 alpha)
 {
-    // :302-315
-    const float nDotDirection = gmax(dot(normal, direction), 0.0f);
+    // :302-315, nDotDirection = max(dot(normal, direction), 0)
     if (nDotDirection <= 0.0f) return 0.0f;
-    const float3 axisX = orthogonalTangent(normal, tangent);
-    const float3 axisY = cross(normal, axisX);
-    const float2 alpha = clampRoughness(roughness);
-    const float projected = gpow2(alpha.x * dot(direction, axisX)) + gpow2(alpha.y * dot(direction, axisY));
+    const float projected = gpow2(alpha.x * dot(direction, f.axisX)) + gpow2(alpha.y * dot(direction, f.axisY));
     const float lambda = (-1.0f + sqrtf(1.0f + projected / gmax(nDotDirection * nDotDirection, 1e-8f))) * 0.5f;
     return 1.0f / (1.0f + lambda);
 }
 
-HDCX_D float evaluateGGXAnisotropic(float3 normal, float3 tangent, float3 viewDirection, float3 lightDirection,
-                                    float2 roughness, float f0)
+template <bool kFull>
+HDCX_D ShadingFrame shadingFrame(float3 normal, float3 tangent, float3 view, float nDotV, float2 roughness, float2 coatRoughness,
+                                 float coat)
 {
-    // :317-332
-    const float3 halfway = normalize(viewDirection + lightDirection);
-    const float nDotV = gmax(dot(normal, viewDirection), 0.0f);
-    const float nDotL = gmax(dot(normal, lightDirection), 0.0f);
-    const float vDotH = gmax(dot(viewDirection, halfway), 0.0f);
-    if (nDotV <= 0.0f || nDotL <= 0.0f || vDotH <= 0.0f) return 0.0f;
-    const float distribution = distributionGGXAnisotropic(halfway, normal, tangent, roughness);
-    const float geometry = geometryGGXAnisotropic(viewDirection, normal, tangent, roughness) *
-                           geometryGGXAnisotropic(lightDirection, normal, tangent, roughness);
-    return distribution * geometry * fresnelSchlick(vDotH, f0) / gmax(4.0f * nDotV * nDotL, 1e-5f);
+    ShadingFrame f;
+    f.normal = normal;
+    f.view = view;
+    f.nDotV = nDotV;
+    f.axisX = orthogonalTangent(normal, tangent);
+    f.axisY = cross(normal, f.axisX);
+    f.alpha = clampRoughness(roughness);
+    f.maskView = geometryGGXAnisotropic(view, nDotV, f, f.alpha);
+    // Without a coat its pdf is multiplied by zero; a NaN roughness keeps it.
+    f.coated = kFull && (coat > 0.0f || !(coatRoughness.x == coatRoughness.x) || !(coatRoughness.y == coatRoughness.y));
+    f.coatAlpha = kFull ? clampRoughness(coatRoughness) : make_float2(1.0f, 1.0f);
+    f.maskViewCoat = kFull && coat > 0.0f ? geometryGGXAnisotropic(view, nDotV, f, f.coatAlpha) : 0.0f;
+    return f;
 }
 
-HDCX_D float3 sampleGGXReflectionAnisotropic(float3 incident, float3 normal, float3 tangent, float2 roughness,
-                                             uint32_t& state)
+HDCX_D LobeTerms lobeTerms(const ShadingFrame& f, float3 direction)
+{
+    LobeTerms t;
+    t.signedNdotL = dot(f.normal, direction);
+    t.nDotL = gmax(t.signedNdotL, 0.0f);
+    t.cosine = t.nDotL / kPi;
+    const float3 halfway = t.nDotL > 0.0f ? normalize(f.view + direction) : f.normal;
+    t.vDotH = gmax(dot(f.view, halfway), 0.0f);
+    t.nDotH = gmax(dot(f.normal, halfway), 0.0f);
+    t.d = 0.0f;
+    t.dCoat = 0.0f;
+    if (!(f.nDotV <= 0.0f) && !(t.nDotL <= 0.0f)) {
+        t.d = distributionGGXAnisotropic(halfway, f, f.alpha);
+        if (f.coated) t.dCoat = distributionGGXAnisotropic(halfway, f, f.coatAlpha);
+    }
+    return t;
+}
+
+template <class V>
+HDCX_D V evaluateGGXAnisotropic(const ShadingFrame& f, const LobeTerms& t, float3 lightDirection, float2 alpha, float maskView,
+                                float distribution, V f0)
+{
+    // :317-332
+    if (f.nDotV <= 0.0f || t.nDotL <= 0.0f || t.vDotH <= 0.0f) return V(0.0f);
+    const float geometry = maskView * geometryGGXAnisotropic(lightDirection, t.nDotL, f, alpha);
+    return V(distribution * geometry) * fresnelSchlick(t.vDotH, f0) / V(gmax(4.0f * f.nDotV * t.nDotL, 1e-5f));
+}
+
+HDCX_D float3 sampleGGXReflectionAnisotropic(float3 incident, const ShadingFrame& f, float2 alpha, uint32_t& state)
 {
     // :334-350
-    const float3 axisX = orthogonalTangent(normal, tangent);
-    const float3 axisY = cross(normal, axisX);
-    const float2 alpha = clampRoughness(roughness);
     const float phi = kTwoPi * randomFloat(state);
     const float elevationSample = randomFloat(state);
     const float radius = sqrtf(elevationSample / gmax(1.0f - elevationSample, 1e-6f));
-    float3 halfway = normalize(axisX * (alpha.x * radius * gcos(phi)) + axisY * (alpha.y * radius * gsin(phi)) + normal);
+    float sine, cosine;
+    gsincos(phi, sine, cosine);
+    float3 halfway = normalize(f.axisX * (alpha.x * radius * cosine) + f.axisY * (alpha.y * radius * sine) + f.normal);
     if (dot(halfway, -incident) < 0.0f) halfway = -halfway;
-    const float3 reflected = reflect(incident, halfway);
-    return dot(reflected, normal) > 0.0f ? normalize(reflected) : normalize(reflect(incident, normal));
+    float3 reflected = reflect(incident, halfway);
+    if (!(dot(reflected, f.normal) > 0.0f)) reflected = reflect(incident, f.normal);
+    return normalize(reflected);
 }
 
-HDCX_D float ggxSampleWeightAnisotropic(float3 incident, float3 outgoing, float3 normal, float3 tangent,
-                                        float2 roughness, float f0)
+template <class V>
+HDCX_D V ggxSampleWeightAnisotropic(const ShadingFrame& f, const LobeTerms& t, float3 outgoing, float2 alpha, float maskView,
+                                    float distribution, V f0)
 {
     // :352-367
-    const float3 viewDirection = normalize(-incident);
-    const float3 halfway = normalize(viewDirection + outgoing);
-    const float nDotL = gmax(dot(normal, outgoing), 0.0f);
-    const float nDotH = gmax(dot(normal, halfway), 0.0f);
-    const float vDotH = gmax(dot(viewDirection, halfway), 0.0f);
-    if (nDotL <= 0.0f || nDotH <= 0.0f || vDotH <= 0.0f) return 0.0f;
-    const float distribution = distributionGGXAnisotropic(halfway, normal, tangent, roughness);
-    const float pdf = distribution * nDotH / gmax(4.0f * vDotH, 1e-6f);
-    return evaluateGGXAnisotropic(normal, tangent, viewDirection, outgoing, roughness, f0) * nDotL / gmax(pdf, 1e-6f);
+    if (t.nDotL <= 0.0f || t.nDotH <= 0.0f || t.vDotH <= 0.0f) return V(0.0f);
+    const float pdf = distribution * t.nDotH / gmax(4.0f * t.vDotH, 1e-6f);
+    return evaluateGGXAnisotropic(f, t, outgoing, alpha, maskView, distribution, f0) * V(t.nDotL) / V(gmax(pdf, 1e-6f));
 }
 
-HDCX_D float ggxReflectionPdfAnisotropic(float3 normal, float3 tangent, float3 viewDirection, float3 lightDirection,
-                                         float2 roughness)
+// :371-383
+HDCX_D float ggxReflectionPdfAnisotropic(const ShadingFrame& f, const LobeTerms& t, float distribution)
 {
-    // :371-383
-    if (dot(normal, viewDirection) <= 0.0f || dot(normal, lightDirection) <= 0.0f) return 0.0f;
-    const float3 halfway = normalize(viewDirection + lightDirection);
-    const float nDotH = gmax(dot(normal, halfway), 0.0f);
-    const float vDotH = gmax(dot(viewDirection, halfway), 0.0f);
-    return distributionGGXAnisotropic(halfway, normal, tangent, roughness) * nDotH / gmax(4.0f * vDotH, 1e-6f);
+    if (f.nDotV <= 0.0f || t.nDotL <= 0.0f) return 0.0f;
+    return distribution * t.nDotH / gmax(4.0f * t.vDotH, 1e-6f);
 }
 
-HDCX_D float powerHeuristic(float firstPdf, float secondPdf)
+template <class V>
+HDCX_D V powerHeuristic(V firstPdf, V secondPdf)
 {
     // :385-390
-    const float firstSquared = firstPdf * firstPdf;
-    const float secondSquared = secondPdf * secondPdf;
-    return firstSquared / gmax(firstSquared + secondSquared, 1e-12f);
+    const V firstSquared = firstPdf * firstPdf;
+    const V secondSquared = secondPdf * secondPdf;
+    return firstSquared / gmax(firstSquared + secondSquared, V(1e-12f));
 }
 
 HDCX_D float sheenDirectionalAlbedo(float nDotV, float roughness)
@@ -437,8 +499,9 @@ HDCX_D float eonDirectionalAlbedo(float nDotDirection, float roughness)
     return clampf(a + roughness * a * g / kPi, 0.0f, 1.0f);
 }
 
-HDCX_D float evaluateDiffuseReflection(float3 normal, float3 viewDirection, float3 lightDirection, float diffuseColor,
-                                       float roughness, uint32_t model)
+template <class V>
+HDCX_D V evaluateDiffuseReflection(float3 normal, float3 viewDirection, float3 lightDirection, V diffuseColor,
+                                   float roughness, uint32_t model)
 {
     // :946-1009
     const float nDotL = gmax(dot(normal, lightDirection), 0.0f);
@@ -481,88 +544,93 @@ HDCX_D float evaluateDiffuseReflection(float3 normal, float3 viewDirection, floa
         const float outgoingAlbedo = eonDirectionalAlbedo(nDotV, sigma);
         const float incidentAlbedo = eonDirectionalAlbedo(nDotL, sigma);
         const float directionalFactor = (1.0f - outgoingAlbedo) * (1.0f - incidentAlbedo) / gmax(1.0f - averageAlbedo, 1e-5f);
-        const float rho = clampf(diffuseColor, 0.0f, 0.9999f);
-        const float multipleScatterOverRho = rho * averageAlbedo / gmax(1.0f - rho * (1.0f - averageAlbedo), 1e-5f);
-        return nDotL / kPi * (singleScatter + multipleScatterOverRho * directionalFactor);
+        const V rho = clampf(diffuseColor, 0.0f, 0.9999f);
+        const V multipleScatterOverRho = rho * V(averageAlbedo) / gmax(V(1.0f) - rho * V(1.0f - averageAlbedo), V(1e-5f));
+        return V(nDotL / kPi) * (V(singleScatter) + multipleScatterOverRho * V(directionalFactor));
     }
     return nDotL / kPi;
 }
 
-// Material parameters of one shading point, per lane (the locals of main()).
+// Material parameters of one shading point (the locals of main()).
+template <class V>
 struct SurfaceParams {
-    float diffuseColor;
+    V diffuseColor;
     float transmission, subsurface, diffuseWeight, diffuseRoughness;
     uint32_t diffuseModel;
     float translucentWeight;
-    float translucentColor;
+    V translucentColor;
     float metalness;
     float2 roughness;
-    float f0;
+    V f0;
     float coat;
     float2 coatRoughness;
-    float coatF0;
+    V coatF0;
     float sheen;
-    float sheenColor;
+    V sheenColor;
     float sheenRoughness;
     bool sheenZeltner;
 };
 
-HDCX_D float diffuseLayerSum(float diffuse, float translucent, float specular) { return diffuse + translucent + specular; }
-
-HDCX_D float evaluateDirectSurface(float3 normal, float3 tangent, float3 viewDirection, float3 lightDirection,
-                                   const SurfaceParams& p, float diffuseScale, float specularScale)
+// kFull = false: no sheen, coat, subsurface, transmission or diffuse
+// transmission and the Lambert model; their terms are exact zeros (the colours
+// they multiply are finite, which the host checks).
+template <bool kFull, class V>
+HDCX_D V evaluateDirectSurface(const ShadingFrame& f, const LobeTerms& t, float3 lightDirection, const SurfaceParams<V>& p,
+                               float diffuseScale, float specularScale)
 {
     // :1013-1069
-    const float signedNdotL = dot(normal, lightDirection);
-    const float nDotL = gmax(signedNdotL, 0.0f);
-    const float backNdotL = gmax(-signedNdotL, 0.0f);
-    const float wrappedNdotL = gmax((signedNdotL + 0.5f * p.subsurface) / (1.0f + 0.5f * p.subsurface), 0.0f);
-    if (wrappedNdotL <= 0.0f && nDotL <= 0.0f && backNdotL * p.translucentWeight <= 0.0f) return 0.0f;
-    const float3 halfway = nDotL > 0.0f ? normalize(viewDirection + lightDirection) : normal;
-    const float baseFresnel = fresnelSchlick(gmax(dot(viewDirection, halfway), 0.0f), p.f0);
-    const float diffuseResponse = mix(evaluateDiffuseReflection(normal, viewDirection, lightDirection, p.diffuseColor,
-                                                                p.diffuseRoughness, p.diffuseModel),
-                                      wrappedNdotL / kPi, p.subsurface);
-    const float diffuse = diffuseScale * (1.0f - baseFresnel) * p.diffuseWeight * (1.0f - p.translucentWeight) *
-                          (1.0f - p.metalness) * p.diffuseColor * diffuseResponse * (1.0f - p.transmission);
-    const float viewFresnel = fresnelSchlick(gmax(dot(normal, viewDirection), 0.0f), p.f0);
-    const float translucent = diffuseScale * (1.0f - viewFresnel) * p.translucentWeight * (1.0f - p.metalness) *
-                              p.translucentColor * (backNdotL / kPi) * (1.0f - p.transmission);
-    const float specular =
-        specularScale * nDotL * evaluateGGXAnisotropic(normal, tangent, viewDirection, lightDirection, p.roughness, p.f0);
-    float coatFresnel = 0.0f;
-    float coatSpecular = 0.0f;
-    if (p.coat > 0.0f) {
-        coatFresnel = fresnelSchlick(gmax(dot(viewDirection, halfway), 0.0f), p.coatF0);
-        coatSpecular = specularScale * p.coat * nDotL *
-                       evaluateGGXAnisotropic(normal, tangent, viewDirection, lightDirection, p.coatRoughness, p.coatF0);
+    if (!kFull) {
+        if (t.nDotL <= 0.0f) return V(0.0f);
+        const float response = f.nDotV <= 0.0f ? 0.0f : t.cosine;
+        const V diffuse = V(diffuseScale) * (V(1.0f) - fresnelSchlick(t.vDotH, p.f0)) * V(p.diffuseWeight) * V(1.0f - p.metalness) *
+                          p.diffuseColor * V(response);
+        return diffuse + V(specularScale * t.nDotL) * evaluateGGXAnisotropic(f, t, lightDirection, f.alpha, f.maskView, t.d, p.f0);
     }
-    const float baseLayer = (1.0f - p.coat * coatFresnel) * (diffuseLayerSum(diffuse, translucent, specular)) + coatSpecular;
+    const float backNdotL = gmax(-t.signedNdotL, 0.0f);
+    const float wrappedNdotL = gmax((t.signedNdotL + 0.5f * p.subsurface) / (1.0f + 0.5f * p.subsurface), 0.0f);
+    if (wrappedNdotL <= 0.0f && t.nDotL <= 0.0f && backNdotL * p.translucentWeight <= 0.0f) return V(0.0f);
+    const V baseFresnel = fresnelSchlick(t.vDotH, p.f0);
+    const V diffuseResponse = mix(evaluateDiffuseReflection(f.normal, f.view, lightDirection, p.diffuseColor,
+                                                            p.diffuseRoughness, p.diffuseModel),
+                                  V(wrappedNdotL / kPi), p.subsurface);
+    const V diffuse = V(diffuseScale) * (V(1.0f) - baseFresnel) * V(p.diffuseWeight) * V(1.0f - p.translucentWeight) *
+                      V(1.0f - p.metalness) * p.diffuseColor * diffuseResponse * V(1.0f - p.transmission);
+    const V viewFresnel = fresnelSchlick(f.nDotV, p.f0);
+    const V translucent = V(diffuseScale) * (V(1.0f) - viewFresnel) * V(p.translucentWeight) * V(1.0f - p.metalness) *
+                          p.translucentColor * V(backNdotL / kPi) * V(1.0f - p.transmission);
+    const V specular = V(specularScale * t.nDotL) * evaluateGGXAnisotropic(f, t, lightDirection, f.alpha, f.maskView, t.d, p.f0);
+    V coatFresnel = V(0.0f);
+    V coatSpecular = V(0.0f);
+    if (p.coat > 0.0f) {
+        coatFresnel = fresnelSchlick(t.vDotH, p.coatF0);
+        coatSpecular = V(specularScale * p.coat * t.nDotL) *
+                       evaluateGGXAnisotropic(f, t, lightDirection, f.coatAlpha, f.maskViewCoat, t.dCoat, p.coatF0);
+    }
+    const V baseLayer = (V(1.0f) - V(p.coat) * coatFresnel) * (diffuse + translucent + specular) + coatSpecular;
     // With sheen == 0 the sheen terms are exact zeros (the albedo and the
     // response are finite), leaving baseLayer * 1 + 0.
     if (p.sheen == 0.0f) return baseLayer;
-    const float sheenAlbedo = p.sheenZeltner ? sheenZeltnerDirectionalAlbedo(gmax(dot(normal, viewDirection), 0.0f), p.sheenRoughness)
-                                             : sheenDirectionalAlbedo(gmax(dot(normal, viewDirection), 0.0f), p.sheenRoughness);
-    const float sheenLayer = specularScale * p.sheen * p.sheenColor *
-                             sheenResponse(normal, viewDirection, lightDirection, p.sheenRoughness, p.sheenZeltner);
-    return baseLayer * (1.0f - clampf(p.sheen * sheenAlbedo, 0.0f, 1.0f)) + sheenLayer;
+    const float sheenAlbedo = p.sheenZeltner ? sheenZeltnerDirectionalAlbedo(f.nDotV, p.sheenRoughness)
+                                             : sheenDirectionalAlbedo(f.nDotV, p.sheenRoughness);
+    const V sheenLayer = V(specularScale * p.sheen) * p.sheenColor *
+                         V(sheenResponse(f.normal, f.view, lightDirection, p.sheenRoughness, p.sheenZeltner));
+    return baseLayer * V(1.0f - clampf(p.sheen * sheenAlbedo, 0.0f, 1.0f)) + sheenLayer;
 }
 
-// Not inlined: called from several sites of the shade kernel, one shared
-// copy keeps the kernel's instruction footprint smaller (measured faster).
-HDCX_NOINLINE float surfaceReflectionPdf(float3 normal, float3 tangent, float3 viewDirection, float3 lightDirection,
-                                  float2 roughness, float2 coatRoughness, float sheenProbability, float coatProbability,
-                                  float specularProbability, float translucentProbability)
+template <bool kFull, class V>
+HDCX_D V surfaceReflectionPdf(const ShadingFrame& f, const LobeTerms& t, V sheenProbability, V coatProbability,
+                              V specularProbability, V translucentProbability)
 {
     // :392-415
-    const float reflectionCosinePdf = gmax(dot(normal, lightDirection), 0.0f) / kPi;
-    const float transmissionCosinePdf = gmax(-dot(normal, lightDirection), 0.0f) / kPi;
-    const float coatPdf = ggxReflectionPdfAnisotropic(normal, tangent, viewDirection, lightDirection, coatRoughness);
-    const float specularPdf = ggxReflectionPdfAnisotropic(normal, tangent, viewDirection, lightDirection, roughness);
-    const float diffusePdf = mix(reflectionCosinePdf, transmissionCosinePdf, translucentProbability);
-    const float basePdf = coatProbability * coatPdf +
-                          (1.0f - coatProbability) * (specularProbability * specularPdf + (1.0f - specularProbability) * diffusePdf);
-    return sheenProbability * reflectionCosinePdf + (1.0f - sheenProbability) * basePdf;
+    const float specularPdf = ggxReflectionPdfAnisotropic(f, t, t.d);
+    // kFull = false: sheen, coat and diffuse transmission have probability zero.
+    if (!kFull) return specularProbability * V(specularPdf) + (V(1.0f) - specularProbability) * V(t.cosine);
+    const float transmissionCosinePdf = gmax(-t.signedNdotL, 0.0f) / kPi;
+    const float coatPdf = f.coated ? ggxReflectionPdfAnisotropic(f, t, t.dCoat) : 0.0f;
+    const V diffusePdf = mixBy(t.cosine, transmissionCosinePdf, translucentProbability);
+    const V basePdf = coatProbability * V(coatPdf) +
+                      (V(1.0f) - coatProbability) * (specularProbability * V(specularPdf) + (V(1.0f) - specularProbability) * diffusePdf);
+    return sheenProbability * V(t.cosine) + (V(1.0f) - sheenProbability) * basePdf;
 }
 
 HDCX_D float3 offsetSurfaceOrigin(float3 position, float3 geometricNormal, float3 direction)
@@ -591,18 +659,18 @@ HDCX_D float shapingConeFactor(const GpuLight& light, float cosine)
                                : (outer <= inner + 1e-6f ? (angle <= outer ? 1.0f : 0.0f) : 1.0f - smoothstep(inner, outer, angle));
 }
 
-HDCX_D float dispersedIor(float iorAtD, float scale, float abbeNumber, float wavelength)
+template <class V>
+HDCX_D V dispersedIor(float iorAtD, float scale, float abbeNumber, V wavelength)
 {
     // :1096-1110 (Cauchy fit through the Abbe number)
-    if (scale <= 0.0f || abbeNumber <= 1.0f) return iorAtD;
+    if (scale <= 0.0f || abbeNumber <= 1.0f) return V(iorAtD);
     const float lambdaF = 486.13f;
     const float lambdaD = 587.56f;
     const float lambdaC = 656.27f;
     const float reciprocalDelta = 1.0f / (lambdaF * lambdaF) - 1.0f / (lambdaC * lambdaC);
     const float b = (iorAtD - 1.0f) / gmax(abbeNumber * reciprocalDelta, 1e-8f);
     const float a = iorAtD - b / (lambdaD * lambdaD);
-    const float cauchyIor = a + b / (wavelength * wavelength);
-    return mix(iorAtD, cauchyIor, clampf(scale, 0.0f, 1.0f));
+    return dispersed(iorAtD, b, a, scale, wavelength);
 }
 
 HDCX_D float3 sampleHenyeyGreenstein(float3 forward, float anisotropy, uint32_t& state)
@@ -672,13 +740,20 @@ HDCX_D float3 domeLocalDirection(const GpuLight& light, float3 worldDirection)
                         dot(worldDirection, xyz(light.basisZ))));
 }
 
-HDCX_D float3 sampleDome(const DeviceScene& s, const GpuLight& light, float3 worldDirection)
+// Texture coordinates of a world direction in a dome's texture and importance
+// texture (one lookup serves both). Not inlined: the light sample and the
+// environment pdf share the copy.
+HDCX_NOINLINE float2 domeUv(const GpuLight& light, float3 worldDirection)
 {
-    // :527-537
-    const float3 localDirection = domeLocalDirection(light, worldDirection);
+    return domeTextureCoordinates(domeLocalDirection(light, worldDirection), light.textureInfo.y);
+}
+
+HDCX_D float3 sampleDomeAt(const DeviceScene& s, const GpuLight& light, float2 uv)
+{
+    // :527-537, uv = domeUv of the direction (any value without a texture)
     float3 textureValue = f3(1.0f);
     if (light.textureInfo.x != kMissingTexture) {
-        const float4 t = textureSample(s, light.textureInfo.x, domeTextureCoordinates(localDirection, light.textureInfo.y));
+        const float4 t = textureSample(s, light.textureInfo.x, uv);
         textureValue = f3(t.x, t.y, t.z);
     }
     return xyz(light.colorIntensity) * light.colorIntensity.w * textureValue;
@@ -697,7 +772,10 @@ HDCX_D float3 environment(const DeviceScene& s, const FrameConst& f, float3 dire
     }
     for (uint32_t index = 0; index < lightCount; ++index) {
         const GpuLight& light = s.lights[index];
-        if (light.textureInfo.z == 0u) result = result + sampleDome(s, light, direction);
+        if (light.textureInfo.z == 0u) {
+            const float2 uv = light.textureInfo.x != kMissingTexture ? domeUv(light, direction) : make_float2(0.0f, 0.0f);
+            result = result + sampleDomeAt(s, light, uv);
+        }
     }
     return result;
 }
@@ -707,23 +785,20 @@ HDCX_D float3 latLongDirection(float u, float v)
     // :571-579
     const float theta = kPi * (1.0f - v);
     const float phi = 2.0f * kPi * u;
-    const float sineTheta = gsin(theta);
-    return f3(sineTheta * gsin(phi), gcos(theta), -sineTheta * gcos(phi));
+    float sineTheta, cosineTheta, sinePhi, cosinePhi;
+    gsincos(theta, sineTheta, cosineTheta);
+    gsincos(phi, sinePhi, cosinePhi);
+    return f3(sineTheta * sinePhi, cosineTheta, -sineTheta * cosinePhi);
 }
 
-HDCX_D const TexDesc* importanceTexture(const DeviceScene& s, uint32_t index)
+HDCX_D const TexDesc* importanceTexture(const TexDesc* textures, uint32_t textureCount, uint32_t index)
 {
-    return (index == kMissingTexture || index >= s.textureCount) ? nullptr : s.textures + index;
+    return (index == kMissingTexture || index >= textureCount) ? nullptr : textures + index;
 }
 
-HDCX_D float domeLightPdf(const DeviceScene& s, const GpuLight& light, float3 worldDirection)
+HDCX_D float domeLightPdf(const TexDesc& t, float2 uv)
 {
-    // :583-598
-    const TexDesc* tp = importanceTexture(s, light.textureInfo.w);
-    if (!tp) return 1.0f / 12.5663706144f;
-    const TexDesc t = *tp;
-    const float3 localDirection = domeLocalDirection(light, worldDirection);
-    const float2 uv = domeTextureCoordinates(localDirection, light.textureInfo.y);
+    // :583-598, with an importance texture; uv = domeUv of the direction
     const int w = static_cast<int>(t.width), h = static_cast<int>(t.height);
     const float fx = uv.x * u2f(t.width), fy = uv.y * u2f(t.height);
     int tx = fabsf(fx) < 2147483520.0f ? static_cast<int>(fx) : 0;
@@ -760,7 +835,7 @@ HDCX_D int cdfSearch(const float* values, const float* skip, int n, float target
 HDCX_D void sampleDomeLight(const DeviceScene& s, const GpuLight& light, uint32_t& rng, float3& worldDirection, float& pdf)
 {
     // :600-650
-    const TexDesc* tp = importanceTexture(s, light.textureInfo.w);
+    const TexDesc* tp = importanceTexture(s.textures, s.textureCount, light.textureInfo.w);
     if (!tp) {
         worldDirection = uniformSphere(rng);
         pdf = 1.0f / 12.5663706144f;
@@ -817,98 +892,138 @@ HDCX_D void sampleDomeLight(const DeviceScene& s, const GpuLight& light, uint32_
     pdf = gmax(__ldg(&rowTexels[column].z), 0.0f);
 }
 
-HDCX_D float lightSelectionWeight(const GpuLight& light, float3 position, float3 normal, float diffuseEnergy,
-                                  float specularEnergy, float translucentEnergy)
+// normalize(basisZ) of a light: from the block's table, if it has one.
+HDCX_D float3 lightAxisOf(const GpuLight* lights, const float3* lightAxes, uint32_t index)
+{
+    return lightAxes ? lightAxes[index] : normalize(xyz(lights[index].basisZ));
+}
+
+template <class V>
+HDCX_D V domeSelectionWeight(const GpuLight& light, V diffuseEnergy, V specularEnergy, V translucentEnergy)
+{
+    // :652-691, type 0
+    const float power = gmax(light.geometry.w, 0.0f);
+    if (power <= 0.0f) return V(0.0f);
+    const V diffuseResponse = gmax(diffuseEnergy, V(0.0f)) * V(light.controls.x);
+    const V specularResponse = gmax(specularEnergy, V(0.0f)) * V(light.controls.y);
+    const V transmissionResponse = gmax(translucentEnergy, V(0.0f)) * V(light.controls.x);
+    return gmax(V(power * 0.01f), V(power) * (V(0.5f) * (diffuseResponse + transmissionResponse) + specularResponse));
+}
+
+template <class V>
+HDCX_D V lightSelectionWeight(const GpuLight& light, float3 lightAxis, float3 position, float3 normal, V diffuseEnergy, V specularEnergy,
+                              V translucentEnergy)
 {
     // :652-691
     const float power = gmax(light.geometry.w, 0.0f);
-    if (power <= 0.0f) return 0.0f;
-    const float diffuseResponse = gmax(diffuseEnergy, 0.0f) * light.controls.x;
-    const float specularResponse = gmax(specularEnergy, 0.0f) * light.controls.y;
-    const float transmissionResponse = gmax(translucentEnergy, 0.0f) * light.controls.x;
+    if (power <= 0.0f) return V(0.0f);
+    const V diffuseResponse = gmax(diffuseEnergy, V(0.0f)) * V(light.controls.x);
+    const V specularResponse = gmax(specularEnergy, V(0.0f)) * V(light.controls.y);
+    const V transmissionResponse = gmax(translucentEnergy, V(0.0f)) * V(light.controls.x);
     const float minimumWeight = power * 0.01f;
     const uint32_t type = light.textureInfo.z;
-    if (type == 0u) {
-        return gmax(minimumWeight, power * (0.5f * (diffuseResponse + transmissionResponse) + specularResponse));
-    }
+    if (type == 0u) return domeSelectionWeight(light, diffuseEnergy, specularEnergy, translucentEnergy);
     float3 direction;
     float geometryFactor = 1.0f;
     if (type == 5u) {
-        direction = normalize(xyz(light.basisZ));
+        direction = lightAxis;
     } else {
         const float3 toLight = xyz(light.position) - position;
         const float distanceSquared = gmax(dot(toLight, toLight), 1e-4f);
         direction = toLight * inversesqrt(distanceSquared);
         geometryFactor = 1.0f / distanceSquared;
         if (type == 1u || type == 2u) {
-            const float3 lightNormal = -normalize(xyz(light.basisZ));
+            const float3 lightNormal = -lightAxis;
             geometryFactor = geometryFactor * gmax(dot(lightNormal, -direction), 0.0f);
         } else if (type == 4u) {
             geometryFactor = geometryFactor * 0.5f;
         }
     }
     const float nDotL = dot(normal, direction);
-    const float response = gmax(nDotL, 0.0f) * (diffuseResponse + specularResponse) + gmax(-nDotL, 0.0f) * transmissionResponse;
-    return gmax(minimumWeight, power * geometryFactor * response);
+    const V response = V(gmax(nDotL, 0.0f)) * (diffuseResponse + specularResponse) + V(gmax(-nDotL, 0.0f)) * transmissionResponse;
+    return gmax(V(minimumWeight), V(power * geometryFactor) * response);
 }
 
-// `lights`: the scene's light records, s.lights or a shared-memory copy of them.
-HDCX_D float totalAnalyticLightWeight(const DeviceScene& s, const GpuLight* lights, float3 position, float3 normal,
-                                      float diffuseEnergy, float specularEnergy, float translucentEnergy)
+// The light of each lane of `mask`, its selection probability and the total
+// weight, which environmentLightPdf takes. One draw for all lanes. `lights`:
+// the scene's light records, s.lights or a shared-memory copy of them.
+// Both passes over the lights go through one copy of the weight's code.
+template <class V>
+HDCX_D void sampleAnalyticLight(uint32_t lightCount, const GpuLight* lights, const float3* lightAxes, float3 position, float3 normal,
+                                V diffuseEnergy, V specularEnergy, V translucentEnergy, uint32_t mask, uint32_t& rng,
+                                typename LaneTraits<V>::U& lightIndex, V& selectionPdf, V& total)
 {
-    // :693-705
-    float total = 0.0f;
-    for (uint32_t index = 0; index < s.lightCount; ++index) {
-        total += lightSelectionWeight(lights[index], position, normal, diffuseEnergy, specularEnergy, translucentEnergy);
+    // :693-737
+    constexpr int kCount = LaneTraits<V>::kCount;
+    const float u = randomFloat(rng);
+    V accumulated = V(0.0f);
+    V target = V(0.0f);
+    V chosen = V(0.0f);
+    uint32_t open = 0u;  // lanes still without a light (second pass)
+    total = V(0.0f);
+    for (uint32_t step = 0; step < 2u * lightCount; ++step) {
+        const bool picking = step >= lightCount;
+        const uint32_t index = picking ? step - lightCount : step;
+        if (step == lightCount) {
+            total = accumulated;
+            accumulated = V(0.0f);
+            target = V(u) * total;
+            open = mask;
+        }
+        const V weight = lightSelectionWeight(lights[index], lightAxisOf(lights, lightAxes, index), position, normal, diffuseEnergy, specularEnergy, translucentEnergy);
+        accumulated = accumulated + weight;
+        if (!picking) continue;
+#pragma unroll
+        for (int k = 0; k < kCount; ++k) {
+            // The last light takes what rounding leaves over.
+            if ((open >> k & 1u) && (at(target, k) <= at(accumulated, k) || index + 1u == lightCount)) {
+                put(lightIndex, k, index);
+                put(chosen, k, at(weight, k));
+                open &= ~(1u << k);
+            }
+        }
+        if (open == 0u) break;
     }
-    return total;
-}
-
-HDCX_D void sampleAnalyticLight(const DeviceScene& s, const GpuLight* lights, float3 position, float3 normal,
-                                float diffuseEnergy, float specularEnergy, float translucentEnergy, uint32_t& rng,
-                                uint32_t& lightIndex, float& selectionPdf)
-{
-    // :707-737
-    const uint32_t lightCount = s.lightCount;
-    const float total = totalAnalyticLightWeight(s, lights, position, normal, diffuseEnergy, specularEnergy, translucentEnergy);
-    if (total <= 0.0f) {
-        const float scaled = randomFloat(rng) * u2f(lightCount);
-        const uint32_t pick = scaled >= 4294967296.0f ? 0xffffffffu : static_cast<uint32_t>(scaled);
-        lightIndex = min(pick, lightCount - 1u);
-        selectionPdf = 1.0f / u2f(lightCount);
-        return;
-    }
-    const float target = randomFloat(rng) * total;
-    float accumulated = 0.0f;
-    lightIndex = lightCount - 1u;
-    for (uint32_t index = 0; index < lightCount; ++index) {
-        const float weight = lightSelectionWeight(lights[index], position, normal, diffuseEnergy, specularEnergy, translucentEnergy);
-        accumulated += weight;
-        if (target <= accumulated) {
-            lightIndex = index;
-            break;
+    selectionPdf = ratioLikelyOne(chosen, total);  // one light: the ratio is one
+#pragma unroll
+    for (int k = 0; k < kCount; ++k) {
+        if (at(total, k) <= 0.0f) {
+            const float scaled = u * u2f(lightCount);
+            const uint32_t pick = scaled >= 4294967296.0f ? 0xffffffffu : static_cast<uint32_t>(scaled);
+            put(lightIndex, k, min(pick, lightCount - 1u));
+            put(selectionPdf, k, 1.0f / u2f(lightCount));
         }
     }
-    selectionPdf = lightSelectionWeight(lights[lightIndex], position, normal, diffuseEnergy, specularEnergy, translucentEnergy) / total;
 }
 
-// Not inlined: called from several sites of the shade kernel, one shared
-// copy keeps the kernel's instruction footprint smaller (measured faster).
-HDCX_NOINLINE float environmentLightPdf(const DeviceScene& s, const GpuLight* lights, float3 position, float3 normal,
-                                        float3 direction, float diffuseEnergy, float specularEnergy, float translucentEnergy)
+// Probability density of `direction` under dome light selection and sampling.
+// `total`: the total light weight of the same position and energies
+// (sampleAnalyticLight); `known`, `knownUv`: a light whose domeUv of the
+// direction the caller has (~0u: none). Not inlined: called from two sites of
+// the shade kernel, one shared copy keeps its instruction footprint smaller;
+// the arguments are scalars, so that the scene record stays in constant
+// memory.
+template <class V>
+HDCX_NOINLINE V environmentLightPdf(const TexDesc* textures, uint32_t textureCount, uint32_t lightCount, const GpuLight* lights,
+                                    float3 direction, V diffuseEnergy, V specularEnergy, V translucentEnergy, V total,
+                                    uint32_t known, float2 knownUv)
 {
     // :739-758
-    if (s.lightCount == 0u) return 0.0f;
-    const float total = totalAnalyticLightWeight(s, lights, position, normal, diffuseEnergy, specularEnergy, translucentEnergy);
-    if (total <= 0.0f) return 0.0f;
-    float pdf = 0.0f;
-    for (uint32_t index = 0; index < s.lightCount; ++index) {
+    V pdf = V(0.0f);
+    for (uint32_t index = 0; index < lightCount; ++index) {
         const GpuLight& light = lights[index];
         if (light.textureInfo.z == 0u) {
-            const float selectionPdf =
-                lightSelectionWeight(light, position, normal, diffuseEnergy, specularEnergy, translucentEnergy) / total;
-            pdf += selectionPdf * domeLightPdf(s, light, direction);
+            const V selectionPdf = ratioLikelyOne(domeSelectionWeight(light, diffuseEnergy, specularEnergy, translucentEnergy), total);
+            const TexDesc* tp = importanceTexture(textures, textureCount, light.textureInfo.w);
+            float density = 1.0f / 12.5663706144f;
+            if (tp) density = domeLightPdf(*tp, index == known ? knownUv : domeUv(light, direction));
+            pdf = pdf + selectionPdf * V(density);
         }
+    }
+    // A lane without any light weight has no light sample.
+#pragma unroll
+    for (int k = 0; k < LaneTraits<V>::kCount; ++k) {
+        if (at(total, k) <= 0.0f) put(pdf, k, 0.0f);
     }
     return pdf;
 }

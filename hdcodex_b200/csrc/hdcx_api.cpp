@@ -105,29 +105,24 @@ struct PathStore {
         p.capacity = n;
         p.wavePaths = n;
         p.shadowPerPath = shadowPerPath;
-        p.rng = alloc<uint32_t>(n);
         p.wavelength = alloc<float>(n);
         p.spectrum = alloc<float4>(n);
         p.throughput = alloc<float>(n);
         p.radiance = alloc<float>(n);
-        p.rayOrigin = alloc<float4>(n);
-        p.rayDirection = alloc<float4>(n);
-        p.flags = alloc<uint32_t>(n);
+        p.ray = alloc<float4>(2 * n);
         p.previousPdf = alloc<float2>(n);
         p.medium = alloc<float4>(n);
         p.hit = alloc<float4>(n);
         p.contribution = alloc<float>(3 * n);
-        p.contributionValid = alloc<uint8_t>(3 * n);
         p.queue[0] = alloc<uint32_t>(n);
         p.queue[1] = alloc<uint32_t>(n);
+        p.groupQueue = alloc<uint32_t>(n / 2 + 1);
         p.hitQueue = alloc<uint32_t>(n);
         p.missQueue = alloc<uint32_t>(n);
-        p.shadowOrigin = alloc<float4>(ns);
-        p.shadowDirection = alloc<float4>(ns);
+        p.shadowRay = alloc<float4>(2 * ns);
         p.shadowFactors = alloc<float4>(ns);
-        p.shadowSlot = alloc<uint32_t>(ns);
         p.shadowInfo = alloc<uint32_t>(ns);
-        p.counters = alloc<uint32_t>(8);
+        p.counters = alloc<uint32_t>(kCountEnd);
         p.sortedHits = alloc<uint32_t>(n);
         p.hitBins = alloc<uint32_t>(2 * kHitBins);
         p.walkEntry = alloc<float4>(n);
@@ -417,6 +412,15 @@ bool needsFullShading(const PackedSceneData& d)
         if (!(m.transmissionOpacityIor.x <= 0.0F) || !(m.coatColor.w <= 0.0F) || !(m.translucentColorWeight.w <= 0.0F)) {
             return true;  // NaN weights take the general kernel
         }
+        // The specialised kernel leaves out the terms that a zero weight
+        // multiplies: exact zeros while their factors are finite.
+        for (float v : {m.sheenColorMode.x, m.sheenColorMode.y, m.sheenColorMode.z, m.translucentColorWeight.x,
+                        m.translucentColorWeight.y, m.translucentColorWeight.z, m.coatWeightRoughnessIor.y,
+                        m.subsurfaceRadius.w, m.transmissionScatter.w, m.baseColorMetalness.x, m.baseColorMetalness.y,
+                        m.baseColorMetalness.z, m.specularWeightColor.x, m.specularWeightColor.y, m.specularWeightColor.z,
+                        m.specularWeightColor.w, m.transmissionOpacityIor.z}) {
+            if (!std::isfinite(v)) return true;
+        }
     }
     return false;
 }
@@ -685,8 +689,17 @@ void uploadScene(hdcx_tracer* t, const PackedSceneData& d)
     s.lights = reinterpret_cast<const GpuLight*>(t->upload(d.lights));
     s.emissive = reinterpret_cast<const float4*>(t->upload(d.emissive));
     std::vector<TexDesc> descs;
+    std::vector<float> byteTable;  // TexDesc::bytes, where a texture has 8-bit texels
+    const float* bytes = nullptr;
     for (const PackedTexture& pt : d.textures) {
         TexDesc td{};
+        if (pt.format != HDCX_TEXEL_RGBA32F && !bytes) {
+            byteTable.resize(512);
+            srgbTable(byteTable.data());
+            for (int v = 0; v < 256; ++v) byteTable[256 + v] = static_cast<float>(v) / 255.0F;
+            bytes = t->upload(byteTable);
+        }
+        td.bytes = bytes;
         td.width = pt.width;
         td.height = pt.height;
         td.format = pt.format;
@@ -1045,10 +1058,6 @@ HDCX_API hdcx_status hdcx_create(int32_t device, hdcx_tracer** out)
         check(cudaStreamCreateWithFlags(&t->stream, cudaStreamNonBlocking), "cudaStreamCreate");
         check(cudaEventCreate(&t->start), "cudaEventCreate");
         check(cudaEventCreate(&t->stop), "cudaEventCreate");
-        float table[256];
-        srgbTable(table);
-        uploadSrgbTable(table, t->stream);
-        check(cudaStreamSynchronize(t->stream), "init");
     });
     if (s != HDCX_OK) {
         delete t;

@@ -39,35 +39,47 @@ struct CacheDevice {
 // Material bins of the hit sort (material index modulo kHitBins).
 constexpr uint32_t kHitBins = 256;
 
-// Device buffers of one wave of paths (structure of arrays, 16-byte records).
+// Queue counters of a wave (32-bit words of PathBuffers::counters). The
+// extension and shadow queues count entries in a 64-bit counter's low half
+// and lanes in its high half. One clear per bounce covers the counters that
+// the bounce fills: kCountQueue0 .. kCountEnd without the queue it reads.
+enum : uint32_t {
+    kCountQueue0 = 0,    // 64-bit: extension queue of even bounces
+    kCountShadow = 2,    // 64-bit: shadow queue
+    kCountGroups = 4,    // hits of entries with several lanes
+    kCountSingles = 5,   // hits of entries with one lane
+    kCountMisses = 6,
+    kCountWalks = 7,     // deferred subsurface walks
+    kCountReplays = 8,   // failed walks to re-shade
+    kCountQueue1 = 10,   // 64-bit: extension queue of odd bounces
+    kCountEnd = 12,
+};
+
+// Device buffers of one wave of paths (structure of arrays; slot 3 g + lane,
+// see device/paths.cuh for groups and leaders).
 struct PathBuffers {
-    uint64_t capacity = 0;          // paths the buffers hold (the stride of the per-slot arrays)
+    uint64_t capacity = 0;          // paths the buffers hold
     uint64_t wavePaths = 0;         // paths per wave, at most capacity (0: capacity)
     uint32_t shadowPerPath = 0;     // shadow-ray slots per path per bounce
-    uint32_t* rng = nullptr;
+    uint32_t lightSlots = 3;        // light-sample slots in use: 1 (analytic), 2 (+ mesh lights) or 3 (fallback sun and sky)
+    uint32_t split = 0;             // 1: every lane travels as an entry of its own from the start
     float* wavelength = nullptr;
     float4* spectrum = nullptr;     // basis r, g, b and Planck factor of the lane
     float* throughput = nullptr;
     float* radiance = nullptr;
-    float4* rayOrigin = nullptr;
-    float4* rayDirection = nullptr;
-    uint32_t* flags = nullptr;
+    float4* ray = nullptr;          // at leaders, two per slot: origin and RNG state, direction and flags
     float2* previousPdf = nullptr;  // previousBsdfPdf, previousEnvironmentLightPdf
     float4* medium = nullptr;       // absorption, scattering, anisotropy
-    float4* hit = nullptr;          // t, primitive (bits), b1, b2
-    float* contribution = nullptr;  // 3 * capacity: path slot s, light-sample slot k at 3 s + k
-    uint8_t* contributionValid = nullptr;  // same indexing as contribution
-    uint32_t* queue[2] = {nullptr, nullptr};
-    uint32_t* hitQueue = nullptr;       // extend's output: paths whose ray hit (shaded)
-    uint32_t* missQueue = nullptr;      // extend's output: paths whose ray missed (environment)
-    float4* shadowOrigin = nullptr;     // xyz, tmax
-    float4* shadowDirection = nullptr;  // xyz, partial product
-    float4* shadowFactors = nullptr;    // f1, f2, f3
-    uint32_t* shadowSlot = nullptr;     // path slot * 4 + k
-    uint32_t* shadowInfo = nullptr;     // kind | light << 8
-    // [0], [1] extension queues, [2] shadow queue, [4] hits, [5] misses,
-    // [6] deferred subsurface walks, [7] failed walks to re-shade (8 entries)
-    uint32_t* counters = nullptr;
+    float4* hit = nullptr;          // at leaders: t, primitive (bits), b1, b2
+    float* contribution = nullptr;  // 3 * capacity: path slot s, light-sample slot j at lightSlots * s + j
+    uint32_t* queue[2] = {nullptr, nullptr};  // extension entries
+    uint32_t* groupQueue = nullptr;     // extend's output: entries of several lanes whose ray hit
+    uint32_t* hitQueue = nullptr;       // extend's output: entries of one lane whose ray hit
+    uint32_t* missQueue = nullptr;      // extend's output: entries whose ray missed (environment)
+    float4* shadowRay = nullptr;        // two per shadow ray: origin and tmax, direction and entry
+    float4* shadowFactors = nullptr;    // per path slot and light-sample slot (kShadowGeneral): partial product, f1, f2, f3
+    uint32_t* shadowInfo = nullptr;     // kind, light-sample slot, light (device/paths.cuh)
+    uint32_t* counters = nullptr;       // kCountEnd words
     // extension, shadow, subsurface rays; extension node visits and triangle
     // tests; shadow node visits and triangle tests (counting mode)
     unsigned long long* stats = nullptr;
@@ -110,8 +122,6 @@ struct StageTimes {
     uint32_t waves = 0;
     uint32_t extendLaunches = 0;
 };
-
-void uploadSrgbTable(const float* table256, cudaStream_t stream);
 
 // Renders sampleCount samples per pixel into fb (running mean update).
 // `timing` non-null records per-stage device times with CUDA events.

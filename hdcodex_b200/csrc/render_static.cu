@@ -40,29 +40,24 @@ constexpr uint64_t alignUp(uint64_t v) { return (v + kAlign - 1) / kAlign * kAli
 constexpr uint64_t kN = kStaticWavePaths;
 constexpr uint64_t kShadow = kN * kStaticShadowPerPath;
 constexpr uint64_t kRegionBytes[] = {
-    4 * kN,                        // rng
     4 * kN,                        // wavelength
     16 * kN,                       // spectrum
     4 * kN,                        // throughput
     4 * kN,                        // radiance
-    16 * kN,                       // rayOrigin
-    16 * kN,                       // rayDirection
-    4 * kN,                        // flags
+    32 * kN,                       // ray
     8 * kN,                        // previousPdf
     16 * kN,                       // medium
     16 * kN,                       // hit
     4 * 3 * kN,                    // contribution (3 slots)
-    3 * kN,                        // contributionValid
     4 * kN,                        // queue[0]
     4 * kN,                        // queue[1]
+    4 * (kN / 2 + 1),              // groupQueue
     4 * kN,                        // hitQueue
     4 * kN,                        // missQueue
-    16 * kShadow,                  // shadowOrigin
-    16 * kShadow,                  // shadowDirection
+    32 * kShadow,                  // shadowRay
     16 * kShadow,                  // shadowFactors
-    4 * kShadow,                   // shadowSlot
     4 * kShadow,                   // shadowInfo
-    4 * 8,                         // counters
+    4 * kCountEnd,                 // counters
     8 * 8,                         // stats
     16 * kStaticMaxPixels,         // batch (float4 per pixel)
     24 * kStaticMaxPixels,         // batchXyz (3 doubles per pixel)
@@ -127,37 +122,32 @@ unsigned int renderStatic(const DeviceScene& scene, const FrameConst& frame, flo
     p.capacity = kN;
     p.wavePaths = kN;
     p.shadowPerPath = kStaticShadowPerPath;
-    p.rng = reinterpret_cast<uint32_t*>(region[0]);
-    p.wavelength = reinterpret_cast<float*>(region[1]);
-    p.spectrum = reinterpret_cast<float4*>(region[2]);
-    p.throughput = reinterpret_cast<float*>(region[3]);
-    p.radiance = reinterpret_cast<float*>(region[4]);
-    p.rayOrigin = reinterpret_cast<float4*>(region[5]);
-    p.rayDirection = reinterpret_cast<float4*>(region[6]);
-    p.flags = reinterpret_cast<uint32_t*>(region[7]);
-    p.previousPdf = reinterpret_cast<float2*>(region[8]);
-    p.medium = reinterpret_cast<float4*>(region[9]);
-    p.hit = reinterpret_cast<float4*>(region[10]);
-    p.contribution = reinterpret_cast<float*>(region[11]);
-    p.contributionValid = reinterpret_cast<uint8_t*>(region[12]);
-    p.queue[0] = reinterpret_cast<uint32_t*>(region[13]);
-    p.queue[1] = reinterpret_cast<uint32_t*>(region[14]);
-    p.hitQueue = reinterpret_cast<uint32_t*>(region[15]);
-    p.missQueue = reinterpret_cast<uint32_t*>(region[16]);
-    p.shadowOrigin = reinterpret_cast<float4*>(region[17]);
-    p.shadowDirection = reinterpret_cast<float4*>(region[18]);
-    p.shadowFactors = reinterpret_cast<float4*>(region[19]);
-    p.shadowSlot = reinterpret_cast<uint32_t*>(region[20]);
-    p.shadowInfo = reinterpret_cast<uint32_t*>(region[21]);
-    p.counters = reinterpret_cast<uint32_t*>(region[22]);
-    p.stats = reinterpret_cast<unsigned long long*>(region[23]);
+    p.wavelength = reinterpret_cast<float*>(region[0]);
+    p.spectrum = reinterpret_cast<float4*>(region[1]);
+    p.throughput = reinterpret_cast<float*>(region[2]);
+    p.radiance = reinterpret_cast<float*>(region[3]);
+    p.ray = reinterpret_cast<float4*>(region[4]);
+    p.previousPdf = reinterpret_cast<float2*>(region[5]);
+    p.medium = reinterpret_cast<float4*>(region[6]);
+    p.hit = reinterpret_cast<float4*>(region[7]);
+    p.contribution = reinterpret_cast<float*>(region[8]);
+    p.queue[0] = reinterpret_cast<uint32_t*>(region[9]);
+    p.queue[1] = reinterpret_cast<uint32_t*>(region[10]);
+    p.groupQueue = reinterpret_cast<uint32_t*>(region[11]);
+    p.hitQueue = reinterpret_cast<uint32_t*>(region[12]);
+    p.missQueue = reinterpret_cast<uint32_t*>(region[13]);
+    p.shadowRay = reinterpret_cast<float4*>(region[14]);
+    p.shadowFactors = reinterpret_cast<float4*>(region[15]);
+    p.shadowInfo = reinterpret_cast<uint32_t*>(region[16]);
+    p.counters = reinterpret_cast<uint32_t*>(region[17]);
+    p.stats = reinterpret_cast<unsigned long long*>(region[18]);
 
     FrameBuffers fb;
     fb.width = frame.width;
     fb.height = frame.height;
     fb.rgba = rgba;
-    fb.batch = reinterpret_cast<float4*>(region[24]);
-    fb.batchXyz = reinterpret_cast<double*>(region[25]);
+    fb.batch = reinterpret_cast<float4*>(region[19]);
+    fb.batchXyz = reinterpret_cast<double*>(region[20]);
     // The frame's FP64 XYZ running sums are not kept by this variant: the
     // finalize pass adds them into the batch sums of the same pixel (each
     // thread reads and writes only its own pixel), which the next call clears.
@@ -165,7 +155,7 @@ unsigned int renderStatic(const DeviceScene& scene, const FrameConst& frame, flo
 
     // The array keeps the previous call's contents: the queue counters and
     // ray statistics must start at zero (renderFrame clears the batch sums).
-    ok(cudaMemsetAsync(p.counters, 0, 8 * sizeof(uint32_t), stream), "clear counters");
+    ok(cudaMemsetAsync(p.counters, 0, kCountEnd * sizeof(uint32_t), stream), "clear counters");
     ok(cudaMemsetAsync(p.stats, 0, 8 * sizeof(unsigned long long), stream), "clear stats");
     renderFrame(scene, frame, p, fb, stream, nullptr, false, nullptr);
     // The lock covers the GPU work too: the next call may reuse the array.

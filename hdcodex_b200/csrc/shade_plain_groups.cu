@@ -1,0 +1,24 @@
+// shade_plain_groups.cu - shade variants of scenes without textures and layered lobes, entries of several lanes.
+#include "device/shade.cuh"
+#include "shade.h"
+
+namespace hdcx {
+
+namespace {
+
+template <int kLanes, bool kFull, bool kLit, bool kCache, int kWalk>
+void launch(const ShadeLaunch& l)
+{
+    shadeKernel<kLanes, kFull, kLit, kCache, kWalk><<<l.grid, 128, 0, l.stream>>>(l.scene, l.frame, l.paths, l.bounce, l.queue,
+                                                                                  l.count, l.nextQueue, l.nextCount);
+}
+
+}  // namespace
+
+void shadePlainGroups(bool lit, const ShadeLaunch& l)
+{
+    if (lit) launch<3, false, true, false, kWalkInline>(l);
+    else launch<3, false, false, false, kWalkInline>(l);
+}
+
+}  // namespace hdcx

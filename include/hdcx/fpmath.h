@@ -131,22 +131,37 @@ HDCX_FP float hdcx_fp_reduce_half_pi(float x, int32_t* quadrant)
     return r;
 }
 
-HDCX_FP float hdcx_fp_sin(float x)
+/* Both polynomials are evaluated and one picked, so that the threads of a warp
+ * run one instruction sequence whatever their quadrants. */
+HDCX_FP void hdcx_fp_sincos(float x, float* sine, float* cosine)
 {
-    if (!(x == x) || x - x != 0.0f) return (x - x) / (x - x); /* NaN for NaN and inf */
+#if !defined(__CUDA_ARCH__)
+    if (!(x == x) || x - x != 0.0f) { /* NaN for NaN and inf; on the GPU the reduction gives it */
+        *sine = *cosine = (x - x) / (x - x);
+        return;
+    }
+#endif
     int32_t q;
     const float r = hdcx_fp_reduce_half_pi(x, &q);
-    const float s = (q & 1) ? hdcx_fp_cos_poly(r) : hdcx_fp_sin_poly(r);
-    return (q & 2) ? -s : s;
+    const float sp = hdcx_fp_sin_poly(r), cp = hdcx_fp_cos_poly(r);
+    const float s = (q & 1) ? cp : sp;
+    const float c = (q & 1) ? sp : cp;
+    *sine = (q & 2) ? -s : s;
+    *cosine = ((q + 1) & 2) ? -c : c;
+}
+
+HDCX_FP float hdcx_fp_sin(float x)
+{
+    float s, c;
+    hdcx_fp_sincos(x, &s, &c);
+    return s;
 }
 
 HDCX_FP float hdcx_fp_cos(float x)
 {
-    if (!(x == x) || x - x != 0.0f) return (x - x) / (x - x);
-    int32_t q;
-    const float r = hdcx_fp_reduce_half_pi(x, &q);
-    const float c = (q & 1) ? hdcx_fp_sin_poly(r) : hdcx_fp_cos_poly(r);
-    return ((q + 1) & 2) ? -c : c;
+    float s, c;
+    hdcx_fp_sincos(x, &s, &c);
+    return c;
 }
 
 HDCX_FP float hdcx_fp_exp(float x)
@@ -342,10 +357,10 @@ HDCX_FP float hdcx_fp_atan2(float y, float x)
     if (ax - ax != 0.0f || ay - ay != 0.0f) { /* infinities */
         if (ax - ax != 0.0f && ay - ay != 0.0f) a = 0.78539816339744830962f;
         else a = (ay - ay != 0.0f) ? 1.57079632679489661923f : 0.0f;
-    } else if (ay <= ax) {
-        a = hdcx_fp_atan01(ay / ax);
-    } else {
-        a = 1.57079632679489661923f - hdcx_fp_atan01(ax / ay);
+    } else { /* one evaluation for both octants */
+        const int steep = ay > ax;
+        a = hdcx_fp_atan01((steep ? ax : ay) / (steep ? ay : ax));
+        if (steep) a = 1.57079632679489661923f - a;
     }
     if (negX) a = 3.14159265358979323846f - a;
     return negY ? -a : a;
@@ -374,18 +389,17 @@ HDCX_FP float hdcx_fp_acos(float x)
 {
     if (!(x >= -1.0f && x <= 1.0f)) return hdcx_fp_bits_to_float(0x7fc00000u);
     const float ax = x < 0.0f ? -x : x;
-    float r;
-    if (ax <= 0.5f) {
-        r = 1.57079632679489661923f - (x < 0.0f ? -hdcx_fp_asin_half(ax) : hdcx_fp_asin_half(ax));
-    } else {
-        /* acos|x| = 2 asin(sqrt((1 - |x|)/2)) */
+    /* acos|x| = pi/2 - asin|x|, or 2 asin(sqrt((1 - |x|)/2)) above 1/2: one
+     * series for both. */
+    const int large = ax > 0.5f;
 #if defined(__CUDA_ARCH__)
-        const float h = 2.0f * hdcx_fp_asin_half(__fsqrt_rn((1.0f - ax) * 0.5f));
+    const float root = __fsqrt_rn((1.0f - ax) * 0.5f);
 #else
-        const float h = 2.0f * hdcx_fp_asin_half(sqrtf((1.0f - ax) * 0.5f));
+    const float root = sqrtf((1.0f - ax) * 0.5f);
 #endif
-        r = x < 0.0f ? 3.14159265358979323846f - h : h;
-    }
+    const float p = hdcx_fp_asin_half(large ? root : ax);
+    const float h = 2.0f * p;
+    const float r = large ? (x < 0.0f ? 3.14159265358979323846f - h : h) : 1.57079632679489661923f - (x < 0.0f ? -p : p);
     return r;
 }
 
