@@ -78,10 +78,15 @@ struct DeviceBuffer {
 struct PathStore {
     std::vector<DeviceBuffer*> buffers;
     PathBuffers paths;
+    unsigned long long* hostStats = nullptr;  // pinned, 8 counters: a render's statistics arrive with its image
     PathStore() = default;
     PathStore(const PathStore&) = delete;
     PathStore& operator=(const PathStore&) = delete;
-    ~PathStore() { release(); }
+    ~PathStore()
+    {
+        release();
+        if (hostStats) cudaFreeHost(hostStats);
+    }
     void release()
     {
         for (DeviceBuffer* b : buffers) delete b;
@@ -100,6 +105,11 @@ struct PathStore {
     void allocate(uint64_t n, uint32_t shadowPerPath)
     {
         release();
+        if (!hostStats &&
+            cudaHostAlloc(reinterpret_cast<void**>(&hostStats), 8 * sizeof(unsigned long long), cudaHostAllocDefault) != cudaSuccess) {
+            hostStats = nullptr;  // finishRender copies to ordinary memory instead
+            cudaGetLastError();
+        }
         PathBuffers& p = paths;
         const uint64_t ns = n * shadowPerPath;
         p.capacity = n;
@@ -835,7 +845,9 @@ uint64_t ensureStore(hdcx_tracer* t, PathStore& store, uint64_t needed, uint64_t
     const uint64_t cap = t->wavePaths ? t->wavePaths : (capOverride ? capOverride : kAutomaticWavePaths);
     uint64_t capacity = std::max<uint64_t>(3, std::min(needed, cap));
     if (fixed) return std::min(capacity, store.paths.capacity);
-    if (t->wavePaths == 0) {
+    // (Buffers that already hold the wave serve as they are: no memory query,
+    // a driver call that took from 0.1 ms up to milliseconds on a busy host.)
+    if (t->wavePaths == 0 && (store.paths.capacity < capacity || store.paths.shadowPerPath < kShadowSlots)) {
         size_t freeBytes = 0, totalBytes = 0;
         check(cudaMemGetInfo(&freeBytes, &totalBytes), "cudaMemGetInfo");
         const uint64_t held = store.paths.capacity * (143ull + 56ull * store.paths.shadowPerPath);
@@ -1335,6 +1347,7 @@ void enqueueAovs(hdcx_tracer* t, const FrameConst& frame);
 struct RenderCall {
     FrameConst frame{};
     PathBuffers paths;  // the buffers this call renders with: the tracer's own, or a batch lane's
+    unsigned long long* hostStats = nullptr;  // pinned, with the buffers
     uint64_t pathsNeeded = 0;
     StageTimes times;
     uint64_t launches = 0;
@@ -1360,6 +1373,7 @@ void prepareRender(hdcx_tracer* t, const hdcx_camera& camera, uint32_t width, ui
     const bool fixed = fixedArena && &store != &t->own;
     const uint64_t wave = ensureStore(t, store, call.pathsNeeded, waveCap, fixed);
     call.paths = store.paths;
+    call.hostStats = store.hostStats;
     call.paths.wavePaths = wave;
     call.paths.stats = tracerStats(t);
     call.paths.traceBlocksPerSm = t->traceBlocksPerSm;
@@ -1422,13 +1436,15 @@ void throwOnTraversalFault(unsigned long long word)
 // `graphMs` >= 0: the render ran inside a batch graph, which measured its device time.
 void finishRender(hdcx_tracer* t, RenderCall& call, float graphMs = -1.0F)
 {
+    unsigned long long counters[8];
     {
         NvtxRange range("hdcx wait for render");
+        unsigned long long* const landing = call.hostStats ? call.hostStats : counters;
+        check(cudaMemcpyAsync(landing, call.paths.stats, sizeof counters, cudaMemcpyDeviceToHost, t->stream), "read stats");
         check(cudaStreamSynchronize(t->stream), "render");
+        if (landing != counters) std::memcpy(counters, landing, sizeof counters);
     }
     t->xyzSamples = (call.frame.sampleIndex == 0 ? 0 : t->xyzSamples) + call.frame.sampleCount;
-    unsigned long long counters[8];
-    check(cudaMemcpy(counters, call.paths.stats, sizeof counters, cudaMemcpyDeviceToHost), "read stats");
     throwOnTraversalFault(counters[7]);
     float ms = graphMs;
     if (graphMs < 0.0F) check(cudaEventElapsedTime(&ms, t->start, t->stop), "cudaEventElapsedTime");
@@ -1821,17 +1837,29 @@ BatchPlan planBatch(hdcx_batch_job* jobs, uint32_t count, uint64_t pathBudget)
         }
         if (leases.empty()) continue;
         const uint32_t lanes = static_cast<uint32_t>(leases.size());
+        std::vector<uint64_t> paths;
+        for (uint32_t j : eligible) paths.push_back(need(j));
         uint64_t budget = pathBudget;
+        LanePlan lanePlan;
+        bool planned = false;
         if (budget == 0) {
+            // Lanes whose arenas already hold what they would ask of ample
+            // memory need no look at the memory that is free.
+            lanePlan = planLanes(paths, lanes, ~0ull / kPathStateBytes, kBatchLaneWave, 1ull << 20);
+            planned = true;
+            for (uint32_t l = 0; l < lanes; ++l) {
+                const PathStore& store = leases[l].arena->store;
+                planned = planned && store.paths.capacity >= lanePlan.capacity[l] && store.paths.shadowPerPath >= 3u;
+            }
+        }
+        if (budget == 0 && !planned) {
             size_t freeBytes = 0, totalBytes = 0;
             if (cudaMemGetInfo(&freeBytes, &totalBytes) != cudaSuccess) freeBytes = 0;
             uint64_t held = 0;
             for (const ArenaLease& l : leases) held += l.arena->store.paths.capacity * kPathStateBytes;
             budget = (freeBytes + held) / 2 / kPathStateBytes;
         }
-        std::vector<uint64_t> paths;
-        for (uint32_t j : eligible) paths.push_back(need(j));
-        const LanePlan lanePlan = planLanes(paths, lanes, budget, kBatchLaneWave, 1ull << 20);
+        if (!planned) lanePlan = planLanes(paths, lanes, budget, kBatchLaneWave, 1ull << 20);
         for (uint32_t l = 0; l < lanes; ++l) {
             std::vector<uint32_t> members;
             for (uint32_t k : lanePlan.members[l]) members.push_back(eligible[k]);
