@@ -37,6 +37,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <mutex>
 #include <random>
 #include <stdexcept>
 #include <string>
@@ -181,29 +182,60 @@ __device__ __forceinline__ void levelCorners(const DeviceParams& p, int level, f
     }
 }
 
-// The 64 network inputs of query record q (zeros for a missing query).
-__device__ void encodeQuery(const DeviceParams& p, const float* q, float in[kWidth])
+// Hash-grid encoding of a chunk of records: 16 levels x 2 features per query,
+// rounded to BF16 as the network takes them, one row of kGridFeatures each.
+//
+// The encoding is 128 gathers of 4 bytes per query and was the cost of the
+// query kernel (1.75 ms per 2^21 queries, tensor pipe 2%): inside it, four
+// blocks of 51 KB of shared memory left 16 warps and 24 KB of L1 per SM for
+// gathers that wait on L2. Here it has the whole SM (few registers, no shared
+// memory), a thread gathers four levels of one query, and the corners of a
+// cell that differ in x arrive together: their indices differ by an XOR of
+// x ^ (x + 1) in the hashed levels and by one in the dense ones, so three
+// times in four both lie in one aligned group of four entries, a 16-byte load.
+// Same products and sums in the same order as corner by corner.
+constexpr int kEncodeLevels = 4;       // levels per thread
+constexpr uint32_t kGridFeatures = kLevels * kFeatures;
+
+__device__ __forceinline__ float2 entryOf(const uint4& four, uint32_t index)
 {
+    const uint32_t low = (index & 1u) ? four.y : four.x, high = (index & 1u) ? four.w : four.z;
+    const uint32_t bits = (index & 2u) ? high : low;
+    return __half22float2(*reinterpret_cast<const __half2*>(&bits));
+}
+
+__global__ void __launch_bounds__(256) encodeKernel(DeviceParams p, const float* queries, uint32_t count, __nv_bfloat16* features)
+{
+    const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= count) return;
+    // Scalar loads: callers' records need no more than float alignment.
+    const float* record = queries + static_cast<size_t>(q) * kQueryFloats;
+    const float3 pos = make_float3(__ldg(record), __ldg(record + 1), __ldg(record + 2));
+    const int firstLevel = static_cast<int>(blockIdx.y) * kEncodeLevels;
+    __align__(16) __nv_bfloat162 out[kEncodeLevels];
 #pragma unroll
-    for (int i = 0; i < kWidth; ++i) in[i] = 0.0f;
-    if (!q) return;
-    const float3 pos = make_float3(q[0], q[1], q[2]);
-    for (int level = 0; level < kLevels; ++level) {
+    for (int l = 0; l < kEncodeLevels; ++l) {
         uint32_t index[8];
         float weight[8];
-        levelCorners(p, level, pos, index, weight);
+        levelCorners(p, firstLevel + l, pos, index, weight);
+        // The four corner pairs (x, x + 1).
+        uint4 four[4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) four[c] = __ldg(reinterpret_cast<const uint4*>(p.grid) + (index[2 * c] >> 2));
         float f0 = 0.0f, f1 = 0.0f;
 #pragma unroll
-        for (int c = 0; c < 8; ++c) {
-            const float2 v = __half22float2(p.grid[index[c]]);
-            f0 = fmaf(weight[c], v.x, f0);
-            f1 = fmaf(weight[c], v.y, f1);
+        for (int c = 0; c < 4; ++c) {
+            const float2 a = entryOf(four[c], index[2 * c]);
+            float2 b = entryOf(four[c], index[2 * c + 1]);
+            if ((index[2 * c] ^ index[2 * c + 1]) > 3u) b = __half22float2(__ldg(p.grid + index[2 * c + 1]));
+            f0 = fmaf(weight[2 * c], a.x, f0);
+            f1 = fmaf(weight[2 * c], a.y, f1);
+            f0 = fmaf(weight[2 * c + 1], b.x, f0);
+            f1 = fmaf(weight[2 * c + 1], b.y, f1);
         }
-        in[2 * level] = f0;
-        in[2 * level + 1] = f1;
+        out[l] = __nv_bfloat162(__float2bfloat16_rn(f0), __float2bfloat16_rn(f1));
     }
-#pragma unroll
-    for (int i = 0; i < 9; ++i) in[32 + i] = q[3 + i];
+    *reinterpret_cast<uint4*>(features + static_cast<size_t>(q) * kGridFeatures + 2 * firstLevel) = *reinterpret_cast<const uint4*>(out);
 }
 
 // Writes 64 values of row `row` as BF16 into a tile with `colGroups` column groups.
@@ -214,6 +246,31 @@ __device__ __forceinline__ void storeRow(__nv_bfloat16* tile, uint32_t row, cons
 #pragma unroll
         for (int i = 0; i < 8; ++i) b[i] = __float2bfloat16_rn(v[c + i]);
         *reinterpret_cast<uint4*>(tile + tiled(row, static_cast<uint32_t>(c), colGroups)) = *reinterpret_cast<const uint4*>(b);
+    }
+}
+
+// Input row of query `q`: its encoded features (columns 0..31), the record's
+// direction, normal, roughness and wavelength (32..40), zeros; all zeros for a
+// missing query.
+__device__ __forceinline__ void storeInputRow(__nv_bfloat16* tile, uint32_t row, const __nv_bfloat16* features, const float* record)
+{
+    const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+    for (uint32_t c = 0; c < kGridFeatures; c += 8)
+        *reinterpret_cast<uint4*>(tile + tiled(row, c, 8u)) = record ? __ldg(reinterpret_cast<const uint4*>(features + c)) : zero;
+    float rest[kWidth - static_cast<int>(kGridFeatures)];
+#pragma unroll
+    for (int i = 0; i < kWidth - static_cast<int>(kGridFeatures); ++i) rest[i] = 0.0f;
+    if (record) {
+#pragma unroll
+        for (int i = 0; i < 9; ++i) rest[i] = __ldg(record + 3 + i);
+    }
+#pragma unroll
+    for (int c = 0; c < kWidth - static_cast<int>(kGridFeatures); c += 8) {
+        __align__(16) __nv_bfloat16 h[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) h[i] = __float2bfloat16_rn(rest[c + i]);
+        *reinterpret_cast<uint4*>(tile + tiled(row, kGridFeatures + static_cast<uint32_t>(c), 8u)) = *reinterpret_cast<const uint4*>(h);
     }
 }
 
@@ -238,46 +295,69 @@ __device__ __forceinline__ void issueForward(uint32_t dTmem, const __nv_bfloat16
 // ---------------------------------------------------------------------------
 // Kernels
 // ---------------------------------------------------------------------------
-constexpr uint32_t kQuerySmem = kWeightCount * 2u + kTile * kWidth * 2u + 16u;
+// Queries per block: kQueryGroups tiles of 128, one per group of four warps
+// with its own activations, tensor-memory columns and barriers; the weights
+// (35 KB) are shared. A tile is a chain of five dependent GEMMs, each far too
+// small for the tensor pipe, so the kernel runs at tiles in flight per SM:
+// two blocks of four tiles fit (99 KB each) where blocks of one tile (51 KB)
+// fitted four.
+constexpr uint32_t kQueryGroups = 4;
+constexpr uint32_t kQueryThreads = kQueryGroups * 128u;
+constexpr uint32_t kQuerySmem = kWeightCount * 2u + kQueryGroups * kTile * kWidth * 2u + (kQueryGroups + 1u) * 8u;
 
-__global__ void __launch_bounds__(128) queryKernel(DeviceParams p, const float* queries, uint32_t count, float* out,
-                                                   uint32_t* error)
+// Barrier of one group of four warps (named barrier 1 + group).
+__device__ __forceinline__ void groupSync(uint32_t group) { asm volatile("barrier.cta.sync %0, 128;" ::"r"(group + 1u) : "memory"); }
+__device__ __forceinline__ bool groupSyncOr(uint32_t group, bool value)
+{
+    uint32_t any;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %2, 0;\n\tbarrier.cta.red.or.pred q, %1, 128, p;\n\tselp.u32 %0, 1, 0, q;\n\t}\n"
+        : "=r"(any)
+        : "r"(group + 1u), "r"(value ? 1u : 0u)
+        : "memory");
+    return any != 0u;
+}
+
+__global__ void __launch_bounds__(kQueryThreads, 2) queryKernel(DeviceParams p, const float* queries, const __nv_bfloat16* features,
+                                                                uint32_t count, float* out, uint32_t* error)
 {
     extern __shared__ __align__(16) uint8_t smem[];
     __nv_bfloat16* w = reinterpret_cast<__nv_bfloat16*>(smem);
-    __nv_bfloat16* x = w + kWeightCount;
-    uint64_t* bar = reinterpret_cast<uint64_t*>(x + kTile * kWidth);
-    uint32_t* slot = reinterpret_cast<uint32_t*>(bar + 1);
-    const uint32_t warp = threadIdx.x >> 5;
+    const uint32_t group = threadIdx.x / 128u, row = threadIdx.x % 128u;
+    const uint32_t warp = row >> 5;  // in its group
+    __nv_bfloat16* x = w + kWeightCount + group * kTile * kWidth;
+    uint64_t* bars = reinterpret_cast<uint64_t*>(w + kWeightCount + kQueryGroups * kTile * kWidth);
+    uint64_t* bar = bars + group;
+    uint32_t* slot = reinterpret_cast<uint32_t*>(bars + kQueryGroups);
     loadWeights(w, p.weights);
-    if (threadIdx.x == 0) barrierInit(bar);
-    if (warp == 0) tmemAllocate(slot, 64u);
+    if (row == 0) barrierInit(bar);
+    if (threadIdx.x < 32u) tmemAllocate(slot, 64u * kQueryGroups);
     fenceProxyAsync();
     fenceBeforeSync();
     __syncthreads();
     fenceAfterSync();
-    const uint32_t tmem = *slot;
+    const uint32_t tmem = *slot + 64u * group;  // the group's columns
     const uint32_t laneBase = tmem + ((warp * 32u) << 16);
     uint32_t phase = 0;
     bool failed = false;
-    for (uint32_t base = blockIdx.x * kTile; base < count && !failed; base += gridDim.x * kTile) {
-        const uint32_t row = threadIdx.x;
+    for (uint32_t base = (blockIdx.x * kQueryGroups + group) * kTile; base < count && !failed; base += gridDim.x * kQueryGroups * kTile) {
         const uint32_t q = base + row;
         float v[kWidth];
-        encodeQuery(p, q < count ? queries + static_cast<size_t>(q) * kQueryFloats : nullptr, v);
-        storeRow(x, row, v, 8u, kWidth);
+        storeInputRow(x, row, features + static_cast<size_t>(q) * kGridFeatures,
+                      q < count ? queries + static_cast<size_t>(q) * kQueryFloats : nullptr);
         for (int layer = 0; layer < kLayers; ++layer) {
             fenceProxyAsync();
             fenceBeforeSync();
-            __syncthreads();
+            groupSync(group);
             fenceAfterSync();
-            if (threadIdx.x == 0) {
+            if (row == 0) {
                 issueForward(tmem, x, w, layer);
                 commitTo(bar);
             }
-            // Every thread takes the same decision, so that no barrier or
-            // warp-collective tensor-memory load is reached by only some.
-            if (__syncthreads_or(barrierWait(bar, phase) ? 0 : 1)) {
+            // Every thread of the group takes the same decision, so that no
+            // barrier or warp-collective tensor-memory load is reached by
+            // only some.
+            if (groupSyncOr(group, !barrierWait(bar, phase))) {
                 failed = true;
                 break;
             }
@@ -298,20 +378,22 @@ __global__ void __launch_bounds__(128) queryKernel(DeviceParams p, const float* 
     if (failed) {
         // Bounded: lets an MMA still in flight finish before the memory is freed.
         const bool drained = barrierWait(bar, phase);
-        if (threadIdx.x == 0) atomicOr(error, drained ? kErrorTimeout : (kErrorTimeout | kErrorDrain));
+        if (row == 0) atomicOr(error, drained ? kErrorTimeout : (kErrorTimeout | kErrorDrain));
     }
     __syncthreads();
     fenceAfterSync();
-    if (warp == 0) tmemFree(tmem, 64u);
+    if (threadIdx.x < 32u) tmemFree(*slot, 64u * kQueryGroups);
 }
 
 // Forward and backward of every tile of 128 training records; weight
 // gradients accumulate in tensor memory and are added to `mlpGrad` at the
-// end; hash-grid gradients are scattered with atomics into `gridGrad`.
+// end; the gradients of the encoded features go to `featureGrad`, one row of
+// kGridFeatures per record, from which scatterKernel adds them to the table.
 constexpr uint32_t kTrainSmem = kWeightCount * 2u + 5u * kTile * kWidth * 2u + kTile * 128u * 2u + 16u;
 
-__global__ void __launch_bounds__(128) trainKernel(DeviceParams p, const float* queries, const float* targets, uint32_t count,
-                                                   float gradientScale, float* mlpGrad, float* gridGrad, float* lossSum,
+__global__ void __launch_bounds__(128) trainKernel(DeviceParams p, const float* queries, const __nv_bfloat16* features,
+                                                   const float* targets, uint32_t count, float gradientScale, float* mlpGrad,
+                                                   float* featureGrad, float* lossSum,
                                                    uint32_t* error)
 {
     extern __shared__ __align__(16) uint8_t smem[];
@@ -342,8 +424,7 @@ __global__ void __launch_bounds__(128) trainKernel(DeviceParams p, const float* 
         const bool valid = q < count;
         const float* record = valid ? queries + static_cast<size_t>(q) * kQueryFloats : nullptr;
         float v[kWidth];
-        encodeQuery(p, record, v);
-        storeRow(xs, row, v, 8u, kWidth);
+        storeInputRow(xs, row, features + static_cast<size_t>(q) * kGridFeatures, record);
         float prediction = 0.0f;
         // Forward, keeping X_0 .. X_4.
         for (int layer = 0; layer < kLayers && !failed; ++layer) {
@@ -431,20 +512,10 @@ __global__ void __launch_bounds__(128) trainKernel(DeviceParams p, const float* 
                 }
                 storeRow(g, row, v, 16u, kWidth);
             } else if (valid) {
-                // Hash-grid gradients: input columns 0..31.
-                const float3 pos = make_float3(record[0], record[1], record[2]);
-                for (int level = 0; level < kLevels; ++level) {
-                    uint32_t index[8];
-                    float weight[8];
-                    levelCorners(p, level, pos, index, weight);
-                    const float d0 = v[2 * level], d1 = v[2 * level + 1];
-                    if (d0 == 0.0f && d1 == 0.0f) continue;
+                // Gradients of the encoded features: input columns 0..31.
+                float4* dst = reinterpret_cast<float4*>(featureGrad + static_cast<size_t>(q) * kGridFeatures);
 #pragma unroll
-                    for (int c = 0; c < 8; ++c) {
-                        atomicAdd(gridGrad + 2u * index[c], weight[c] * d0);
-                        atomicAdd(gridGrad + 2u * index[c] + 1u, weight[c] * d1);
-                    }
-                }
+                for (int c = 0; c < static_cast<int>(kGridFeatures); c += 4) dst[c / 4] = make_float4(v[c], v[c + 1], v[c + 2], v[c + 3]);
             }
             fenceBeforeSync();
         }
@@ -467,7 +538,9 @@ __global__ void __launch_bounds__(128) trainKernel(DeviceParams p, const float* 
             for (int c = 0; c < kWidth; c += 16) tmemLoad16(tmem + laneOffset + 64u + 64u * layer + static_cast<uint32_t>(c), d + c);
             if (r < static_cast<uint32_t>(layerRows(layer))) {
                 float* dst = mlpGrad + layerOffset(layer) + r * kWidth;
-                for (int c = 0; c < kWidth; ++c) atomicAdd(dst + c, d[c]);
+#pragma unroll
+                for (int c = 0; c < kWidth; c += 4)
+                    atomicAdd(reinterpret_cast<float4*>(dst + c), make_float4(d[c], d[c + 1], d[c + 2], d[c + 3]));
             }
         }
     }
@@ -476,6 +549,51 @@ __global__ void __launch_bounds__(128) trainKernel(DeviceParams p, const float* 
     __syncthreads();
     fenceAfterSync();
     if (warp == 0) tmemFree(tmem, 512u);
+}
+
+// Hash-grid gradients: every feature gradient times its corner's weight, added
+// to the table's FP32 gradients. One thread per record and kEncodeLevels
+// levels, a two-float vector atomic per corner. (Inside trainKernel, with one
+// block of four warps per SM, the scatter waited on its own latency: 228 us a
+// step of 2^16 records for the whole kernel.)
+__global__ void __launch_bounds__(256) scatterKernel(DeviceParams p, const float* queries, const float* featureGrad, uint32_t count,
+                                                     float* gridGrad)
+{
+    const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= count) return;
+    // Scalar loads: callers' records need no more than float alignment.
+    const float* record = queries + static_cast<size_t>(q) * kQueryFloats;
+    const float3 pos = make_float3(__ldg(record), __ldg(record + 1), __ldg(record + 2));
+    const int firstLevel = static_cast<int>(blockIdx.y) * kEncodeLevels;
+    const float4* row = reinterpret_cast<const float4*>(featureGrad + static_cast<size_t>(q) * kGridFeatures + 2 * firstLevel);
+    float d[2 * kEncodeLevels];
+#pragma unroll
+    for (int i = 0; i < kEncodeLevels / 2; ++i) {
+        const float4 v = __ldg(row + i);
+        d[4 * i] = v.x, d[4 * i + 1] = v.y, d[4 * i + 2] = v.z, d[4 * i + 3] = v.w;
+    }
+#pragma unroll
+    for (int l = 0; l < kEncodeLevels; ++l) {
+        const float d0 = d[2 * l], d1 = d[2 * l + 1];
+        if (d0 == 0.0f && d1 == 0.0f) continue;
+        uint32_t index[8];
+        float weight[8];
+        levelCorners(p, firstLevel + l, pos, index, weight);
+        // Corners that differ in x share an aligned pair of entries when their
+        // indices differ in the lowest bit alone: one four-float atomic.
+#pragma unroll
+        for (int c = 0; c < 8; c += 2) {
+            const float2 a = make_float2(weight[c] * d0, weight[c] * d1), b = make_float2(weight[c + 1] * d0, weight[c + 1] * d1);
+            if ((index[c] ^ index[c + 1]) == 1u) {
+                const bool swapped = (index[c] & 1u) != 0u;
+                atomicAdd(reinterpret_cast<float4*>(gridGrad) + (index[c] >> 1),
+                          swapped ? make_float4(b.x, b.y, a.x, a.y) : make_float4(a.x, a.y, b.x, b.y));
+            } else {
+                atomicAdd(reinterpret_cast<float2*>(gridGrad) + index[c], a);
+                atomicAdd(reinterpret_cast<float2*>(gridGrad) + index[c + 1], b);
+            }
+        }
+    }
 }
 
 // The kernels' bounded wait on an mbarrier that nothing arrives at: the wait
@@ -489,26 +607,67 @@ __global__ void waitTimeoutKernel(uint32_t limit, uint32_t* error)
     if (__syncthreads_or(barrierWait(&bar, 0u, limit) ? 0 : 1) && threadIdx.x == 0) atomicOr(error, kErrorTimeout);
 }
 
-// Adam on `n` FP32 parameters; refreshes the BF16 tiled weights (mlp) or the
-// FP16 table (grid) and clears the gradients.
-__global__ void adamKernel(float* params, float* grad, float* m, float* v, uint32_t n, float lr, float beta1, float beta2,
-                           float epsilon, float correction1, float correction2, __nv_bfloat16* tiledWeights, __half* table)
+// Adam on the FP32 parameters of the table and the network in one launch (the
+// network's 17,408 weights in the last blocks); refreshes the FP16 table and
+// the BF16 tiled weights and clears the gradients. Bound by memory: 34 bytes
+// per parameter, four parameters a thread. A parameter without gradient and
+// moments stays as it is and is only read (its step is exactly zero).
+struct AdamArrays {
+    float* params;
+    float* grad;
+    float* m;
+    float* v;
+};
+struct AdamStep {
+    float lr, beta1, beta2, epsilon, correction1, correction2;
+};
+
+__device__ __forceinline__ float adamUpdate(const AdamStep& a, float g, float& m, float& v, float param)
 {
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const float gi = grad[i];
-        const float mi = beta1 * m[i] + (1.0f - beta1) * gi;
-        const float vi = beta2 * v[i] + (1.0f - beta2) * gi * gi;
-        m[i] = mi;
-        v[i] = vi;
-        const float pi = params[i] - lr * (mi / correction1) / (sqrtf(vi / correction2) + epsilon);
-        params[i] = pi;
-        grad[i] = 0.0f;
-        if (tiledWeights) {
+    m = a.beta1 * m + (1.0f - a.beta1) * g;
+    v = a.beta2 * v + (1.0f - a.beta2) * g * g;
+    return param - a.lr * (m / a.correction1) / (sqrtf(v / a.correction2) + a.epsilon);
+}
+
+constexpr uint32_t kAdamThreads = 256;
+constexpr uint32_t kAdamMlpBlocks = kWeightCount / 4u / kAdamThreads;
+static_assert(kAdamMlpBlocks * kAdamThreads * 4u == kWeightCount, "the network's weights fill whole blocks");
+
+__global__ void __launch_bounds__(kAdamThreads) adamKernel(AdamArrays grid, uint32_t gridCount, AdamArrays mlp, AdamStep step,
+                                                           __nv_bfloat16* tiledWeights, __half* table)
+{
+    const uint32_t gridBlocks = gridDim.x - kAdamMlpBlocks;
+    const bool network = blockIdx.x >= gridBlocks;
+    const AdamArrays a = network ? mlp : grid;
+    const uint32_t n = network ? kWeightCount : gridCount;
+    const uint32_t stride = (network ? kAdamMlpBlocks : gridBlocks) * kAdamThreads * 4u;
+    for (uint32_t i = ((network ? blockIdx.x - gridBlocks : blockIdx.x) * kAdamThreads + threadIdx.x) * 4u; i < n; i += stride) {
+        const float4 g = *reinterpret_cast<const float4*>(a.grad + i);
+        float4 m = *reinterpret_cast<const float4*>(a.m + i), v = *reinterpret_cast<const float4*>(a.v + i);
+        const bool idle = step.epsilon > 0.0f && g.x == 0.0f && g.y == 0.0f && g.z == 0.0f && g.w == 0.0f && m.x == 0.0f && m.y == 0.0f && m.z == 0.0f &&
+                          m.w == 0.0f && v.x == 0.0f && v.y == 0.0f && v.z == 0.0f && v.w == 0.0f;
+        if (idle) continue;
+        float4 param = *reinterpret_cast<const float4*>(a.params + i);
+        param.x = adamUpdate(step, g.x, m.x, v.x, param.x);
+        param.y = adamUpdate(step, g.y, m.y, v.y, param.y);
+        param.z = adamUpdate(step, g.z, m.z, v.z, param.z);
+        param.w = adamUpdate(step, g.w, m.w, v.w, param.w);
+        *reinterpret_cast<float4*>(a.m + i) = m;
+        *reinterpret_cast<float4*>(a.v + i) = v;
+        *reinterpret_cast<float4*>(a.params + i) = param;
+        *reinterpret_cast<float4*>(a.grad + i) = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (network) {
+            // Four columns of one row: half a row of a core-matrix block.
             const uint32_t layer = i < 16384u ? i / 4096u : 4u;
             const uint32_t local = i - layerOffset(static_cast<int>(layer));
-            tiledWeights[layerOffset(static_cast<int>(layer)) + tiled(local / 64u, local % 64u, 8u)] = __float2bfloat16_rn(pi);
+            __align__(8) __nv_bfloat16 h[4] = {__float2bfloat16_rn(param.x), __float2bfloat16_rn(param.y), __float2bfloat16_rn(param.z),
+                                               __float2bfloat16_rn(param.w)};
+            *reinterpret_cast<uint2*>(tiledWeights + layerOffset(static_cast<int>(layer)) + tiled(local / 64u, local % 64u, 8u)) =
+                *reinterpret_cast<const uint2*>(h);
+        } else {
+            __align__(8) __half h[4] = {__float2half_rn(param.x), __float2half_rn(param.y), __float2half_rn(param.z), __float2half_rn(param.w)};
+            *reinterpret_cast<uint2*>(table + i) = *reinterpret_cast<const uint2*>(h);
         }
-        if (table) table[i] = __float2half_rn(pi);
     }
 }
 
@@ -547,8 +706,15 @@ struct Cache {
     float* gridM = nullptr;
     float* gridV = nullptr;
     __half* gridHalf = nullptr;
-    float* loss = nullptr;
-    uint32_t* error = nullptr;
+    float* loss = nullptr;      // the loss sum, and after it the error word: one copy reads both
+    uint32_t* error = nullptr;  // loss + 1
+    // Encoded features and their gradients of one chunk of records. Calls on
+    // one cache share them: each holds `work` until its kernels have finished.
+    std::mutex work;
+    __nv_bfloat16* features = nullptr;
+    float* featureGrad = nullptr;
+    uint32_t chunk = 0;         // records `features` holds
+    uint32_t trainChunk = 0;    // records `featureGrad` holds
     uint64_t step = 0;
     int sms = 148;
 
@@ -566,11 +732,15 @@ struct Cache {
 
 namespace {
 
-void checkError(Cache* c, cudaStream_t stream)
+// Waits for the stream; throws if a kernel recorded an error. `loss` gets the
+// loss sum.
+void finish(Cache* c, cudaStream_t stream, float* loss = nullptr)
 {
-    uint32_t e = 0;
-    NRC_OK(cudaMemcpyAsync(&e, c->error, sizeof e, cudaMemcpyDeviceToHost, stream));
+    uint32_t words[2] = {0, 0};
+    NRC_OK(cudaMemcpyAsync(words, c->loss, sizeof words, cudaMemcpyDeviceToHost, stream));
     NRC_OK(cudaStreamSynchronize(stream));
+    if (loss) std::memcpy(loss, words, sizeof(float));
+    const uint32_t e = words[1];
     if (e != 0u) {
         NRC_OK(cudaMemsetAsync(c->error, 0, sizeof(uint32_t), stream));
         throw std::runtime_error((e & kErrorDrain) != 0u
@@ -580,12 +750,21 @@ void checkError(Cache* c, cudaStream_t stream)
     }
 }
 
-void runTrainKernel(Cache* c, const float* queries, const float* targets, uint32_t count, cudaStream_t stream)
+dim3 encodeGrid(uint32_t count) { return dim3((count + 255u) / 256u, kLevels / kEncodeLevels); }
+
+// Forward and backward of all records, chunk by chunk; gradients and loss add up.
+void runTrainKernels(Cache* c, const float* queries, const float* targets, uint32_t count, cudaStream_t stream)
 {
-    const int blocks = static_cast<int>(std::min<uint32_t>((count + kTile - 1) / kTile, static_cast<uint32_t>(c->sms)));
-    trainKernel<<<blocks, 128, kTrainSmem, stream>>>(c->params(), queries, targets, count, 1.0f / static_cast<float>(count),
-                                                     c->mlpGrad, c->gridGrad, c->loss, c->error);
-    NRC_OK(cudaGetLastError());
+    for (uint32_t begin = 0; begin < count; begin += c->trainChunk) {
+        const uint32_t n = std::min(c->trainChunk, count - begin);
+        const float* records = queries + static_cast<size_t>(begin) * kQueryFloats;
+        encodeKernel<<<encodeGrid(n), 256, 0, stream>>>(c->params(), records, n, c->features);
+        const int blocks = static_cast<int>(std::min<uint32_t>((n + kTile - 1) / kTile, static_cast<uint32_t>(c->sms)));
+        trainKernel<<<blocks, 128, kTrainSmem, stream>>>(c->params(), records, c->features, targets + begin, n,
+                                                         1.0f / static_cast<float>(count), c->mlpGrad, c->featureGrad, c->loss, c->error);
+        scatterKernel<<<encodeGrid(n), 256, 0, stream>>>(c->params(), records, c->featureGrad, n, c->gridGrad);
+        NRC_OK(cudaGetLastError());
+    }
 }
 
 }  // namespace
@@ -618,8 +797,23 @@ Cache* create(int device, const Config& config)
     c->gridM = deviceAlloc<float>(c->gridCount);
     c->gridV = deviceAlloc<float>(c->gridCount);
     c->gridHalf = deviceAlloc<__half>(c->gridCount);
-    c->loss = deviceAlloc<float>(1);
-    c->error = deviceAlloc<uint32_t>(1);
+    c->loss = deviceAlloc<float>(2);
+    c->error = reinterpret_cast<uint32_t*>(c->loss + 1);
+    // Chunks of 2^20 records to encode (64 MB of features, which stay in L2
+    // between the kernels; chunks of 2^18 cost 0.14 ms of launch gaps in a
+    // query of 10^6) and of 2^18 to train on (32 MB), fewer where memory is short.
+    for (c->chunk = 1u << 20;; c->chunk >>= 1) {
+        c->trainChunk = std::min(c->chunk, 1u << 18);
+        try {
+            c->features = deviceAlloc<__nv_bfloat16>(static_cast<size_t>(c->chunk) * kGridFeatures);
+            c->featureGrad = deviceAlloc<float>(static_cast<size_t>(c->trainChunk) * kGridFeatures);
+            break;
+        } catch (const std::exception&) {
+            deviceFree(c->features);
+            c->features = nullptr;
+            if (c->chunk <= kTile) throw;
+        }
+    }
     NRC_OK(cudaFuncSetAttribute(queryKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kQuerySmem));
     NRC_OK(cudaFuncSetAttribute(trainKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTrainSmem));
     // Initialisation: weights uniform in +-sqrt(6 / (fan_in + fan_out)), table uniform in +-1e-4.
@@ -646,7 +840,8 @@ void destroy(Cache* c)
     for (void* p : {static_cast<void*>(c->mlp), static_cast<void*>(c->mlpGrad), static_cast<void*>(c->mlpM),
                     static_cast<void*>(c->mlpV), static_cast<void*>(c->mlpTiled), static_cast<void*>(c->grid),
                     static_cast<void*>(c->gridGrad), static_cast<void*>(c->gridM), static_cast<void*>(c->gridV),
-                    static_cast<void*>(c->gridHalf), static_cast<void*>(c->loss), static_cast<void*>(c->error)})
+                    static_cast<void*>(c->gridHalf), static_cast<void*>(c->loss), static_cast<void*>(c->features),
+                    static_cast<void*>(c->featureGrad)})
         deviceFree(p);
     delete c;
 }
@@ -680,9 +875,10 @@ void getParameters(Cache* c, float* mlp, float* grid)
 
 void checkWaitTimeout(Cache* c, uint32_t polls, cudaStream_t stream)
 {
+    std::lock_guard<std::mutex> hold(c->work);
     waitTimeoutKernel<<<1, 128, 0, stream>>>(polls, c->error);
     NRC_OK(cudaGetLastError());
-    checkError(c, stream);
+    finish(c, stream);
 }
 
 uint64_t gridParameterCount(const Cache* c) { return c->gridCount; }
@@ -691,42 +887,50 @@ uint32_t resolution(const Cache* c, int level) { return c->resolution[level]; }
 void query(Cache* c, const float* queries, uint32_t count, float* out, cudaStream_t stream)
 {
     if (count == 0) return;
-    const int blocks = static_cast<int>(std::min<uint32_t>((count + kTile - 1) / kTile, static_cast<uint32_t>(c->sms) * 4u));
-    queryKernel<<<blocks, 128, kQuerySmem, stream>>>(c->params(), queries, count, out, c->error);
-    NRC_OK(cudaGetLastError());
-    checkError(c, stream);
+    std::lock_guard<std::mutex> hold(c->work);
+    for (uint32_t begin = 0; begin < count; begin += c->chunk) {
+        const uint32_t n = std::min(c->chunk, count - begin);
+        const float* records = queries + static_cast<size_t>(begin) * kQueryFloats;
+        encodeKernel<<<encodeGrid(n), 256, 0, stream>>>(c->params(), records, n, c->features);
+        const uint32_t tiles = kQueryGroups * kTile;  // per block
+        const int blocks = static_cast<int>(std::min<uint32_t>((n + tiles - 1) / tiles, static_cast<uint32_t>(c->sms) * 2u));
+        queryKernel<<<blocks, kQueryThreads, kQuerySmem, stream>>>(c->params(), records, c->features, n, out + begin, c->error);
+        NRC_OK(cudaGetLastError());
+    }
+    finish(c, stream);
 }
 
 float train(Cache* c, const float* queries, const float* targets, uint32_t count, uint32_t steps, cudaStream_t stream)
 {
     if (count == 0 || steps == 0) return 0.0f;
+    std::lock_guard<std::mutex> hold(c->work);
+    const uint32_t gridCount = static_cast<uint32_t>(c->gridCount);
+    const uint32_t gridBlocks = std::min((gridCount / 4u + kAdamThreads - 1u) / kAdamThreads, static_cast<uint32_t>(c->sms) * 16u);
     float lossValue = 0.0f;
     for (uint32_t s = 0; s < steps; ++s) {
         NRC_OK(cudaMemsetAsync(c->loss, 0, sizeof(float), stream));
-        runTrainKernel(c, queries, targets, count, stream);
+        runTrainKernels(c, queries, targets, count, stream);
         ++c->step;
         const float b1 = 1.0f - std::pow(c->config.beta1, float(c->step));
         const float b2 = 1.0f - std::pow(c->config.beta2, float(c->step));
-        adamKernel<<<64, 256, 0, stream>>>(c->mlp, c->mlpGrad, c->mlpM, c->mlpV, kWeightCount, c->config.learningRate,
-                                           c->config.beta1, c->config.beta2, c->config.epsilon, b1, b2, c->mlpTiled, nullptr);
-        adamKernel<<<c->sms * 8, 256, 0, stream>>>(c->grid, c->gridGrad, c->gridM, c->gridV, static_cast<uint32_t>(c->gridCount),
-                                                   c->config.learningRate, c->config.beta1, c->config.beta2,
-                                                   c->config.epsilon, b1, b2, nullptr, c->gridHalf);
+        adamKernel<<<gridBlocks + kAdamMlpBlocks, kAdamThreads, 0, stream>>>(
+            AdamArrays{c->grid, c->gridGrad, c->gridM, c->gridV}, gridCount, AdamArrays{c->mlp, c->mlpGrad, c->mlpM, c->mlpV},
+            AdamStep{c->config.learningRate, c->config.beta1, c->config.beta2, c->config.epsilon, b1, b2}, c->mlpTiled, c->gridHalf);
         NRC_OK(cudaGetLastError());
     }
-    NRC_OK(cudaMemcpyAsync(&lossValue, c->loss, sizeof(float), cudaMemcpyDeviceToHost, stream));
-    checkError(c, stream);
+    finish(c, stream, &lossValue);
     return lossValue / static_cast<float>(count);
 }
 
 void gradients(Cache* c, const float* queries, const float* targets, uint32_t count, float* mlpGrad, float* gridGrad,
                cudaStream_t stream)
 {
+    std::lock_guard<std::mutex> hold(c->work);
     NRC_OK(cudaMemsetAsync(c->mlpGrad, 0, kWeightCount * sizeof(float), stream));
     NRC_OK(cudaMemsetAsync(c->gridGrad, 0, c->gridCount * sizeof(float), stream));
     NRC_OK(cudaMemsetAsync(c->loss, 0, sizeof(float), stream));
-    if (count > 0) runTrainKernel(c, queries, targets, count, stream);
-    checkError(c, stream);
+    if (count > 0) runTrainKernels(c, queries, targets, count, stream);
+    finish(c, stream);
     if (mlpGrad) NRC_OK(cudaMemcpy(mlpGrad, c->mlpGrad, kWeightCount * sizeof(float), cudaMemcpyDeviceToHost));
     if (gridGrad) NRC_OK(cudaMemcpy(gridGrad, c->gridGrad, c->gridCount * sizeof(float), cudaMemcpyDeviceToHost));
     NRC_OK(cudaMemsetAsync(c->mlpGrad, 0, kWeightCount * sizeof(float), stream));
