@@ -254,13 +254,15 @@ HDCX_D float radians(float degrees) { return degrees * 0.017453292519943295f; }
 
 // Transcendentals: the binary32 functions of hdcx/fpmath.h, bit-identical to
 // the CPU evaluations of the integrator.
-HDCX_D float gexp(float x) { return hdcx_fp_exp(x); }
-HDCX_D float glog(float x) { return hdcx_fp_log(x); }
-HDCX_D float gpow(float x, float y) { return hdcx_fp_pow(x, y); }
+// Those with long bodies that a kernel meets in several places are one shared
+// copy each: the shade kernels are bound by instruction fetch.
+HDCX_NOINLINE float gexp(float x) { return hdcx_fp_exp(x); }
+HDCX_NOINLINE float glog(float x) { return hdcx_fp_log(x); }
+HDCX_NOINLINE float gpow(float x, float y) { return hdcx_fp_pow(x, y); }
 HDCX_D float gsin(float x) { return hdcx_fp_sin(x); }
 HDCX_D float gcos(float x) { return hdcx_fp_cos(x); }
 HDCX_D void gsincos(float x, float& sine, float& cosine) { hdcx_fp_sincos(x, &sine, &cosine); }
-HDCX_D float gacos(float x) { return hdcx_fp_acos(x); }
+HDCX_NOINLINE float gacos(float x) { return hdcx_fp_acos(x); }
 HDCX_D float gatan2(float y, float x) { return hdcx_fp_atan2(y, x); }
 
 #endif  // __CUDACC__

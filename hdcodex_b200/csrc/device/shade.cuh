@@ -114,17 +114,36 @@ HDCX_D bool decide(V p, int f, uint32_t& sub, uint32_t& rng)
     return yes;
 }
 
-template <int kLanes, bool kFull, bool kLit, bool kCache, int kWalk>
+// Threads per block and resident blocks per SM of a variant.
+//
+// The kernels are 120-220 KB of instructions, more than an SM's instruction
+// cache holds, and a warp runs most of them once per entry: warps at different
+// places of the code evict each other's instructions (ncu: 27.7 cycles of
+// `no_instruction` stall per issue on a textured scene, 0.08 issued per cycle
+// and scheduler). So the warps of an SM are kept together: one block of 16
+// warps per SM shades several lanes at 128 registers, with a barrier at the
+// top of each iteration and one before the BSDF sample. Shade time per frame
+// (800x450 4 spp textured / 639x361 8 spp, seven lights / 1920x1080 16 spp,
+// 1M triangles): blocks of 128 without barriers 8.2 / 2.7 / 29.3 ms; with a
+// barrier per iteration 6.0 / 2.4 / 25.2; one block of 512 with both barriers
+// 2.7 / 1.5 / 23.3. Blocks of 768 (80 registers) 2.7 / 1.7 / 25.5, of 640
+// 2.9 / 1.6 / 27.1; two barriers more change nothing. Entries of one lane are
+// few and scattered: smaller blocks (glass scene 27.5 ms; 28.8 in one block
+// of 384).
+template <int kLanes, bool kFull>
+constexpr int shadeThreads()
+{
+    return kLanes == 3 ? 512 : (kFull ? 128 : 256);
+}
+template <int kLanes, bool kFull, bool kLit>
 constexpr int shadeMinBlocks()
 {
-    // Resident blocks of 128 threads per SM the lit variants are compiled for.
-    if (!kLit) return 1;
-    if (kLanes == 3) return kFull ? 3 : 5;
-    return kFull ? 4 : 6;
+    if (kLanes == 3) return 1;
+    return kFull ? (kLit ? 4 : 1) : (kLit ? 3 : 1);
 }
 
 template <int kLanes, bool kFull, bool kLit, bool kCache, int kWalk>
-__global__ void __launch_bounds__(128, shadeMinBlocks<kLanes, kFull, kLit, kCache, kWalk>())
+__global__ void __launch_bounds__((shadeThreads<kLanes, kFull>()), (shadeMinBlocks<kLanes, kFull, kLit>()))
     shadeKernel(DeviceScene s, FrameConst f, PathBuffers p, uint32_t bounce, const uint32_t* queue,
                 const uint32_t* count, uint32_t* nextQueue, unsigned long long* nextCount)
 {
@@ -173,13 +192,15 @@ __global__ void __launch_bounds__(128, shadeMinBlocks<kLanes, kFull, kLit, kCach
             }
             __syncthreads();
         }
-        const uint32_t i = blockBase + threadIdx.x;
-        if (i >= n) continue;
+        __syncthreads();  // the block's warps together (see shadeThreads)
+        // A thread without an entry follows another's, with no lane of its own:
+        // every thread of the block reaches every barrier.
+        const uint32_t i = min(blockBase + threadIdx.x, n - 1u);
         const uint32_t entry = queue[i];
         const uint32_t group = entry >> 3;
         const uint32_t slot = entryLeader(entry);  // the leader's
         // Component k of a V is lane k of the group, or the one lane there is.
-        const uint32_t mask = kLanes == 3 ? entry & 7u : 1u;
+        uint32_t mask = blockBase + threadIdx.x >= n ? 0u : (kLanes == 3 ? entry & 7u : 1u);
         const uint32_t first = kLanes == 3 ? group * 3u : slot;
         const float4 ray0 = p.ray[2u * slot], ray1 = p.ray[2u * slot + 1u];
         float3 rayOrigin = xyz(ray0);
@@ -218,7 +239,7 @@ __global__ void __launch_bounds__(128, shadeMinBlocks<kLanes, kFull, kLit, kCach
                     }
                     p.hitQueue[appendIndex(p.counters + kCountSingles)] = (group << 3) | (1u << k);
                 }
-                continue;
+                mask = 0u;
             }
         }
         V radiance, throughput, previousBsdfPdf, previousEnvironmentLightPdf;
@@ -321,7 +342,7 @@ __global__ void __launch_bounds__(128, shadeMinBlocks<kLanes, kFull, kLit, kCach
             const float3 hit = rayOrigin + rayDirection * distance;
             if (insideMedium) {
                 // :1279-1295
-                if (kLanes == 1 && at(mediumScattering, 0) > 0.0f) {
+                if (kLanes == 1 && mask != 0u && at(mediumScattering, 0) > 0.0f) {
                     const float scatterDistance = -glog(gmax(1.0f - randomFloat(rng), 1e-6f)) / at(mediumScattering, 0);
                     if (scatterDistance < distance) {
                         throughput = throughput * V(gexp(-at(mediumAbsorption, 0) * scatterDistance));
@@ -332,7 +353,7 @@ __global__ void __launch_bounds__(128, shadeMinBlocks<kLanes, kFull, kLit, kCach
                             advance(mask, rayOrigin, rayDirection, rng,
                                     kFlagEnvironmentOnMiss | kFlagPreviousWasDelta | kFlagInsideMedium, false, throughput,
                                     V(0.0f), previousEnvironmentLightPdf);
-                        continue;
+                        mask = 0u;
                     }
                 }
 #pragma unroll
@@ -373,7 +394,7 @@ __global__ void __launch_bounds__(128, shadeMinBlocks<kLanes, kFull, kLit, kCach
             const float3 tangent = surfaceTangent(normal, p0, p1, p2, uv0, uv1, uv2);
             // (A replay re-shades a bounce whose first pass went past this
             // point without ending the path and has recorded its vertex.)
-            if constexpr (kCache && !kReplay) {
+            if constexpr (kCache && !kReplay) if (mask != 0u) {
                 const bool training = (flags & kFlagTraining) != 0u;
                 bool terminate = bounce >= p.cache.prefixBounces;
                 if (p.cache.spreadFactor > 0.0f) {
@@ -416,7 +437,7 @@ __global__ void __launch_bounds__(128, shadeMinBlocks<kLanes, kFull, kLit, kCach
                         p.cache.querySlot[j] = slot;
                         p.throughput[slot] = throughput;
                         p.radiance[slot] = radiance;
-                        continue;
+                        mask = 0u;
                     }
                 }
             }
@@ -440,7 +461,7 @@ __global__ void __launch_bounds__(128, shadeMinBlocks<kLanes, kFull, kLit, kCach
                 const float4 t = materialTexture<kFull>(lodBase, s, material->textureIndices1.z, surfaceUv, f4(transmissionColorRgb, 1.0f));
                 transmissionColorRgb = f3(t.x, t.y, t.z);
             }
-            const V transmissionColor = kFull ? reflectanceSpectrum(transmissionColorRgb, spec) : V(0.0f);
+            const V transmissionColor = kFull ? weightedReflectance(transmission, transmissionColorRgb, spec) : V(0.0f);
             float subsurface = 0.0f;
             V diffuseColor = baseColor;
             float3 subsurfaceColorRgb = xyz(material->subsurfaceColor);
@@ -501,7 +522,7 @@ __global__ void __launch_bounds__(128, shadeMinBlocks<kLanes, kFull, kLit, kCach
                       : 0.0f;
             const float4 sheenColorSample = materialTexture<kFull>(lodBase, s, material->textureIndices2.w, surfaceUv,
                                                                   f4(xyz(material->sheenColorMode), 1.0f));
-            const V sheenColor = kFull ? reflectanceSpectrum(f3(sheenColorSample.x, sheenColorSample.y, sheenColorSample.z), spec) : V(0.0f);
+            const V sheenColor = kFull ? weightedReflectance(sheen, f3(sheenColorSample.x, sheenColorSample.y, sheenColorSample.z), spec) : V(0.0f);
             const float sheenRoughness = clampf(
                 materialTexture<kFull>(lodBase, s, material->textureIndices4.y, surfaceUv, f4(material->transmissionScatter.w)).x, 0.01f, 1.0f);
             const bool sheenZeltner = material->sheenColorMode.w > 0.5f;
@@ -509,7 +530,7 @@ __global__ void __launch_bounds__(128, shadeMinBlocks<kLanes, kFull, kLit, kCach
                 materialTexture<kFull>(lodBase, s, material->textureIndices5.x, surfaceUv, f4(material->translucentColorWeight.w)).x, 0.0f, 1.0f);
             const float4 translucentSample = materialTexture<kFull>(lodBase, s, material->textureIndices5.y, surfaceUv,
                                                                    f4(xyz(material->translucentColorWeight), 1.0f));
-            const V translucentColor = kFull ? reflectanceSpectrum(f3(translucentSample.x, translucentSample.y, translucentSample.z), spec) : V(0.0f);
+            const V translucentColor = kFull ? weightedReflectance(translucentWeight, f3(translucentSample.x, translucentSample.y, translucentSample.z), spec) : V(0.0f);
 
             const float3 viewDirection = normalize(-rayDirection);
             const float nDotView = gmax(dot(normal, viewDirection), 0.0f);
@@ -594,7 +615,8 @@ __global__ void __launch_bounds__(128, shadeMinBlocks<kLanes, kFull, kLit, kCach
                            offsetSurfaceOrigin(hit, orientedGeometricNormal, direction), direction, traceDistance);
             };
             uint32_t open = mask;
-            do {
+#pragma unroll 1
+            while (open != 0u) {
             uint32_t lanes = open;
             uint32_t lightRng = rng;
             if (lightCount > 0u) {
@@ -775,14 +797,16 @@ __global__ void __launch_bounds__(128, shadeMinBlocks<kLanes, kFull, kLit, kCach
             for (int k = 0; k < kLanes; ++k)
                 if (lanes >> k & 1u) put(rngAfter, k, lightRng);
             open &= ~lanes;
-            } while (kLanes == 3 && open != 0u);
+            }
 
             if (!kReplay) storeRadiance();
-            if (lastBounce) continue;
+            if (lastBounce) continue;  // the same for every thread
+            __syncthreads();
 
             // The BSDF sample, one pass per part of lanes that decide alike.
             open = mask;
-            do {
+#pragma unroll 1
+            while (open != 0u) {
             const int lead = kLanes == 3 ? static_cast<int>(firstLane(open)) : 0;
             uint32_t lanes = open;
             uint32_t state = at(rngAfter, lead);
@@ -966,7 +990,7 @@ __global__ void __launch_bounds__(128, shadeMinBlocks<kLanes, kFull, kLit, kCach
                 }
             }
             if (alive != 0u) advance(alive, origin, direction, state, newFlags, coneKept, weight, bsdfPdf, lightPdf);
-            } while (kLanes == 3 && open != 0u);
+            }
     }
 }
 

@@ -75,6 +75,14 @@ HDCX_D V reflectanceSpectrum(float3 rgb, const SpectrumOf<V>& s)
 {
     return clampf(reconstructRgb(rgb, s), 0.0f, 1.0f);
 }
+// reflectanceSpectrum of a colour that `weight` multiplies: a zero weight takes
+// any finite colour to the same zero, so the spectrum is not built for it.
+template <class V>
+HDCX_D V weightedReflectance(float weight, float3 rgb, const SpectrumOf<V>& s)
+{
+    if (weight == 0.0f && fabsf(rgb.x) < INFINITY && fabsf(rgb.y) < INFINITY && fabsf(rgb.z) < INFINITY) return V(0.0f);
+    return reflectanceSpectrum(rgb, s);
+}
 template <class V>
 HDCX_D V illuminantSpectrum(float3 rgb, const SpectrumOf<V>& s)
 {
@@ -168,6 +176,7 @@ HDCX_D float4 sampleMipBilinear(const TexDesc& t, uint32_t level, float2 uv)
 {
     const float4* m = t.mips;
     uint32_t w = t.width, h = t.height;
+#pragma unroll 1
     for (uint32_t k = 1; k <= level; ++k) {
         const uint32_t nw = max(1u, w >> 1), nh = max(1u, h >> 1);
         if (k < level) m += size_t(nw) * nh;
@@ -465,7 +474,7 @@ HDCX_D float sheenImageworksResponse(float3 normal, float3 viewDirection, float3
     return brdf * nDotL;
 }
 
-HDCX_D float sheenZeltnerDirectionalAlbedo(float nDotV, float roughness)
+HDCX_NOINLINE float sheenZeltnerDirectionalAlbedo(float nDotV, float roughness)
 {
     // :448-460
     const float x = clampf(nDotV, 0.0f, 1.0f);
@@ -477,7 +486,7 @@ HDCX_D float sheenZeltnerDirectionalAlbedo(float nDotV, float roughness)
                   0.0f, 1.0f);
 }
 
-HDCX_D float sheenResponse(float3 normal, float3 viewDirection, float3 lightDirection, float roughness, bool zeltner)
+HDCX_NOINLINE float sheenResponse(float3 normal, float3 viewDirection, float3 lightDirection, float roughness, bool zeltner)
 {
     // :462-471
     if (!zeltner) return sheenImageworksResponse(normal, viewDirection, lightDirection, roughness);
@@ -499,8 +508,9 @@ HDCX_D float eonDirectionalAlbedo(float nDotDirection, float roughness)
     return clampf(a + roughness * a * g / kPi, 0.0f, 1.0f);
 }
 
+// Models other than Lambert are rare and long: not inlined.
 template <class V>
-HDCX_D V evaluateDiffuseReflection(float3 normal, float3 viewDirection, float3 lightDirection, V diffuseColor,
+HDCX_NOINLINE V evaluateDiffuseReflection(float3 normal, float3 viewDirection, float3 lightDirection, V diffuseColor,
                                    float roughness, uint32_t model)
 {
     // :946-1009
@@ -590,14 +600,18 @@ HDCX_D V evaluateDirectSurface(const ShadingFrame& f, const LobeTerms& t, float3
     const float wrappedNdotL = gmax((t.signedNdotL + 0.5f * p.subsurface) / (1.0f + 0.5f * p.subsurface), 0.0f);
     if (wrappedNdotL <= 0.0f && t.nDotL <= 0.0f && backNdotL * p.translucentWeight <= 0.0f) return V(0.0f);
     const V baseFresnel = fresnelSchlick(t.vDotH, p.f0);
-    const V diffuseResponse = mix(evaluateDiffuseReflection(f.normal, f.view, lightDirection, p.diffuseColor,
-                                                            p.diffuseRoughness, p.diffuseModel),
-                                  V(wrappedNdotL / kPi), p.subsurface);
+    V reflection = V(t.nDotL <= 0.0f || f.nDotV <= 0.0f ? 0.0f : t.cosine);
+    if (p.diffuseModel != 0u)
+        reflection = evaluateDiffuseReflection(f.normal, f.view, lightDirection, p.diffuseColor, p.diffuseRoughness, p.diffuseModel);
+    const V diffuseResponse = mix(reflection, V(wrappedNdotL / kPi), p.subsurface);
     const V diffuse = V(diffuseScale) * (V(1.0f) - baseFresnel) * V(p.diffuseWeight) * V(1.0f - p.translucentWeight) *
                       V(1.0f - p.metalness) * p.diffuseColor * diffuseResponse * V(1.0f - p.transmission);
-    const V viewFresnel = fresnelSchlick(f.nDotV, p.f0);
-    const V translucent = V(diffuseScale) * (V(1.0f) - viewFresnel) * V(p.translucentWeight) * V(1.0f - p.metalness) *
-                          p.translucentColor * V(backNdotL / kPi) * V(1.0f - p.transmission);
+    V translucent = V(0.0f);  // a zero weight multiplies finite terms
+    if (p.translucentWeight != 0.0f || !(fabsf(diffuseScale) < INFINITY)) {
+        const V viewFresnel = fresnelSchlick(f.nDotV, p.f0);
+        translucent = V(diffuseScale) * (V(1.0f) - viewFresnel) * V(p.translucentWeight) * V(1.0f - p.metalness) *
+                      p.translucentColor * V(backNdotL / kPi) * V(1.0f - p.transmission);
+    }
     const V specular = V(specularScale * t.nDotL) * evaluateGGXAnisotropic(f, t, lightDirection, f.alpha, f.maskView, t.d, p.f0);
     V coatFresnel = V(0.0f);
     V coatSpecular = V(0.0f);
@@ -817,6 +831,7 @@ HDCX_D int cdfSearch(const float* values, const float* skip, int n, float target
 {
     int low = 0;
     int high = (n + 31) / 32 - 1;
+#pragma unroll 1
     while (low < high) {
         const int middle = (low + high) / 2;
         if (target <= __ldg(skip + middle)) high = middle;
@@ -824,6 +839,7 @@ HDCX_D int cdfSearch(const float* values, const float* skip, int n, float target
     }
     high = min(low * 32 + 31, n - 1);
     low = low * 32;
+#pragma unroll 1
     while (low < high) {
         const int middle = (low + high) / 2;
         if (target <= __ldg(values + middle)) high = middle;
@@ -859,6 +875,7 @@ HDCX_D void sampleDomeLight(const DeviceScene& s, const GpuLight& light, uint32_
     } else {
         int low = 0;
         int high = h - 1;
+#pragma unroll 1
         while (low < high) {
             const int middle = (low + high) / 2;
             const float cdf = __ldg(&texels[static_cast<size_t>(middle) * t.width].y);
@@ -870,6 +887,7 @@ HDCX_D void sampleDomeLight(const DeviceScene& s, const GpuLight& light, uint32_
         low = 0;
         high = w - 1;
         const float4* rowTexels = texels + static_cast<size_t>(row) * t.width;
+#pragma unroll 1
         while (low < high) {
             const int middle = (low + high) / 2;
             const float cdf = __ldg(&rowTexels[middle].x);
@@ -961,6 +979,7 @@ HDCX_D void sampleAnalyticLight(uint32_t lightCount, const GpuLight* lights, con
     V chosen = V(0.0f);
     uint32_t open = 0u;  // lanes still without a light (second pass)
     total = V(0.0f);
+#pragma unroll 1
     for (uint32_t step = 0; step < 2u * lightCount; ++step) {
         const bool picking = step >= lightCount;
         const uint32_t index = picking ? step - lightCount : step;
@@ -1010,6 +1029,7 @@ HDCX_NOINLINE V environmentLightPdf(const TexDesc* textures, uint32_t textureCou
 {
     // :739-758
     V pdf = V(0.0f);
+#pragma unroll 1
     for (uint32_t index = 0; index < lightCount; ++index) {
         const GpuLight& light = lights[index];
         if (light.textureInfo.z == 0u) {

@@ -9,7 +9,9 @@ namespace {
 template <int kLanes, bool kFull, bool kLit, bool kCache, int kWalk>
 void launch(const ShadeLaunch& l)
 {
-    shadeKernel<kLanes, kFull, kLit, kCache, kWalk><<<l.grid, 128, 0, l.stream>>>(l.scene, l.frame, l.paths, l.bounce, l.queue,
+    constexpr int kThreads = shadeThreads<kLanes, kFull>();
+    const int grid = (l.grid * 128 + kThreads - 1) / kThreads;
+    shadeKernel<kLanes, kFull, kLit, kCache, kWalk><<<grid, kThreads, 0, l.stream>>>(l.scene, l.frame, l.paths, l.bounce, l.queue,
                                                                                   l.count, l.nextQueue, l.nextCount);
 }
 
