@@ -8,57 +8,75 @@
 namespace hdcx {
 namespace {
 
-template <int kInst = -1>
-__device__ bool traceOpaqueBoundary(const DeviceScene& s, PathBuffers& p, float3 origin, float3 direction,
-                                    float3& boundary, float3& boundaryNormal, float& boundaryDistance)
+// A walk under way: one boundary ray per step, at most kWalkSteps of them.
+constexpr int kWalkSteps = 8;
+struct SubsurfaceWalk {
+    float3 origin, direction;
+    float sigmaS, sigmaA, anisotropy;
+    float attenuation;
+    uint32_t rng;
+    int step;
+};
+
+enum : int { kWalkContinues = 0, kWalkExits = 1, kWalkFails = 2 };
+
+HDCX_D SubsurfaceWalk beginWalk(float3 entry, float3 outwardNormal, float meanFreePath, float albedo, float anisotropy, uint32_t rng)
 {
-    // :1130-1151
-    atomicAdd(p.stats + 2, 1ull);
-    HitRecord h;
-    uint32_t fault = 0u;
-    const bool found = traceRay<Accept::Opaque, false, false, kInst>(s, origin, direction, 0.001f, 10000.0f, 0u, h, fault);
-    if (fault != 0u) atomicOr(reinterpret_cast<unsigned int*>(p.stats + 7), fault);
-    if (!found) return false;
-    const uint32_t primitive = h.primitive;
-    const float3 p0 = xyz(__ldg(s.vertices + __ldg(s.indices + primitive * 3u + 0u)));
-    const float3 p1 = xyz(__ldg(s.vertices + __ldg(s.indices + primitive * 3u + 1u)));
-    const float3 p2 = xyz(__ldg(s.vertices + __ldg(s.indices + primitive * 3u + 2u)));
-    boundaryDistance = h.t;
-    boundary = origin + direction * boundaryDistance;
-    boundaryNormal = normalize(cross(p1 - p0, p2 - p0));
-    if (dot(boundaryNormal, direction) > 0.0f) boundaryNormal = -boundaryNormal;
-    return true;
+    // :1153-1160
+    SubsurfaceWalk w;
+    const float radius = gmax(meanFreePath, 0.001f);
+    w.sigmaS = 1.0f / radius;
+    w.sigmaA = -glog(clampf(albedo, 0.001f, 0.9999f)) / radius;
+    w.origin = entry - outwardNormal * 0.003f;
+    w.rng = rng;
+    w.direction = cosineHemisphere(-outwardNormal, w.rng);
+    w.anisotropy = anisotropy;
+    w.attenuation = 1.0f;
+    w.step = 0;
+    return w;
 }
 
+// One step (:1161-1186): the boundary ray (:1130-1151; an escaping one ends
+// the walk), then a scattering event or the exit, whose ray is left in
+// origin and direction.
 template <int kInst = -1>
-__device__ bool randomWalkSubsurface(const DeviceScene& s, PathBuffers& p, float3 entry, float3 outwardNormal,
-                                     float meanFreePath, float albedo, float anisotropy, uint32_t& state,
-                                     float3& exitOrigin, float3& exitDirection, float& attenuation)
+__device__ __forceinline__ int stepWalk(const DeviceScene& s, SubsurfaceWalk& w, uint32_t& fault)
 {
-    // :1153-1186
-    const float radius = gmax(meanFreePath, 0.001f);
-    const float sigmaS = 1.0f / radius;
-    const float sigmaA = -glog(clampf(albedo, 0.001f, 0.9999f)) / radius;
-    float3 origin = entry - outwardNormal * 0.003f;
-    float3 direction = cosineHemisphere(-outwardNormal, state);
-    attenuation = 1.0f;
-    for (int step = 0; step < 8; ++step) {
-        float3 boundary, boundaryNormal;
-        float boundaryDistance;
-        if (!traceOpaqueBoundary<kInst>(s, p, origin, direction, boundary, boundaryNormal, boundaryDistance)) return false;
-        const float scatterDistance = -glog(gmax(1.0f - randomFloat(state), 1e-6f)) / sigmaS;
-        const bool forceExit = step == 7;
-        const float travel = forceExit ? boundaryDistance : gmin(scatterDistance, boundaryDistance);
-        attenuation = attenuation * gexp(-sigmaA * travel);
-        if (forceExit || scatterDistance >= boundaryDistance) {
-            exitDirection = direction;
-            exitOrigin = boundary + direction * 0.003f;
-            return true;
-        }
-        origin = origin + direction * scatterDistance;
-        direction = sampleHenyeyGreenstein(direction, anisotropy, state);
+    HitRecord h;
+    if (!traceRay<Accept::Opaque, false, false, kInst>(s, w.origin, w.direction, 0.001f, 10000.0f, 0u, h, fault)) return kWalkFails;
+    const float boundaryDistance = h.t;
+    const float scatterDistance = -glog(gmax(1.0f - randomFloat(w.rng), 1e-6f)) / w.sigmaS;
+    const bool forceExit = w.step == kWalkSteps - 1;
+    const float travel = forceExit ? boundaryDistance : gmin(scatterDistance, boundaryDistance);
+    w.attenuation = w.attenuation * gexp(-w.sigmaA * travel);
+    if (forceExit || scatterDistance >= boundaryDistance) {
+        w.origin = (w.origin + w.direction * boundaryDistance) + w.direction * 0.003f;
+        return kWalkExits;
     }
-    return false;
+    w.origin = w.origin + w.direction * scatterDistance;
+    w.direction = sampleHenyeyGreenstein(w.direction, w.anisotropy, w.rng);
+    ++w.step;
+    return kWalkContinues;
+}
+
+// A whole walk in one call, for renders without walk buffers.
+__device__ inline bool randomWalkSubsurface(const DeviceScene& s, PathBuffers& p, float3 entry, float3 outwardNormal,
+                                            float meanFreePath, float albedo, float anisotropy, uint32_t& state,
+                                            float3& exitOrigin, float3& exitDirection, float& attenuation)
+{
+    SubsurfaceWalk w = beginWalk(entry, outwardNormal, meanFreePath, albedo, anisotropy, state);
+    uint32_t fault = 0u;
+    int result;
+    do {
+        result = stepWalk(s, w, fault);
+    } while (result == kWalkContinues);
+    atomicAdd(p.stats + 2, static_cast<unsigned long long>(w.step + 1));
+    if (fault != 0u) atomicOr(reinterpret_cast<unsigned int*>(p.stats + 7), fault);
+    state = w.rng;
+    exitOrigin = w.origin;
+    exitDirection = w.direction;
+    attenuation = w.attenuation;
+    return result == kWalkExits;
 }
 
 }  // namespace

@@ -167,36 +167,54 @@ __global__ void __launch_bounds__(128, HDCX_TRACE_MIN_BLOCKS) extendKernel(Devic
 // a walk whose boundary ray escapes stores its RNG state and queues the path
 // for shadeKernel<..., kWalkReplay>, which finishes the bounce the inline way.
 // ---------------------------------------------------------------------------
+//
+// A thread steps one walk at a time and takes the next when its walk ends, so
+// every iteration of a warp traces a boundary ray per thread: walks end after
+// one to eight rays, and a thread per walk left most of a warp waiting for its
+// longest one.
 template <int kInst>
 __global__ void __launch_bounds__(128, HDCX_TRACE_MIN_BLOCKS)
     walkKernel(DeviceScene s, PathBuffers p, const uint32_t* walks, uint32_t* nextQueue, unsigned long long* nextCount,
                uint32_t* replayQueue)
 {
     const uint32_t n = p.counters[kCountWalks];
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const uint32_t slot = walks[i];
-        const float4 entry = p.walkEntry[slot];
-        const float4 outward = p.walkNormal[slot];
+    uint32_t rays = 0u, fault = 0u;
+    uint32_t slot = 0u;
+    bool walking = false;
+    SubsurfaceWalk w;
+    for (;;) {
+        if (!walking) {
+            const uint32_t i = appendIndex(p.counters + kCountWalkNext);
+            if (i >= n) break;
+            slot = walks[i];
+            const float4 entry = p.walkEntry[slot];
+            const float4 outward = p.walkNormal[slot];
+            const float4 state = p.walkState[slot];
+            w = beginWalk(xyz(entry), xyz(outward), entry.w, outward.w, state.x, __float_as_uint(state.y));
+            walking = true;
+        }
+        ++rays;
+        const int result = stepWalk<kInst>(s, w, fault);
+        if (result == kWalkContinues) continue;
+        walking = false;
         const float4 state = p.walkState[slot];
-        uint32_t rng = __float_as_uint(state.y);
-        float3 exitOrigin, exitDirection;
-        float attenuation;
-        if (randomWalkSubsurface<kInst>(s, p, xyz(entry), xyz(outward), entry.w, outward.w, state.x, rng, exitOrigin,
-                                 exitDirection, attenuation)) {
+        const uint32_t lane = 1u << (slot % 3u);
+        if (result == kWalkExits) {
             const uint32_t flags = kFlagEnvironmentOnMiss | kFlagPreviousWasDelta |
                                    (__float_as_uint(p.ray[2u * slot + 1u].w) & (kFlagInsideMedium | kFlagTraining));
-            p.throughput[slot] = state.z * attenuation;
+            p.throughput[slot] = state.z * w.attenuation;
             p.previousPdf[slot] = make_float2(0.0f, p.previousPdf[slot].y);
-            p.ray[2u * slot] = make_float4(exitOrigin.x, exitOrigin.y, exitOrigin.z, __uint_as_float(rng));
-            p.ray[2u * slot + 1u] = make_float4(exitDirection.x, exitDirection.y, exitDirection.z, __uint_as_float(flags));
+            p.ray[2u * slot] = make_float4(w.origin.x, w.origin.y, w.origin.z, __uint_as_float(w.rng));
+            p.ray[2u * slot + 1u] = make_float4(w.direction.x, w.direction.y, w.direction.z, __uint_as_float(flags));
             if (p.cone != nullptr) p.cone[slot] = make_float2(0.0f, -1.0f);
-            const uint32_t lane = 1u << (slot % 3u);
             nextQueue[appendEntry(nextCount, lane)] = ((slot / 3u) << 3) | lane;
         } else {
-            p.walkState[slot] = make_float4(state.x, __uint_as_float(rng), state.z, 0.0f);
-            replayQueue[appendIndex(p.counters + kCountReplays)] = ((slot / 3u) << 3) | (1u << (slot % 3u));
+            p.walkState[slot] = make_float4(state.x, __uint_as_float(w.rng), state.z, 0.0f);
+            replayQueue[appendIndex(p.counters + kCountReplays)] = ((slot / 3u) << 3) | lane;
         }
     }
+    if (rays != 0u) atomicAdd(p.stats + 2, static_cast<unsigned long long>(rays));
+    if (fault != 0u) atomicOr(reinterpret_cast<unsigned int*>(p.stats + 7), fault);
 }
 
 // ---------------------------------------------------------------------------

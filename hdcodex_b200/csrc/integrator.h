@@ -51,6 +51,7 @@ enum : uint32_t {
     kCountMisses = 6,
     kCountWalks = 7,     // deferred subsurface walks
     kCountReplays = 8,   // failed walks to re-shade
+    kCountWalkNext = 9,  // walks taken by walkKernel's threads
     kCountQueue1 = 10,   // 64-bit: extension queue of odd bounces
     kCountEnd = 12,
 };
