@@ -324,6 +324,14 @@ __device__ void nodeFrame(float4 lo, float4 hi, float sceneScale, float origin[3
     }
 }
 
+// The steps of nodeFrame (biased exponents) as the node stores them.
+__device__ void setSteps(WideNode& node, const uint8_t biased[3])
+{
+    node.scaleX = static_cast<uint16_t>(biased[0] << 7);
+    node.scaleY = static_cast<uint16_t>(biased[1] << 7);
+    node.scaleZ = __uint_as_float(static_cast<uint32_t>(biased[2]) << 23);
+}
+
 // A child box [cl, ch] on the node's grid, padded by one step on every side.
 __device__ void quantizeChild(float4 cl, float4 ch, const float origin[3], const double step[3], uint8_t ql[3],
                               uint8_t qh[3])
@@ -462,16 +470,13 @@ __global__ void collapseKernel(CollapseArgs a, const CollapseItem* items, uint32
     node.px = origin[0];
     node.py = origin[1];
     node.pz = origin[2];
-    node.ex = biased[0];
-    node.ey = biased[1];
-    node.ez = biased[2];
-    node.imask = 0;
+    setSteps(node, biased);
     node.childBase = childBase;
     node.triBase = triBase;
+    node.masks = 0u;
     int internalRank = 0, triOffset = 0;
     for (int s = 0; s < 8; ++s) {
         const int i = entryOfSlot[s];
-        node.meta[s] = 0;
         node.qlox[s] = node.qloy[s] = node.qloz[s] = 0;
         node.qhix[s] = node.qhiy[s] = node.qhiz[s] = 0;
         if (i < 0) continue;
@@ -481,8 +486,7 @@ __global__ void collapseKernel(CollapseArgs a, const CollapseItem* items, uint32
         node.qlox[s] = ql[0]; node.qloy[s] = ql[1]; node.qloz[s] = ql[2];
         node.qhix[s] = qh[0]; node.qhiy[s] = qh[1]; node.qhiz[s] = qh[2];
         if (isInternal(b)) {
-            node.imask |= static_cast<uint8_t>(1u << s);
-            node.meta[s] = 0;  // internal children carry no triangle bits
+            node.masks |= 1u << (24 + s);
             const uint32_t slot = atomicAdd(nextCount, 1u);
             nextItems[slot] = CollapseItem{b, childBase + static_cast<uint32_t>(internalRank), item.depth + 1u, 0u};
             internalRank++;
@@ -511,7 +515,7 @@ __global__ void collapseKernel(CollapseArgs a, const CollapseItem* items, uint32
                 }
             }
             const uint32_t unary = written >= 3 ? 7u : (written == 2 ? 3u : 1u);
-            node.meta[s] = static_cast<uint8_t>((unary << 5) | static_cast<uint32_t>(triOffset));
+            node.masks |= unary << (3 * s);
             triOffset += written;
         }
     }
@@ -554,13 +558,13 @@ __global__ void refitLevelKernel(WideNode* nodes, const float4* triVerts, float4
     uint32_t present = 0u;
     float4 lo = make_float4(INFINITY, INFINITY, INFINITY, 0.0f), hi = make_float4(-INFINITY, -INFINITY, -INFINITY, 0.0f);
     for (int s = 0; s < 8; ++s) {
-        const uint32_t meta = node.meta[s];
-        if ((node.imask >> s) & 1u) {
-            const uint32_t child = node.childBase + __popc(node.imask & ((1u << s) - 1u));
+        const uint32_t leaf = (node.masks >> (3 * s)) & 7u;
+        if ((node.masks >> (24 + s)) & 1u) {
+            const uint32_t child = node.childBase + __popc((node.masks >> 24) & ((1u << s) - 1u));
             cl[s] = boxes[2 * child];
             ch[s] = boxes[2 * child + 1];
-        } else if (meta != 0u) {
-            const uint32_t first = node.triBase + (meta & 31u), count = __popc(meta >> 5);
+        } else if (leaf != 0u) {
+            const uint32_t first = node.triBase + __popc(node.masks & ((1u << (3 * s)) - 1u)), count = __popc(leaf);
             cl[s] = make_float4(INFINITY, INFINITY, INFINITY, 0.0f);
             ch[s] = make_float4(-INFINITY, -INFINITY, -INFINITY, 0.0f);
             for (uint32_t t = first; t < first + count; ++t) {
@@ -584,9 +588,7 @@ __global__ void refitLevelKernel(WideNode* nodes, const float4* triVerts, float4
     node.px = origin[0];
     node.py = origin[1];
     node.pz = origin[2];
-    node.ex = biased[0];
-    node.ey = biased[1];
-    node.ez = biased[2];
+    setSteps(node, biased);
     for (int s = 0; s < 8; ++s) {
         uint8_t ql[3] = {0, 0, 0}, qh[3] = {0, 0, 0};
         if ((present >> s) & 1u) quantizeChild(cl[s], ch[s], origin, step, ql, qh);

@@ -105,16 +105,17 @@ struct TexDesc {
 // 8-wide BVH node with quantised child boxes (80 bytes). The layout is the
 // compressed wide node of Ylitie, Karras and Laine, "Efficient Incoherent Ray
 // Traversal on GPUs Through Compressed Wide BVHs", HPG 2017: origin p,
-// power-of-two scale exponents, internal-child mask, base indices of the
-// internal children and of the leaf triangles, one meta byte per slot (leaf
-// children: unary triangle count << 5 | first triangle; internal and empty
-// children: 0) and six quantised planes per child.
+// power-of-two steps, internal-child mask, base indices of the
+// internal children and of the leaf triangles, a mask of the leaf triangles (three
+// bits per slot, none for internal and empty children; the triangles lie in
+// the order of their bits) and six quantised planes per child.
 struct __align__(16) WideNode {
     float px, py, pz;
-    uint8_t ex, ey, ez, imask;
+    uint16_t scaleX, scaleY;  // the steps in x and y: the upper halves of the floats (powers of two)
     uint32_t childBase;
     uint32_t triBase;
-    uint8_t meta[8];
+    uint32_t masks;    // bit 3 s + k: triangle k (of at most 3) of the leaf in slot s; bits 24..31: internal children
+    float scaleZ;      // the step in z
     uint8_t qlox[8], qloy[8], qloz[8];
     uint8_t qhix[8], qhiy[8], qhiz[8];
 };

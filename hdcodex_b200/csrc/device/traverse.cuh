@@ -20,6 +20,17 @@
 //   binary32 slab test conservative. The 48 plane distances of a node are
 //   evaluated two children at a time with the packed fused multiply-add of
 //   sm_100 (__ffma2_rn), the slab intervals with its three-input min/max.
+//   The kernels are bound by the ALU pipe, which runs at half the issue rate
+//   (byte permutes, min/max, selects and logic; 65% issue active with
+//   math_pipe_throttle and not_selected the top stalls), so the node test
+//   keeps work off it: triangle bits of the hit children come from one mask
+//   per node, spread by multiplies, instead of five operations per child
+//   (extend of 1920x1080 16 spp, 1M triangles: 36.7 -> 34.0 ms); hit bits are
+//   the sign bits of a subtraction, funnel-shifted together (34.0 -> 32.7 ms).
+//   Measured and left out: planes as half-precision pairs (33.0 -> 34.1 ms), a
+//   shared-memory table for permuteSlots (within 1%), 48 scalar instead of 24
+//   packed multiply-adds (34.0), one triangle per step (37.1) or a triangle
+//   or a node per step (38.2).
 // * Faults: a node group that finds the stack full, or a traversal that
 //   visits more nodes than the BVH holds (a malformed node array), sets a
 //   bit in the traversal's fault word; the kernels OR it into the render's
@@ -84,6 +95,21 @@ HDCX_D RayPre precomputeRay(float3 o, float3 d)
     return r;
 }
 
+// Three-input minimum and maximum of sm_100 (PTX min/max with three f32
+// operands): one instruction where two-input forms take two.
+HDCX_D float max3(float a, float b, float c)
+{
+    float r;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+HDCX_D float min3(float a, float b, float c)
+{
+    float r;
+    asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+
 HDCX_D bool intersectTriangle(const RayPre& r, float3 v0, float3 v1, float3 v2, float tmin, float tmax, float& tOut,
                               float& b1, float& b2)
 {
@@ -100,12 +126,12 @@ HDCX_D bool intersectTriangle(const RayPre& r, float3 v0, float3 v1, float3 v2, 
     float u = __fsub_rn(__fmul_rn(cx, by), __fmul_rn(cy, bx));
     float v = __fsub_rn(__fmul_rn(ax, cy), __fmul_rn(ay, cx));
     float w = __fsub_rn(__fmul_rn(bx, ay), __fmul_rn(by, ax));
-    if (u == 0.0f || v == 0.0f || w == 0.0f) {
+    if (min3(fabsf(u), fabsf(v), fabsf(w)) == 0.0f) {
         u = __double2float_rn(__dsub_rn(__dmul_rn(cx, by), __dmul_rn(cy, bx)));
         v = __double2float_rn(__dsub_rn(__dmul_rn(ax, cy), __dmul_rn(ay, cx)));
         w = __double2float_rn(__dsub_rn(__dmul_rn(bx, ay), __dmul_rn(by, ax)));
     }
-    if ((u < 0.0f || v < 0.0f || w < 0.0f) && (u > 0.0f || v > 0.0f || w > 0.0f)) return false;
+    if (min3(u, v, w) < 0.0f && max3(u, v, w) > 0.0f) return false;
     const float det = __fadd_rn(__fadd_rn(u, v), w);
     if (det == 0.0f) return false;
     const float saz = __fmul_rn(r.sz, az), sbz = __fmul_rn(r.sz, bz), scz = __fmul_rn(r.sz, cz);
@@ -133,21 +159,6 @@ HDCX_D float biasedByte(uint32_t word, int index)
 HDCX_D float2 planePair(uint32_t word, int k, float2 a, float2 c)
 {
     return __ffma2_rn(make_float2(biasedByte(word, k), biasedByte(word, k + 1)), a, c);
-}
-
-// Three-input minimum and maximum of sm_100 (PTX min/max with three f32
-// operands): one instruction where two-input forms take two.
-HDCX_D float max3(float a, float b, float c)
-{
-    float r;
-    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
-    return r;
-}
-HDCX_D float min3(float a, float b, float c)
-{
-    float r;
-    asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
-    return r;
 }
 
 // Moves bit i of an 8-bit mask to bit i ^ x (x in 0..7): three conditional
@@ -182,6 +193,7 @@ struct Traversal {
     float bestB1, bestB2;
     uint2 nodeGroup;  // x: base index of the internal children; y: hit bits in 24..31 (by visiting order) | imask
     uint2 triGroup;   // x: first triangle slot; y: bits of the triangles left to test
+    uint32_t triMask; // the node's triangle bits (see testNode)
     int sp;
     uint32_t budget;  // every node is entered at most once; guards against a malformed node array
     uint32_t rayRng;
@@ -213,6 +225,13 @@ HDCX_D void beginTraversal(Traversal& st, const DeviceScene& s, float3 o, float3
     st.fault = 0u;
 }
 
+// Slot of the first triangle of `group`: the node's triangles lie in the order
+// of their bits.
+HDCX_D uint32_t triangleSlot(uint2 group, uint32_t triMask)
+{
+    return group.x + static_cast<uint32_t>(__popc(triMask & ((group.y & (0u - group.y)) - 1u)));
+}
+
 // Tests the eight children of node `nodeIndex` against a ray (origin o,
 // inverse direction id, octant mask octInv) up to bestT: hit internal
 // children become nodeGroup (hit bits in 24..31 by visiting order | imask),
@@ -228,16 +247,14 @@ HDCX_D void beginTraversal(Traversal& st, const DeviceScene& s, float3 o, float3
 // 2^32 scene units (|a| * 2^23 below the binary32 range with |id| <= 2^80).
 template <bool kMargin>
 HDCX_D void testNode(const WideNode* nodes, uint32_t nodeIndex, float3 o, float idx, float idy, float idz,
-                     uint32_t octInv, float bestT, float mx, float my, float mz, uint2& nodeGroup, uint2& triGroup)
+                     uint32_t octInv, float bestT, float mx, float my, float mz, uint2& nodeGroup, uint2& triGroup,
+                     uint32_t& triMask)
 {
     const uint4* np = reinterpret_cast<const uint4*>(nodes + nodeIndex);
     const uint4 n0 = __ldg(np + 0), n1 = __ldg(np + 1), n2 = __ldg(np + 2), n3 = __ldg(np + 3), n4 = __ldg(np + 4);
     const float px = __uint_as_float(n0.x), py = __uint_as_float(n0.y), pz = __uint_as_float(n0.z);
-    const uint32_t e = n0.w;
-    const float scx = __uint_as_float((e & 0xffu) << 23);
-    const float scy = __uint_as_float(((e >> 8) & 0xffu) << 23);
-    const float scz = __uint_as_float(((e >> 16) & 0xffu) << 23);
-    const uint32_t imask = e >> 24;
+    const float scx = __uint_as_float(n0.w << 16), scy = __uint_as_float(n0.w & 0xffff0000u), scz = __uint_as_float(n1.w);
+    const uint32_t imask = n1.z >> 24;
     const float ax = scx * idx, ay = scy * idy, az = scz * idz;
     const float bx = (px - o.x) * idx, by = (py - o.y) * idy, bz = (pz - o.z) * idz;
     constexpr float kBias = -8388608.0f;  // -2^23
@@ -255,13 +272,10 @@ HDCX_D void testNode(const WideNode* nodes, uint32_t nodeIndex, float3 o, float 
     const uint32_t nearX0 = sx ? loX0 : hiX0, nearX1 = sx ? loX1 : hiX1, farX0 = sx ? hiX0 : loX0, farX1 = sx ? hiX1 : loX1;
     const uint32_t nearY0 = sy ? loY0 : hiY0, nearY1 = sy ? loY1 : hiY1, farY0 = sy ? hiY0 : loY0, farY1 = sy ? hiY1 : loY1;
     const uint32_t nearZ0 = sz ? loZ0 : hiZ0, nearZ1 = sz ? loZ1 : hiZ1, farZ0 = sz ? hiZ0 : loZ0, farZ1 = sz ? hiZ1 : loZ1;
-    const uint32_t meta0 = n1.z, meta1 = n1.w;
-    uint32_t hits = 0u, triHits = 0u;
-    // Children 2j and 2j+1 share a word per plane (bytes k and k+1). The meta
-    // byte of a leaf child is its unary triangle count << 5 | first triangle;
-    // internal and empty children have meta 0 and add no triangle bits.
+    uint32_t misses = 0u;
+    // Children 2j and 2j+1 share a word per plane (bytes k and k+1).
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
+    for (int j = 3; j >= 0; --j) {
         const int k = (2 * j) & 3;
         const bool low = j < 2;
         const float2 tnx = planePair(low ? nearX0 : nearX1, k, ax2, cxn2);
@@ -271,21 +285,59 @@ HDCX_D void testNode(const WideNode* nodes, uint32_t nodeIndex, float3 o, float 
         const float2 tfy = planePair(low ? farY0 : farY1, k, ay2, cyf2);
         const float2 tfz = planePair(low ? farZ0 : farZ1, k, az2, czf2);
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const int i = 2 * j + h;
-            const uint32_t metaShift = (low ? meta0 : meta1) >> (8 * (k + h));  // low 5 bits: first triangle
-            const uint32_t tris = __funnelshift_l(0u, (metaShift >> 5) & 7u, metaShift);
+        for (int h = 1; h >= 0; --h) {
             const float tNear = max3(h ? tnx.y : tnx.x, h ? tny.y : tny.x, fmaxf(h ? tnz.y : tnz.x, 0.0f));
             const float tFar = min3(h ? tfx.y : tfx.x, h ? tfy.y : tfy.x, fminf(h ? tfz.y : tfz.x, bestT));
-            if (tNear <= tFar) {
-                hits |= 1u << i;
-                triHits |= tris;
-            }
+            // The sign of the difference is the miss bit: a subtraction and a
+            // funnel shift per child.
+            misses = __funnelshift_l(__float_as_uint(tFar - tNear), misses, 1u);
         }
     }
+    const uint32_t hits = ~misses & 0xffu;
     // Internal children in visiting order: bit i goes to i ^ octInv.
     nodeGroup = make_uint2(n1.x, (permuteSlots(hits & imask, octInv) << 24) | imask);
-    triGroup = make_uint2(n1.y, triHits);
+    // Triangle bits of the hit leaf children: child c owns bits 3 c .. 3 c + 2,
+    // those it uses are set in the node's mask; the eight hit bits are spread
+    // to every third bit and filled up.
+    uint32_t spread = (hits * 257u) & 0x0000f00fu;
+    spread = (spread * 17u) & 0x000c30c3u;
+    spread = (spread * 5u) & 0x00249249u;
+    triMask = n1.z;
+    triGroup = make_uint2(n1.y, (spread * 7u) & n1.z);
+}
+
+// Tests the next triangle of the triangle group; true for kAny at a confirmed
+// candidate.
+template <Accept kMode, bool kAny, bool kCount>
+HDCX_D bool testTriangle(Traversal& st, const DeviceScene& s, uint2* work)
+{
+    const uint32_t rest = st.triGroup.y & (st.triGroup.y - 1u);
+    const uint32_t slot = triangleSlot(st.triGroup, st.triMask);
+    st.triGroup.y = rest;
+    const float4 w0 = __ldg(s.triVerts + slot * 3u + 0u);
+    const float4 w1 = __ldg(s.triVerts + slot * 3u + 1u);
+    const float4 w2 = __ldg(s.triVerts + slot * 3u + 2u);
+    if (kCount) work->y++;
+    float t, b1, b2;
+    if (!intersectTriangle(st.pre, xyz(w0), xyz(w1), xyz(w2), st.tmin, st.bestT, t, b1, b2)) return false;
+    const uint32_t prim = __float_as_uint(w0.w);
+    if (!kAny) {
+        if (t > st.bestT) return false;
+        if (t == st.bestT && prim > st.bestPrim) return false;
+    }
+    if (kMode == Accept::Stochastic) {
+        // The threshold lies in [0, 1]: an opacity of 1 always confirms.
+        const float opacity = leafOpacity(w1.w, s, prim, b1, b2);
+        if (opacity < 1.0f && !(anyHitThreshold(st.rayRng, prim) <= opacity)) return false;
+    } else if (kMode == Accept::Threshold) {
+        if (!(leafOpacity(w1.w, s, prim, b1, b2) >= 0.5f)) return false;
+    }
+    if (kAny) return true;
+    st.bestT = t;
+    st.bestPrim = prim;
+    st.bestB1 = b1;
+    st.bestB2 = b2;
+    return false;
 }
 
 // One traversal step: the triangles of the current triangle group, then one
@@ -297,32 +349,7 @@ template <Accept kMode, bool kAny, bool kCount = false>
 HDCX_D int traversalStep(Traversal& st, uint2* stack, const DeviceScene& s, uint2* work)
 {
     while (st.triGroup.y != 0u) {
-        const int bit = __ffs(st.triGroup.y) - 1;
-        st.triGroup.y &= st.triGroup.y - 1u;
-        const uint32_t slot = st.triGroup.x + static_cast<uint32_t>(bit);
-        const float4 w0 = __ldg(s.triVerts + slot * 3u + 0u);
-        const float4 w1 = __ldg(s.triVerts + slot * 3u + 1u);
-        const float4 w2 = __ldg(s.triVerts + slot * 3u + 2u);
-        if (kCount) work->y++;
-        float t, b1, b2;
-        if (!intersectTriangle(st.pre, xyz(w0), xyz(w1), xyz(w2), st.tmin, st.bestT, t, b1, b2)) continue;
-        const uint32_t prim = __float_as_uint(w0.w);
-        if (!kAny) {
-            if (t > st.bestT) continue;
-            if (t == st.bestT && prim > st.bestPrim) continue;
-        }
-        if (kMode == Accept::Stochastic) {
-            // The threshold lies in [0, 1]: an opacity of 1 always confirms.
-            const float opacity = leafOpacity(w1.w, s, prim, b1, b2);
-            if (opacity < 1.0f && !(anyHitThreshold(st.rayRng, prim) <= opacity)) continue;
-        } else if (kMode == Accept::Threshold) {
-            if (!(leafOpacity(w1.w, s, prim, b1, b2) >= 0.5f)) continue;
-        }
-        if (kAny) return kStepAnyHit;
-        st.bestT = t;
-        st.bestPrim = prim;
-        st.bestB1 = b1;
-        st.bestB2 = b2;
+        if (testTriangle<kMode, kAny, kCount>(st, s, work)) return kStepAnyHit;
     }
     if ((st.nodeGroup.y & 0xff000000u) == 0u) {
         if (st.sp == 0) return kStepDone;
@@ -346,7 +373,7 @@ HDCX_D int traversalStep(Traversal& st, uint2* stack, const DeviceScene& s, uint
 
     if (kCount) work->x++;
     testNode<false>(s.nodes, nodeIndex, st.pre.o, st.idx, st.idy, st.idz, st.octInv, st.bestT, 0.0f, 0.0f, 0.0f,
-                    st.nodeGroup, st.triGroup);
+                    st.nodeGroup, st.triGroup, st.triMask);
     return kStepContinue;
 }
 
@@ -448,13 +475,13 @@ HDCX_D bool traceInstance(const DeviceScene& s, const RayPre& pre, float3 o, flo
     const float mx = margin * fabsf(id.x), my = margin * fabsf(id.y), mz = margin * fabsf(id.z);
     uint2 group = B.nodeCount == 0u ? make_uint2(0u, 0u) : make_uint2(0u, (1u << (24u + octInv)) | 1u);
     uint2 tris = make_uint2(0u, 0u);
+    uint32_t triMask = 0u;
     int sp = 0;
     uint32_t budget = B.nodeCount + 1u;
     for (;;) {
         while (tris.y != 0u) {
-            const int bit = __ffs(tris.y) - 1;
+            const uint32_t slot = triangleSlot(tris, triMask);
             tris.y &= tris.y - 1u;
-            const uint32_t slot = tris.x + static_cast<uint32_t>(bit);
             const float4 w0 = __ldg(B.triVerts + slot * 3u + 0u);
             float3 v0, v1, v2;
             uint32_t prim;
@@ -485,9 +512,9 @@ HDCX_D bool traceInstance(const DeviceScene& s, const RayPre& pre, float3 o, flo
         }
         if (kCount) work->x++;
         if (I.identity) {
-            testNode<false>(B.nodes, nodeIndex, ro, id.x, id.y, id.z, octInv, best.t, 0.0f, 0.0f, 0.0f, group, tris);
+            testNode<false>(B.nodes, nodeIndex, ro, id.x, id.y, id.z, octInv, best.t, 0.0f, 0.0f, 0.0f, group, tris, triMask);
         } else {
-            testNode<true>(B.nodes, nodeIndex, ro, id.x, id.y, id.z, octInv, best.t, mx, my, mz, group, tris);
+            testNode<true>(B.nodes, nodeIndex, ro, id.x, id.y, id.z, octInv, best.t, mx, my, mz, group, tris, triMask);
         }
     }
 }
@@ -504,13 +531,13 @@ HDCX_D bool traceInstanced(const DeviceScene& s, float3 o, float3 d, float tmin,
     uint2 stack[kTraversalStack];
     uint2 group = make_uint2(0u, (1u << (24u + octInv)) | 1u);
     uint2 leaves = make_uint2(0u, 0u);
+    uint32_t triMask = 0u;
     int sp = 0;
     uint32_t budget = s.nodeCount + 1u;
     for (;;) {
         while (leaves.y != 0u) {
-            const int bit = __ffs(leaves.y) - 1;
+            const uint32_t slot = triangleSlot(leaves, triMask);
             leaves.y &= leaves.y - 1u;
-            const uint32_t slot = leaves.x + static_cast<uint32_t>(bit);
             const uint32_t inst = __float_as_uint(__ldg(&s.triVerts[slot * 3u].w));
             if (traceInstance<kMode, kAny, kCount>(s, pre, o, d, tmin, rayRng, inst, best, stack, work, fault)) return true;
         }
@@ -521,7 +548,7 @@ HDCX_D bool traceInstanced(const DeviceScene& s, float3 o, float3 d, float tmin,
             break;
         }
         if (kCount) work->x++;
-        testNode<false>(s.nodes, nodeIndex, o, id.x, id.y, id.z, octInv, best.t, 0.0f, 0.0f, 0.0f, group, leaves);
+        testNode<false>(s.nodes, nodeIndex, o, id.x, id.y, id.z, octInv, best.t, 0.0f, 0.0f, 0.0f, group, leaves, triMask);
     }
     if (kAny || best.prim == kInvalidPrimitive) return false;
     hit.t = best.t;
