@@ -232,16 +232,15 @@ __device__ __forceinline__ float surfaceArea(float4 lo, float4 hi)
 // one triangle, A * cPrim for every i. The costs are filled bottom up (the
 // internal nodes of a clustering round only have children from earlier
 // rounds) and read top down by collapseKernel, which gives each wide node
-// the children D(n, 8) chose. cPrim = cNode was measured best among 0.3, 0.6
-// and 1.0 on the heavy and stress scenes (a wide-node test is some 200
-// instructions and a triangle test 80, but a triangle also costs three
-// 16-byte loads, the closest-hit bookkeeping and, for cutouts, an opacity
-// lookup).
+// the children D(n, 8) chose. cPrim = 2 cNode: against 1, 1.5 and 3 the glass
+// scene's extension takes 15.6 ms (16.1, 15.8, 15.6) and the one of the
+// 1M-triangle scene 32.3 ms (32.7, 32.4, 32.3); a triangle test is nearly as
+// long as a node test, and fewer threads of a warp take part in it.
 // decision[8 n + i - 1] for i = 1..7: C(n, 1): 0 leaf, 1 internal; i > 1:
 // 0 take C(n, i - 1), else the k of D(n, i); decision[8 n + 7]: the k of D(n, 8).
 // ---------------------------------------------------------------------------
 #ifndef HDCX_COLLAPSE_PRIM_COST
-#define HDCX_COLLAPSE_PRIM_COST 1.0f
+#define HDCX_COLLAPSE_PRIM_COST 2.0f
 #endif
 constexpr float kCollapseNodeCost = 1.0f;
 constexpr float kCollapsePrimCost = HDCX_COLLAPSE_PRIM_COST;

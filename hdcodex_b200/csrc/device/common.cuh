@@ -170,6 +170,7 @@ struct DeviceScene {
     uint32_t nodeCount;
     uint32_t fullShading;    // 0: no material uses textures or layered lobes (see shadeKernel)
     uint32_t hasSubsurface;  // some material can take the subsurface random walk
+    uint32_t partsLanes;     // some material transmits or scatters inside: many entries end up with one lane
     // Two-level scenes: instances, their BLASes; nodes/triVerts/nodeCount
     // are then the top-level BVH (its leaf "triangles" carry instance indices).
     const InstanceDesc* instances;  // null: single-level scene

@@ -63,10 +63,42 @@ HDCX_D V combineShadow(uint32_t kind, V a, V sv, V g1, V g2, V g3)
 // slot j.
 HDCX_D void emitShadow(PathBuffers& p, uint32_t group, uint32_t lanes, uint32_t info, float3 origin, float3 direction, float tmax)
 {
-    const uint32_t i = appendEntry(reinterpret_cast<unsigned long long*>(p.counters + kCountShadow), lanes);
+    const uint32_t i = appendEntry(reinterpret_cast<unsigned long long*>(p.counters + p.shadowWord), lanes);
     p.shadowRay[2u * i] = make_float4(origin.x, origin.y, origin.z, tmax);
     p.shadowRay[2u * i + 1u] = make_float4(direction.x, direction.y, direction.z, __uint_as_float((group << 3) | lanes));
     p.shadowInfo[i] = info;
+}
+
+// Environment on a miss (vulkan_path_tracer.cpp:1245-1255) of an entry's lanes.
+HDCX_D void shadeMiss(const DeviceScene& s, const FrameConst& f, const PathBuffers& p, uint32_t entry, uint32_t lightSlots)
+{
+    const float4 d = p.ray[2u * entryLeader(entry) + 1u];
+    const uint32_t flags = __float_as_uint(d.w);
+    const bool lit = (flags & kFlagEnvironmentOnMiss) != 0u;
+    const float3 sky = lit ? environment(s, f, xyz(d)) : f3(0.0f);
+#pragma unroll 1
+    for (uint32_t lane = 0; lane < 3u; ++lane) {
+        if (!(entry >> lane & 1u)) continue;
+        const uint32_t slot = (entry >> 3) * 3u + lane;
+        float radiance = p.radiance[slot];
+        // Light samples of the previous bounce, in slot order.
+#pragma unroll 1
+        for (uint32_t j = 0; j < lightSlots; ++j) {
+            float& pending = p.contribution[contributionIndex(slot, lightSlots, j)];
+            const float value = pending;
+            if (value != 0.0f) {
+                radiance += value;
+                pending = 0.0f;
+            }
+        }
+        if (lit) {
+            const Spectrum spec = spectrumFromBasis(p.wavelength[slot], p.spectrum[slot]);
+            const float2 previousPdf = p.previousPdf[slot];
+            const float misWeight = (flags & kFlagPreviousWasDelta) != 0u ? 1.0f : powerHeuristic(previousPdf.x, previousPdf.y);
+            radiance += p.throughput[slot] * misWeight * illuminantSpectrum(sky, spec);
+        }
+        p.radiance[slot] = radiance;
+    }
 }
 
 // kLit: the scene has analytic or dome lights and no emissive triangles, so
@@ -145,7 +177,7 @@ constexpr int shadeMinBlocks()
 template <int kLanes, bool kFull, bool kLit, bool kCache, int kWalk>
 __global__ void __launch_bounds__((shadeThreads<kLanes, kFull>()), (shadeMinBlocks<kLanes, kFull, kLit>()))
     shadeKernel(DeviceScene s, FrameConst f, PathBuffers p, uint32_t bounce, const uint32_t* queue,
-                const uint32_t* count, uint32_t* nextQueue, unsigned long long* nextCount)
+                const uint32_t* count, uint32_t* nextQueue, unsigned long long* nextCount, bool misses)
 {
     using V = std::conditional_t<kLanes == 3, Lanes3, float>;
     using U = typename LaneTraits<V>::U;
@@ -237,7 +269,7 @@ __global__ void __launch_bounds__((shadeThreads<kLanes, kFull>()), (shadeMinBloc
                         p.hit[own] = hitRec;
                         if (p.cone != nullptr) p.cone[own] = p.cone[slot];
                     }
-                    p.hitQueue[appendIndex(p.counters + kCountSingles)] = (group << 3) | (1u << k);
+                    p.hitQueue[appendIndex(p.counters + kCountHits)] = (group << 3) | (1u << k);
                 }
                 mask = 0u;
             }
@@ -992,6 +1024,12 @@ __global__ void __launch_bounds__((shadeThreads<kLanes, kFull>()), (shadeMinBloc
             if (alive != 0u) advance(alive, origin, direction, state, newFlags, coneKept, weight, bsdfPdf, lightPdf);
             }
     }
+    if (!misses) return;
+    // The bounce's misses (:1245-1255), at the end of the launch rather than in
+    // one of their own: the environment, looked up once per entry.
+    const uint32_t missCount = p.counters[kCountMisses];
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < missCount; i += gridDim.x * blockDim.x)
+        shadeMiss(s, f, p, p.missQueue[i], lightSlots);
 }
 
 }  // namespace

@@ -448,6 +448,18 @@ bool hasSubsurfaceMaterial(const PackedSceneData& d)
     return false;
 }
 
+// Whether any material has a transmission weight above zero (or NaN).
+bool hasTransmissiveMaterial(const PackedSceneData& d)
+{
+    const size_t n = d.materials.size() / HDCX_GPU_MATERIAL_BYTES;
+    for (size_t i = 0; i < n; ++i) {
+        GpuMaterial m;
+        std::memcpy(&m, d.materials.data() + i * HDCX_GPU_MATERIAL_BYTES, sizeof m);
+        if (!(m.transmissionOpacityIor.x <= 0.0F)) return true;
+    }
+    return false;
+}
+
 // Per-triangle opacity hints for the BVH's leaf copies: the opacity that
 // surfaceOpacity returns for a triangle whose material has no opacity texture
 // (the material's opacity clamped to [0, 1] as GLSL clamps, a NaN kept), -1
@@ -745,6 +757,7 @@ void uploadScene(hdcx_tracer* t, const PackedSceneData& d)
     s.opaque = d.opaque ? 1u : 0u;
     s.fullShading = needsFullShading(d) ? 1u : 0u;
     s.hasSubsurface = hasSubsurfaceMaterial(d) ? 1u : 0u;
+    s.partsLanes = s.hasSubsurface != 0u || hasTransmissiveMaterial(d) ? 1u : 0u;
     s.hasMeshLights = (d.triangleCount() > 0 && d.emissive[(size_t(d.triangleCount()) - 1) * 4u] > 0.0F) ? 1u : 0u;
     {
         // Scene box (padded by 0.1% per side) for the radiance-cache positions.

@@ -123,39 +123,110 @@ __global__ void generateKernel(FrameConst f, WaveDesc w, PathBuffers p)
 // kInst (traversal kernels): 0 single-level scenes, 1 scenes with instancers.
 //
 // One thread per entry traces the ray its lanes share: up to the first
-// decision that parts them, one traversal serves three paths.
+// decision that parts them, one traversal serves three paths. Hits and misses
+// go to separate queues, so that shading warps hold only hits; entries of
+// several lanes and of one lane have shade kernels of their own, unless the
+// scene keeps nearly all lanes together (PathBuffers::merged).
+// ---------------------------------------------------------------------------
 template <Accept kMode, bool kCount, int kInst>
-__global__ void __launch_bounds__(128, HDCX_TRACE_MIN_BLOCKS) extendKernel(DeviceScene s, PathBuffers p, const uint32_t* queue,
-                                                    const unsigned long long* count)
+HDCX_D void extendEntry(const DeviceScene& s, const PathBuffers& p, uint32_t entry, uint32_t& fault, uint2* work)
 {
-    const unsigned long long counted = *count;
-    const uint32_t n = static_cast<uint32_t>(counted);
-    if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(p.stats + 0, counted >> 32);
+    const uint32_t slot = entryLeader(entry);
+    const float4 o = p.ray[2u * slot];
+    const float4 d = p.ray[2u * slot + 1u];
+    HitRecord h;
+    if (traceRay<kMode, false, kCount, kInst>(s, xyz(o), xyz(d), 0.001f, 10000.0f, __float_as_uint(o.w), h, fault, work)) {
+        p.hit[slot] = make_float4(h.t, __uint_as_float(h.primitive), h.b1, h.b2);
+        if (p.merged != 0u || __popc(entry & 7u) == 1) p.hitQueue[appendIndex(p.counters + kCountHits)] = entry;
+        else p.groupQueue[appendIndex(p.counters + kCountGroups)] = entry;
+    } else {
+        p.missQueue[appendIndex(p.counters + kCountMisses)] = entry;
+    }
+}
+
+// ---------------------------------------------------------------------------
+// shadow: visibility of light samples (vulkan_path_tracer.cpp:855-912). The
+// value of a visible sample is already in its light-sample slots; a blocked
+// ray clears them, or (kShadowGeneral) recomputes them from the factors.
+// ---------------------------------------------------------------------------
+template <bool kOpaque, bool kCount, int kInst>
+HDCX_D void shadowEntry(const DeviceScene& s, const PathBuffers& p, uint32_t i, uint32_t& fault, uint2* work)
+{
+    constexpr Accept kMode = kOpaque ? Accept::Opaque : Accept::Threshold;
+    const float4 o = p.shadowRay[2u * i];
+    const float4 d = p.shadowRay[2u * i + 1u];
+    const uint32_t info = p.shadowInfo[i];
+    const GpuLight& light = s.lights[info >> 8];
+    const bool general = (info & kShadowGeneral) != 0u;
+    const bool falloff = general && light.shadow.y >= 0.0f && light.shadow.z > 0.0f;
+    HitRecord h;
+    h.t = 0.0f;
+    const bool blocked =
+        falloff ? traceRay<kMode, false, kCount, kInst>(s, xyz(o), xyz(d), 0.001f, o.w, 0u, h, fault, work)
+                : traceRay<kMode, true, kCount, kInst>(s, xyz(o), xyz(d), 0.001f, o.w, 0u, h, fault, work);
+    if (!blocked) return;
+    const uint32_t entry = __float_as_uint(d.w);
+    const uint32_t j = (info >> 2) & 3u;
+    float3 visibility = f3(0.0f);
+    if (general) {
+        float strength = 1.0f;
+        if (falloff) {
+            const float falloffDistance = gmin(light.shadow.z, gmax(light.shadow.y, 0.0f));
+            strength = clampf((light.shadow.y - h.t) / gmax(falloffDistance, 1e-6f), 0.0f, 1.0f);
+            strength = gpow(strength, gmax(light.shadow.w, 0.0f));
+        }
+        visibility = mix(f3(1.0f), xyz(light.shadowColor), strength);
+    }
+    for (uint32_t lane = 0; lane < 3u; ++lane) {
+        if (!(entry >> lane & 1u)) continue;
+        const uint32_t slot = (entry >> 3) * 3u + lane;
+        const uint32_t index = contributionIndex(slot, p.lightSlots, j);
+        float value = 0.0f;
+        if (general) {
+            const float4 fct = p.shadowFactors[index];
+            const Spectrum spec = spectrumFromBasis(p.wavelength[slot], p.spectrum[slot]);
+            const float sv = reflectanceSpectrum(visibility, spec);
+            const uint32_t kind = info & 3u;
+            value = kind == kShadowAnalytic ? fct.x * sv * fct.y * fct.z / fct.w : (kind == kShadowSun ? fct.x * sv : fct.x * sv * fct.y);
+        }
+        p.contribution[index] = value;
+    }
+}
+
+// What one launch traces: the extension queue of a bounce, the shadow queue of
+// the bounce before it, or both. The two are independent, and together their
+// rays fill the tail that each launch ends in: when nothing asks for their
+// separate times or counts they are traced in one launch.
+struct TraceWork {
+    const uint32_t* queue;                 // extension entries; null: none
+    const unsigned long long* queueCount;
+    const unsigned long long* shadowCount;  // null: no shadow rays
+};
+
+template <bool kOpaque, bool kCount, int kInst, bool kExtend, bool kShadow>
+__global__ void __launch_bounds__(128, HDCX_TRACE_MIN_BLOCKS) traceKernel(DeviceScene s, PathBuffers p, TraceWork t)
+{
+    const unsigned long long extensions = kExtend ? *t.queueCount : 0ull;
+    const unsigned long long shadows = kShadow ? *t.shadowCount : 0ull;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        if (kExtend) atomicAdd(p.stats + 0, extensions >> 32);
+        if (kShadow) atomicAdd(p.stats + 1, shadows >> 32);
+    }
+    const uint32_t first = static_cast<uint32_t>(extensions);
+    const uint32_t n = first + static_cast<uint32_t>(shadows);
     uint2 work = make_uint2(0u, 0u);
     uint32_t fault = 0u;  // traversal faults of this thread's rays
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const uint32_t entry = queue[i];
-        const uint32_t slot = entryLeader(entry);
-        const float4 o = p.ray[2u * slot];
-        const float4 d = p.ray[2u * slot + 1u];
-        HitRecord h;
-        const bool found = traceRay<kMode, false, kCount, kInst>(s, xyz(o), xyz(d), 0.001f, 10000.0f, __float_as_uint(o.w), h, fault, &work);
-        // Hits and misses go to separate queues, so that shading warps hold
-        // only hits and the short environment path runs in its own kernel;
-        // entries of several lanes and of one lane have shade kernels of
-        // their own.
-        if (found) {
-            p.hit[slot] = make_float4(h.t, __uint_as_float(h.primitive), h.b1, h.b2);
-            if (__popc(entry & 7u) > 1) p.groupQueue[appendIndex(p.counters + kCountGroups)] = entry;
-            else p.hitQueue[appendIndex(p.counters + kCountSingles)] = entry;
-        } else {
-            p.missQueue[appendIndex(p.counters + kCountMisses)] = entry;
+        if (kExtend && (!kShadow || i < first)) {
+            extendEntry<kOpaque ? Accept::Opaque : Accept::Stochastic, kCount, kInst>(s, p, t.queue[i], fault, &work);
+        } else if (kShadow) {
+            shadowEntry<kOpaque, kCount, kInst>(s, p, i - first, fault, &work);
         }
     }
     if (fault != 0u) atomicOr(reinterpret_cast<unsigned int*>(p.stats + 7), fault);
     if (kCount) {
-        atomicAdd(p.stats + 3, static_cast<unsigned long long>(work.x));
-        atomicAdd(p.stats + 4, static_cast<unsigned long long>(work.y));
+        atomicAdd(p.stats + (kExtend ? 3 : 5), static_cast<unsigned long long>(work.x));
+        atomicAdd(p.stats + (kExtend ? 4 : 6), static_cast<unsigned long long>(work.y));
     }
 }
 
@@ -215,105 +286,6 @@ __global__ void __launch_bounds__(128, HDCX_TRACE_MIN_BLOCKS)
     }
     if (rays != 0u) atomicAdd(p.stats + 2, static_cast<unsigned long long>(rays));
     if (fault != 0u) atomicOr(reinterpret_cast<unsigned int*>(p.stats + 7), fault);
-}
-
-// ---------------------------------------------------------------------------
-// miss: environment on a miss (vulkan_path_tracer.cpp:1245-1255), the entries
-// of extend's miss queue. The environment is looked up once per entry.
-// ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(128) missKernel(DeviceScene s, FrameConst f, PathBuffers p)
-{
-    const uint32_t n = p.counters[kCountMisses];
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const uint32_t entry = p.missQueue[i];
-        const float4 d = p.ray[2u * entryLeader(entry) + 1u];
-        const uint32_t flags = __float_as_uint(d.w);
-        const bool lit = (flags & kFlagEnvironmentOnMiss) != 0u;
-        const float3 sky = lit ? environment(s, f, xyz(d)) : f3(0.0f);
-        for (uint32_t lane = 0; lane < 3u; ++lane) {
-            if (!(entry >> lane & 1u)) continue;
-            const uint32_t slot = (entry >> 3) * 3u + lane;
-            float radiance = p.radiance[slot];
-            // Light samples of the previous bounce, in slot order.
-            for (uint32_t j = 0; j < p.lightSlots; ++j) {
-                float& pending = p.contribution[contributionIndex(slot, p.lightSlots, j)];
-                const float value = pending;
-                if (value != 0.0f) {
-                    radiance += value;
-                    pending = 0.0f;
-                }
-            }
-            if (lit) {
-                const Spectrum spec = spectrumFromBasis(p.wavelength[slot], p.spectrum[slot]);
-                const float2 previousPdf = p.previousPdf[slot];
-                const float misWeight =
-                    (flags & kFlagPreviousWasDelta) != 0u ? 1.0f : powerHeuristic(previousPdf.x, previousPdf.y);
-                radiance += p.throughput[slot] * misWeight * illuminantSpectrum(sky, spec);
-            }
-            p.radiance[slot] = radiance;
-        }
-    }
-}
-
-// ---------------------------------------------------------------------------
-// shadow: visibility of light samples (vulkan_path_tracer.cpp:855-912). The
-// value of a visible sample is already in its light-sample slots; a blocked
-// ray clears them, or (kShadowGeneral) recomputes them from the factors.
-// ---------------------------------------------------------------------------
-template <bool kOpaque, bool kCount, int kInst>
-__global__ void __launch_bounds__(128, HDCX_TRACE_MIN_BLOCKS) shadowKernel(DeviceScene s, PathBuffers p)
-{
-    const unsigned long long counted = *reinterpret_cast<const unsigned long long*>(p.counters + kCountShadow);
-    const uint32_t n = static_cast<uint32_t>(counted);
-    if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(p.stats + 1, counted >> 32);
-    constexpr Accept kMode = kOpaque ? Accept::Opaque : Accept::Threshold;
-    uint2 work = make_uint2(0u, 0u);
-    uint32_t fault = 0u;  // traversal faults of this thread's rays
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const float4 o = p.shadowRay[2u * i];
-        const float4 d = p.shadowRay[2u * i + 1u];
-        const uint32_t info = p.shadowInfo[i];
-        const GpuLight& light = s.lights[info >> 8];
-        const bool general = (info & kShadowGeneral) != 0u;
-        const bool falloff = general && light.shadow.y >= 0.0f && light.shadow.z > 0.0f;
-        HitRecord h;
-        h.t = 0.0f;
-        const bool blocked =
-            falloff ? traceRay<kMode, false, kCount, kInst>(s, xyz(o), xyz(d), 0.001f, o.w, 0u, h, fault, &work)
-                    : traceRay<kMode, true, kCount, kInst>(s, xyz(o), xyz(d), 0.001f, o.w, 0u, h, fault, &work);
-        if (!blocked) continue;
-        const uint32_t entry = __float_as_uint(d.w);
-        const uint32_t j = (info >> 2) & 3u;
-        float3 visibility = f3(0.0f);
-        if (general) {
-            float strength = 1.0f;
-            if (falloff) {
-                const float falloffDistance = gmin(light.shadow.z, gmax(light.shadow.y, 0.0f));
-                strength = clampf((light.shadow.y - h.t) / gmax(falloffDistance, 1e-6f), 0.0f, 1.0f);
-                strength = gpow(strength, gmax(light.shadow.w, 0.0f));
-            }
-            visibility = mix(f3(1.0f), xyz(light.shadowColor), strength);
-        }
-        for (uint32_t lane = 0; lane < 3u; ++lane) {
-            if (!(entry >> lane & 1u)) continue;
-            const uint32_t slot = (entry >> 3) * 3u + lane;
-            const uint32_t index = contributionIndex(slot, p.lightSlots, j);
-            float value = 0.0f;
-            if (general) {
-                const float4 fct = p.shadowFactors[index];
-                const Spectrum spec = spectrumFromBasis(p.wavelength[slot], p.spectrum[slot]);
-                const float sv = reflectanceSpectrum(visibility, spec);
-                const uint32_t kind = info & 3u;
-                value = kind == kShadowAnalytic ? fct.x * sv * fct.y * fct.z / fct.w : (kind == kShadowSun ? fct.x * sv : fct.x * sv * fct.y);
-            }
-            p.contribution[index] = value;
-        }
-    }
-    if (fault != 0u) atomicOr(reinterpret_cast<unsigned int*>(p.stats + 7), fault);
-    if (kCount) {
-        atomicAdd(p.stats + 5, static_cast<unsigned long long>(work.x));
-        atomicAdd(p.stats + 6, static_cast<unsigned long long>(work.y));
-    }
 }
 
 // ---------------------------------------------------------------------------
@@ -636,28 +608,33 @@ __global__ void __launch_bounds__(256) sortRaysKernel(PathBuffers p, uint32_t* q
     }
 }
 
-template <int kInst>
-void launchExtend(const DeviceScene& scene, PathBuffers& paths, const uint32_t* inQueue, const unsigned long long* inCount,
-                  bool count, int grid, cudaStream_t stream)
+template <bool kCount, int kInst>
+void launchTraceOf(const DeviceScene& scene, const PathBuffers& paths, const TraceWork& t, int grid, cudaStream_t stream)
 {
-    if (count) {
-        if (scene.opaque) extendKernel<Accept::Opaque, true, kInst><<<grid, 128, 0, stream>>>(scene, paths, inQueue, inCount);
-        else extendKernel<Accept::Stochastic, true, kInst><<<grid, 128, 0, stream>>>(scene, paths, inQueue, inCount);
+    const bool extend = t.queueCount != nullptr, shadow = t.shadowCount != nullptr;
+    if (scene.opaque) {
+        if (extend && shadow) {
+            if constexpr (!kCount) traceKernel<true, false, kInst, true, true><<<grid, 128, 0, stream>>>(scene, paths, t);
+        } else if (extend) traceKernel<true, kCount, kInst, true, false><<<grid, 128, 0, stream>>>(scene, paths, t);
+        else traceKernel<true, kCount, kInst, false, true><<<grid, 128, 0, stream>>>(scene, paths, t);
     } else {
-        if (scene.opaque) extendKernel<Accept::Opaque, false, kInst><<<grid, 128, 0, stream>>>(scene, paths, inQueue, inCount);
-        else extendKernel<Accept::Stochastic, false, kInst><<<grid, 128, 0, stream>>>(scene, paths, inQueue, inCount);
+        if (extend && shadow) {
+            if constexpr (!kCount) traceKernel<false, false, kInst, true, true><<<grid, 128, 0, stream>>>(scene, paths, t);
+        } else if (extend) traceKernel<false, kCount, kInst, true, false><<<grid, 128, 0, stream>>>(scene, paths, t);
+        else traceKernel<false, kCount, kInst, false, true><<<grid, 128, 0, stream>>>(scene, paths, t);
     }
+    CUDA_OK(cudaGetLastError());
 }
 
-template <int kInst>
-void launchShadow(const DeviceScene& scene, PathBuffers& paths, bool count, int grid, cudaStream_t stream)
+// Both queues at once are for renders that do not count (see TraceWork).
+void launchTrace(const DeviceScene& scene, const PathBuffers& paths, const TraceWork& t, bool count, int grid, cudaStream_t stream)
 {
     if (count) {
-        if (scene.opaque) shadowKernel<true, true, kInst><<<grid, 128, 0, stream>>>(scene, paths);
-        else shadowKernel<false, true, kInst><<<grid, 128, 0, stream>>>(scene, paths);
+        if (scene.instances) launchTraceOf<true, 1>(scene, paths, t, grid, stream);
+        else launchTraceOf<true, 0>(scene, paths, t, grid, stream);
     } else {
-        if (scene.opaque) shadowKernel<true, false, kInst><<<grid, 128, 0, stream>>>(scene, paths);
-        else shadowKernel<false, false, kInst><<<grid, 128, 0, stream>>>(scene, paths);
+        if (scene.instances) launchTraceOf<false, 1>(scene, paths, t, grid, stream);
+        else launchTraceOf<false, 0>(scene, paths, t, grid, stream);
     }
 }
 
@@ -727,6 +704,12 @@ void renderFrame(const DeviceScene& sceneIn, const FrameConst& frame, PathBuffer
     // Lanes travel alone in radiance-cache mode (training paths and queries
     // are per lane) and where walks run inside the shade kernel.
     paths.split = cacheMode || (scene.fullShading && !deferWalks(paths)) ? 1u : 0u;
+    // Scenes whose lanes part seldom shade every entry in one launch: entries of
+    // one lane are too few for a kernel of their own to pay for its latency
+    // (40 us a bounce, a warp's walk through cold instructions).
+    paths.merged = !paths.split && scene.partsLanes == 0u ? 1u : 0u;
+    // Stage times and traversal counts are those of separate launches.
+    const bool fused = timing == nullptr && !countTraversal;
     const ShadeVariant variant{scene.fullShading != 0u, lit, cacheMode, deferWalks(paths)};
     uint32_t* counters = paths.counters;
     auto counter64 = [&](uint32_t word) { return reinterpret_cast<unsigned long long*>(counters + word); };
@@ -748,53 +731,57 @@ void renderFrame(const DeviceScene& sceneIn, const FrameConst& frame, PathBuffer
         for (uint32_t bounce = 0; bounce < frame.maxBounces; ++bounce) {
             uint32_t* inQueue = paths.queue[bounce & 1u];
             uint32_t* outQueue = paths.queue[(bounce + 1u) & 1u];
-            const uint32_t inWord = (bounce & 1u) ? kCountQueue1 : kCountQueue0;
-            unsigned long long* inCount = counter64(inWord);
-            unsigned long long* outCount = counter64((bounce & 1u) ? kCountQueue0 : kCountQueue1);
-            // Everything but the queue this bounce reads.
-            const uint32_t clearFrom = inWord == kCountQueue0 ? kCountShadow : kCountQueue0;
-            const uint32_t clearTo = inWord == kCountQueue0 ? kCountEnd : kCountQueue1;
+            const bool odd = (bounce & 1u) != 0u;
+            unsigned long long* inCount = counter64(odd ? kCountQueue1 : kCountQueue0);
+            unsigned long long* outCount = counter64(odd ? kCountQueue0 : kCountQueue1);
+            const unsigned long long* previousShadows = bounce > 0u ? counter64(odd ? kCountShadow0 : kCountShadow1) : nullptr;
+            paths.shadowWord = odd ? kCountShadow1 : kCountShadow0;
+            const uint32_t clearFrom = odd ? 0u : kCountHits, clearTo = odd ? kCountShadow0 : kCountEnd;
             CUDA_OK(cudaMemsetAsync(counters + clearFrom, 0, (clearTo - clearFrom) * sizeof(uint32_t), stream));
             if (sortRays && bounce > 0u) {
                 sortRaysKernel<<<sortGrid, 256, 0, stream>>>(paths, inQueue, inCount);
                 launched += 1;
             }
             timed(0, [&] {
-                if (scene.instances) launchExtend<1>(scene, paths, inQueue, inCount, countTraversal, traceGrid, stream);
-                else launchExtend<0>(scene, paths, inQueue, inCount, countTraversal, traceGrid, stream);
+                launchTrace(scene, paths, TraceWork{inQueue, inCount, fused ? previousShadows : nullptr}, countTraversal, traceGrid, stream);
             });
-            CUDA_OK(cudaGetLastError());
             timed(1, [&] {
-                ShadeLaunch launch{scene, frame, paths, bounce, nullptr, nullptr, outQueue, outCount, shadeGrid, stream};
+                ShadeLaunch launch{scene, frame, paths, bounce, nullptr, nullptr, outQueue, outCount, true, shadeGrid, stream};
                 if (!paths.split) {
-                    launch.count = counters + kCountGroups;
-                    launch.queue = sortedByMaterial(paths.groupQueue, launch.count);
+                    launch.count = counters + (paths.merged ? kCountHits : kCountGroups);
+                    launch.queue = sortedByMaterial(paths.merged ? paths.hitQueue : paths.groupQueue, launch.count);
                     launchShadeGroups(variant, launch);
+                    launch.misses = false;
                     launched += 1;
                 }
-                launch.count = counters + kCountSingles;
-                launch.queue = sortedByMaterial(paths.hitQueue, launch.count);
-                launchShadeSingles(variant, launch);
-                missKernel<<<missGrid, 128, 0, stream>>>(scene, frame, paths);
+                if (!paths.merged) {
+                    launch.count = counters + kCountHits;
+                    launch.queue = sortedByMaterial(paths.hitQueue, launch.count);
+                    launchShadeSingles(variant, launch);
+                    launched += 1;
+                }
                 if (walks) {
                     // The deferred walks (in this bounce's traced extension
                     // queue), then the failed ones re-shaded (queued in the
-                    // miss queue, which missKernel has consumed).
-                    if (scene.instances) walkKernel<1><<<traceGrid, 128, 0, stream>>>(scene, paths, inQueue, outQueue, outCount, paths.missQueue);
-                    else walkKernel<0><<<traceGrid, 128, 0, stream>>>(scene, paths, inQueue, outQueue, outCount, paths.missQueue);
-                    launch.queue = paths.missQueue;
+                    // hit queue, which has been shaded).
+                    if (scene.instances) walkKernel<1><<<traceGrid, 128, 0, stream>>>(scene, paths, inQueue, outQueue, outCount, paths.hitQueue);
+                    else walkKernel<0><<<traceGrid, 128, 0, stream>>>(scene, paths, inQueue, outQueue, outCount, paths.hitQueue);
+                    launch.queue = paths.hitQueue;
                     launch.count = counters + kCountReplays;
+                    launch.misses = false;
                     launch.grid = missGrid;
                     launchShadeReplays(variant, launch);
+                    launched += 2;
                 }
             });
             CUDA_OK(cudaGetLastError());
-            timed(2, [&] {
-                if (scene.instances) launchShadow<1>(scene, paths, countTraversal, traceGrid, stream);
-                else launchShadow<0>(scene, paths, countTraversal, traceGrid, stream);
-            });
-            CUDA_OK(cudaGetLastError());
-            launched += 4 + (walks ? 2 : 0);
+            launched += 1;
+            if (!fused || bounce + 1u == frame.maxBounces) {
+                timed(2, [&] {
+                    launchTrace(scene, paths, TraceWork{nullptr, nullptr, counter64(paths.shadowWord)}, countTraversal, traceGrid, stream);
+                });
+                launched += 1;
+            }
         }
         if (cacheMode) {
             // Predictions for the terminated paths, then one training round on

@@ -41,19 +41,22 @@ constexpr uint32_t kHitBins = 256;
 
 // Queue counters of a wave (32-bit words of PathBuffers::counters). The
 // extension and shadow queues count entries in a 64-bit counter's low half
-// and lanes in its high half. One clear per bounce covers the counters that
-// the bounce fills: kCountQueue0 .. kCountEnd without the queue it reads.
+// and lanes in its high half. A bounce reads its extension queue and the
+// shadow queue of the bounce before it and fills the others, which one clear
+// covers: words kCountHits to the end in even bounces (they read kCountQueue0
+// and kCountShadow1), words 0 to kCountShadow0 in odd ones.
 enum : uint32_t {
     kCountQueue0 = 0,    // 64-bit: extension queue of even bounces
-    kCountShadow = 2,    // 64-bit: shadow queue
-    kCountGroups = 4,    // hits of entries with several lanes
-    kCountSingles = 5,   // hits of entries with one lane
+    kCountShadow1 = 2,   // 64-bit: shadow queue of odd bounces
+    kCountHits = 4,      // entries of hitQueue
+    kCountGroups = 5,    // entries of groupQueue
     kCountMisses = 6,
     kCountWalks = 7,     // deferred subsurface walks
     kCountReplays = 8,   // failed walks to re-shade
     kCountWalkNext = 9,  // walks taken by walkKernel's threads
-    kCountQueue1 = 10,   // 64-bit: extension queue of odd bounces
-    kCountEnd = 12,
+    kCountShadow0 = 10,  // 64-bit: shadow queue of even bounces
+    kCountQueue1 = 12,   // 64-bit: extension queue of odd bounces
+    kCountEnd = 14,
 };
 
 // Device buffers of one wave of paths (structure of arrays; slot 3 g + lane,
@@ -64,6 +67,8 @@ struct PathBuffers {
     uint32_t shadowPerPath = 0;     // shadow-ray slots per path per bounce
     uint32_t lightSlots = 3;        // light-sample slots in use: 1 (analytic), 2 (+ mesh lights) or 3 (fallback sun and sky)
     uint32_t split = 0;             // 1: every lane travels as an entry of its own from the start
+    uint32_t merged = 0;            // 1: hitQueue takes every entry, groupQueue none
+    uint32_t shadowWord = 0;        // counter of the bounce's shadow queue
     float* wavelength = nullptr;
     float4* spectrum = nullptr;     // basis r, g, b and Planck factor of the lane
     float* throughput = nullptr;
@@ -75,7 +80,7 @@ struct PathBuffers {
     float* contribution = nullptr;  // 3 * capacity: path slot s, light-sample slot j at lightSlots * s + j
     uint32_t* queue[2] = {nullptr, nullptr};  // extension entries
     uint32_t* groupQueue = nullptr;     // extend's output: entries of several lanes whose ray hit
-    uint32_t* hitQueue = nullptr;       // extend's output: entries of one lane whose ray hit
+    uint32_t* hitQueue = nullptr;       // extend's output: entries of one lane whose ray hit (all of them if merged)
     uint32_t* missQueue = nullptr;      // extend's output: entries whose ray missed (environment)
     float4* shadowRay = nullptr;        // two per shadow ray: origin and tmax, direction and entry
     float4* shadowFactors = nullptr;    // per path slot and light-sample slot (kShadowGeneral): partial product, f1, f2, f3

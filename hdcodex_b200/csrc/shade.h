@@ -22,6 +22,7 @@ struct ShadeLaunch {
     const uint32_t* count;
     uint32_t* nextQueue;
     unsigned long long* nextCount;
+    bool misses;  // this launch also shades the bounce's miss queue
     int grid;
     cudaStream_t stream;
 };

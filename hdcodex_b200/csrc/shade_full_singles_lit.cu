@@ -12,7 +12,7 @@ void launch(const ShadeLaunch& l)
     constexpr int kThreads = shadeThreads<kLanes, kFull>();
     const int grid = (l.grid * 128 + kThreads - 1) / kThreads;
     shadeKernel<kLanes, kFull, kLit, kCache, kWalk><<<grid, kThreads, 0, l.stream>>>(l.scene, l.frame, l.paths, l.bounce, l.queue,
-                                                                                  l.count, l.nextQueue, l.nextCount);
+                                                                                  l.count, l.nextQueue, l.nextCount, l.misses);
 }
 
 }  // namespace
