@@ -67,8 +67,27 @@ HDCX_D uint32_t appendEntry(unsigned long long* counter, uint32_t mask)
     return base + static_cast<uint32_t>(__popc(together & ((1u << lane) - 1u)));
 }
 
-// Light-sample slot j of path `slot`: the value it adds to the path's radiance
-// at the next vertex, zero where there is none.
-HDCX_D uint32_t contributionIndex(uint32_t slot, uint32_t lightSlots, uint32_t j) { return slot * lightSlots + j; }
+// PathBuffers::laneLight and laneState: the per-lane state of a group in
+// records of three lanes to a field, so that an entry scattered anywhere in
+// the wave costs few memory sectors, and vector accesses when it holds all
+// lanes. What the light sample completes (laneLight) is written before what
+// the BSDF sample does.
+enum : uint32_t {
+    kLaneRadiance = 0,    // laneLight
+    kLaneLight = 3,       // light-sample slot 0: the value it adds at the next vertex, zero where there is none
+    kLaneThroughput = 0,  // laneState
+    kLaneBsdfPdf = 3,     // previousBsdfPdf
+    kLaneLightPdf = 6,    // previousEnvironmentLightPdf
+};
+HDCX_D float* lightRecord(const PathBuffers& p, uint32_t group) { return reinterpret_cast<float*>(p.laneLight + 2u * static_cast<size_t>(group)); }
+HDCX_D float* laneRecord(const PathBuffers& p, uint32_t group) { return reinterpret_cast<float*>(p.laneState + 3u * static_cast<size_t>(group)); }
+HDCX_D const float* spectrumRecord(const PathBuffers& p, uint32_t group)
+{
+    return reinterpret_cast<const float*>(p.laneSpectrum + 4u * static_cast<size_t>(group));
+}
+
+// Light-sample slots 1 and 2 (mesh lights, fallback sky) of path `slot`, as
+// kLaneLight for slot 0.
+HDCX_D uint32_t contributionIndex(uint32_t slot, uint32_t j) { return slot * 2u + j - 1u; }
 
 }  // namespace hdcx

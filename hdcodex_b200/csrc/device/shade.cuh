@@ -69,35 +69,51 @@ HDCX_D void emitShadow(PathBuffers& p, uint32_t group, uint32_t lanes, uint32_t 
     p.shadowInfo[i] = info;
 }
 
-// Environment on a miss (vulkan_path_tracer.cpp:1245-1255) of an entry's lanes.
+// Environment on a miss (vulkan_path_tracer.cpp:1245-1255) of an entry's lanes,
+// looked up once. All loads come before the stores: lanes that loaded after a
+// neighbour's store to the same sector took ten times as long.
 HDCX_D void shadeMiss(const DeviceScene& s, const FrameConst& f, const PathBuffers& p, uint32_t entry, uint32_t lightSlots)
 {
     const float4 d = p.ray[2u * entryLeader(entry) + 1u];
     const uint32_t flags = __float_as_uint(d.w);
     const bool lit = (flags & kFlagEnvironmentOnMiss) != 0u;
     const float3 sky = lit ? environment(s, f, xyz(d)) : f3(0.0f);
-#pragma unroll 1
+    const uint32_t group = entry >> 3;
+    const float4* light = reinterpret_cast<const float4*>(lightRecord(p, group));
+    const float4* state = reinterpret_cast<const float4*>(laneRecord(p, group));
+    const float4* spectra = p.laneSpectrum + 4u * static_cast<size_t>(group);
+    const float4 l0 = light[0], l1 = light[1], a = state[0], b = state[1], c = state[2];
+    const float4 basis[3] = {spectra[0], spectra[1], spectra[2]}, w = spectra[3];
+    // Light samples of the previous bounce, in slot order.
+    float radiance[3] = {l0.x + l0.w, l0.y + l1.x, l0.z + l1.y};
+    const float throughput[3] = {a.x, a.y, a.z}, bsdfPdf[3] = {a.w, b.x, b.y}, lightPdf[3] = {b.z, b.w, c.x};
+    const float wavelength[3] = {w.x, w.y, w.z};
+#pragma unroll
     for (uint32_t lane = 0; lane < 3u; ++lane) {
-        if (!(entry >> lane & 1u)) continue;
-        const uint32_t slot = (entry >> 3) * 3u + lane;
-        float radiance = p.radiance[slot];
-        // Light samples of the previous bounce, in slot order.
-#pragma unroll 1
-        for (uint32_t j = 0; j < lightSlots; ++j) {
-            float& pending = p.contribution[contributionIndex(slot, lightSlots, j)];
-            const float value = pending;
-            if (value != 0.0f) {
-                radiance += value;
+        if (lightSlots > 1u && (entry >> lane & 1u)) {
+            for (uint32_t j = 1; j < lightSlots; ++j) {
+                float& pending = p.contribution[contributionIndex(group * 3u + lane, j)];
+                radiance[lane] += pending;
                 pending = 0.0f;
             }
         }
         if (lit) {
-            const Spectrum spec = spectrumFromBasis(p.wavelength[slot], p.spectrum[slot]);
-            const float2 previousPdf = p.previousPdf[slot];
-            const float misWeight = (flags & kFlagPreviousWasDelta) != 0u ? 1.0f : powerHeuristic(previousPdf.x, previousPdf.y);
-            radiance += p.throughput[slot] * misWeight * illuminantSpectrum(sky, spec);
+            const Spectrum spec = spectrumFromBasis(wavelength[lane], basis[lane]);
+            const float misWeight = (flags & kFlagPreviousWasDelta) != 0u ? 1.0f : powerHeuristic(bsdfPdf[lane], lightPdf[lane]);
+            radiance[lane] += throughput[lane] * misWeight * illuminantSpectrum(sky, spec);
         }
-        p.radiance[slot] = radiance;
+    }
+    float* out = lightRecord(p, group);
+    if ((entry & 7u) == 7u) {
+        reinterpret_cast<float4*>(out)[0] = make_float4(radiance[0], radiance[1], radiance[2], 0.0f);
+        reinterpret_cast<float4*>(out)[1] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        return;
+    }
+#pragma unroll
+    for (uint32_t lane = 0; lane < 3u; ++lane) {
+        if (!(entry >> lane & 1u)) continue;
+        out[kLaneRadiance + lane] = radiance[lane];
+        out[kLaneLight + lane] = 0.0f;
     }
 }
 
@@ -239,10 +255,8 @@ __global__ void __launch_bounds__((shadeThreads<kLanes, kFull>()), (shadeMinBloc
         float3 rayDirection = xyz(ray1);
         uint32_t rng = __float_as_uint(ray0.w);
         const uint32_t flags = __float_as_uint(ray1.w);
-        const bool environmentBefore = (flags & kFlagEnvironmentOnMiss) != 0u;
         const bool previousWasDelta = (flags & kFlagPreviousWasDelta) != 0u;
         const bool insideMedium = (flags & kFlagInsideMedium) != 0u;
-        (void)environmentBefore;
         const float4 hitRec = p.hit[slot];
         const uint32_t primitive = __float_as_uint(hitRec.y);
         // The medium coefficients matter only inside a medium (entering one
@@ -274,46 +288,62 @@ __global__ void __launch_bounds__((shadeThreads<kLanes, kFull>()), (shadeMinBloc
                 mask = 0u;
             }
         }
+        // The lanes' state and spectra. Light samples of the previous bounce are
+        // added in slot order; a slot without one holds zero. (A replay finds
+        // this bounce's own samples in the slots: they stay.)
         V radiance, throughput, previousBsdfPdf, previousEnvironmentLightPdf;
         SpectrumOf<V> spec;
-#pragma unroll
-        for (int k = 0; k < kLanes; ++k) {
-            const uint32_t own = first + k;
-            put(radiance, k, p.radiance[own]);
-            put(throughput, k, p.throughput[own]);
-            const float2 pdf = p.previousPdf[own];
-            put(previousBsdfPdf, k, pdf.x);
-            put(previousEnvironmentLightPdf, k, pdf.y);
-            const Spectrum one = spectrumFromBasis(p.wavelength[own], p.spectrum[own]);
-            put(spec.wavelength, k, one.wavelength);
-            put(spec.br, k, one.br);
-            put(spec.bg, k, one.bg);
-            put(spec.bb, k, one.bb);
-            put(spec.denominator, k, one.denominator);
-            put(spec.planck, k, one.planck);
+        float* record = laneRecord(p, group);
+        float* lightOf = lightRecord(p, group);
+        const uint32_t onlyLane = firstLane(entry & 7u);  // kLanes = 1
+        if constexpr (kLanes == 3) {
+            const float4* l = reinterpret_cast<const float4*>(lightOf);
+            const float4* r = reinterpret_cast<const float4*>(record);
+            const float4 l0 = l[0], l1 = l[1], a = r[0], b = r[1], c = r[2];
+            radiance = Lanes3(l0.x, l0.y, l0.z) + Lanes3(l0.w, l1.x, l1.y);
+            throughput = Lanes3(a.x, a.y, a.z);
+            previousBsdfPdf = Lanes3(a.w, b.x, b.y);
+            previousEnvironmentLightPdf = Lanes3(b.z, b.w, c.x);
+            const float4* q = p.laneSpectrum + 4u * static_cast<size_t>(group);
+            const float4 s0 = q[0], s1 = q[1], s2 = q[2], w = q[3];
+            spec.wavelength = Lanes3(w.x, w.y, w.z);
+            spec.br = Lanes3(s0.x, s1.x, s2.x);
+            spec.bg = Lanes3(s0.y, s1.y, s2.y);
+            spec.bb = Lanes3(s0.z, s1.z, s2.z);
+            spec.planck = Lanes3(s0.w, s1.w, s2.w);
+            spec.denominator = gmax(spec.br + spec.bg + spec.bb, Lanes3(1e-5f));
+        } else {
+            throughput = record[kLaneThroughput + onlyLane];
+            radiance = lightOf[kLaneRadiance + onlyLane];
+            if (!kReplay) radiance += lightOf[kLaneLight + onlyLane];
+            previousBsdfPdf = record[kLaneBsdfPdf + onlyLane];
+            previousEnvironmentLightPdf = record[kLaneLightPdf + onlyLane];
+            const float* q = spectrumRecord(p, group);
+            spec = spectrumFromBasis(q[12u + onlyLane], reinterpret_cast<const float4*>(q)[onlyLane]);
         }
-        // Light samples of the previous bounce, in slot order; a slot without
-        // one holds zero, and so does a read one. (A replay finds this
-        // bounce's own samples in the slots: they stay.)
-        if (!kReplay) {
+        if (!kReplay && !kLit && lightSlots > 1u) {
+            // All loads before the clears, as in shadeMiss.
+            V second = V(0.0f), third = V(0.0f);
 #pragma unroll
             for (int k = 0; k < kLanes; ++k) {
                 if (!(mask >> k & 1u)) continue;
-                for (uint32_t j = 0; j < lightSlots; ++j) {
-                    float& pending = p.contribution[contributionIndex(first + k, lightSlots, j)];
-                    const float value = pending;
-                    if (value != 0.0f) {
-                        put(radiance, k, at(radiance, k) + value);
-                        pending = 0.0f;
-                    }
-                }
+                put(second, k, p.contribution[contributionIndex(first + k, 1u)]);
+                if (lightSlots > 2u) put(third, k, p.contribution[contributionIndex(first + k, 2u)]);
+            }
+            radiance = radiance + second;
+            if (lightSlots > 2u) radiance = radiance + third;
+#pragma unroll
+            for (int k = 0; k < kLanes; ++k) {
+                if (at(second, k) != 0.0f) p.contribution[contributionIndex(first + k, 1u)] = 0.0f;
+                if (at(third, k) != 0.0f) p.contribution[contributionIndex(first + k, 2u)] = 0.0f;
             }
         }
+        V lightValue = V(0.0f);  // this bounce's light-sample slot 0
         // Ray cone (width, spread) of texture LOD; spread <= 0: level 0.
         const bool lodOn = kFull && f.pixelSpread > 0.0f && p.cone != nullptr;
         const float2 cone = lodOn ? p.cone[slot] : make_float2(0.0f, -1.0f);
         float coneWidth = 0.0f;
-        // Writes the state of lanes `alive` (after this bounce) and queues them.
+        // Writes the state of lanes `alive` after this bounce and queues them.
         auto advance = [&](uint32_t alive, float3 origin, float3 direction, uint32_t state, uint32_t newFlags, bool coneKept,
                            V newThroughput, V bsdfPdf, V lightPdf) {
             const uint32_t lead = first + firstLane(alive);
@@ -321,21 +351,46 @@ __global__ void __launch_bounds__((shadeThreads<kLanes, kFull>()), (shadeMinBloc
             p.ray[2u * lead + 1u] = make_float4(direction.x, direction.y, direction.z,
                                                 __uint_as_float(newFlags | (kCache ? (flags & kFlagTraining) : 0u)));
             if (lodOn) p.cone[lead] = coneKept ? make_float2(coneWidth, cone.y) : make_float2(0.0f, -1.0f);
+            if (kLanes == 3 && alive == 7u) {
+                float4* r = reinterpret_cast<float4*>(record);
+                r[0] = make_float4(at(newThroughput, 0), at(newThroughput, 1), at(newThroughput, 2), at(bsdfPdf, 0));
+                r[1] = make_float4(at(bsdfPdf, 1), at(bsdfPdf, 2), at(lightPdf, 0), at(lightPdf, 1));
+                r[2] = make_float4(at(lightPdf, 2), 0.0f, 0.0f, 0.0f);
+            } else {
 #pragma unroll
-            for (int k = 0; k < kLanes; ++k) {
-                if (!(alive >> k & 1u)) continue;
-                p.throughput[first + k] = at(newThroughput, k);
-                p.previousPdf[first + k] = make_float2(at(bsdfPdf, k), at(lightPdf, k));
-                if ((newFlags & kFlagInsideMedium) != 0u)
-                    p.medium[first + k] = make_float4(at(mediumAbsorption, k), at(mediumScattering, k), at(mediumAnisotropy, k), 0.0f);
+                for (int k = 0; k < kLanes; ++k) {
+                    if (!(alive >> k & 1u)) continue;
+                    const uint32_t lane = kLanes == 3 ? static_cast<uint32_t>(k) : onlyLane;
+                    record[kLaneThroughput + lane] = at(newThroughput, k);
+                    record[kLaneBsdfPdf + lane] = at(bsdfPdf, k);
+                    record[kLaneLightPdf + lane] = at(lightPdf, k);
+                }
+            }
+            if ((newFlags & kFlagInsideMedium) != 0u) {
+#pragma unroll
+                for (int k = 0; k < kLanes; ++k)
+                    if (alive >> k & 1u)
+                        p.medium[first + k] = make_float4(at(mediumAbsorption, k), at(mediumScattering, k), at(mediumAnisotropy, k), 0.0f);
             }
             const uint32_t lanes = kLanes == 3 ? alive : entry & 7u;
             nextQueue[appendEntry(nextCount, lanes)] = (group << 3) | lanes;
         };
-        auto storeRadiance = [&] {
+        // Writes radiance and light sample of the lanes of `mask`.
+        auto storeLight = [&] {
+            if (kReplay) return;
+            if (kLanes == 3 && mask == 7u) {
+                float4* l = reinterpret_cast<float4*>(lightOf);
+                l[0] = make_float4(at(radiance, 0), at(radiance, 1), at(radiance, 2), at(lightValue, 0));
+                l[1] = make_float4(at(lightValue, 1), at(lightValue, 2), 0.0f, 0.0f);
+                return;
+            }
 #pragma unroll
-            for (int k = 0; k < kLanes; ++k)
-                if (mask >> k & 1u) p.radiance[first + k] = at(radiance, k);
+            for (int k = 0; k < kLanes; ++k) {
+                if (!(mask >> k & 1u)) continue;
+                const uint32_t lane = kLanes == 3 ? static_cast<uint32_t>(k) : onlyLane;
+                lightOf[kLaneRadiance + lane] = at(radiance, k);
+                lightOf[kLaneLight + lane] = at(lightValue, k);
+            }
         };
 
             const uint32_t i0 = __ldg(s.indices + primitive * 3u + 0u);
@@ -380,7 +435,7 @@ __global__ void __launch_bounds__((shadeThreads<kLanes, kFull>()), (shadeMinBloc
                         throughput = throughput * V(gexp(-at(mediumAbsorption, 0) * scatterDistance));
                         rayOrigin = rayOrigin + rayDirection * scatterDistance;
                         rayDirection = sampleHenyeyGreenstein(rayDirection, at(mediumAnisotropy, 0), rng);
-                        if (!kReplay) storeRadiance();
+                        storeLight();
                         if (!lastBounce)
                             advance(mask, rayOrigin, rayDirection, rng,
                                     kFlagEnvironmentOnMiss | kFlagPreviousWasDelta | kFlagInsideMedium, false, throughput,
@@ -467,8 +522,8 @@ __global__ void __launch_bounds__((shadeThreads<kLanes, kFull>()), (shadeMinBloc
                         rec[1] = q1;
                         rec[2] = q2;
                         p.cache.querySlot[j] = slot;
-                        p.throughput[slot] = throughput;
-                        p.radiance[slot] = radiance;
+                        storeLight();
+                        record[kLaneThroughput + onlyLane] = at(throughput, 0);
                         mask = 0u;
                     }
                 }
@@ -633,15 +688,16 @@ __global__ void __launch_bounds__((shadeThreads<kLanes, kFull>()), (shadeMinBloc
 #pragma unroll
                 for (int k = 0; k < kLanes; ++k) {
                     if (!(lanes >> k & 1u)) continue;
-                    p.contribution[contributionIndex(first + k, lightSlots, j)] = at(value, k);
+                    if (j != 0u) p.contribution[contributionIndex(first + k, j)] = at(value, k);
                     general = general || !isfinite(at(value, k));
                 }
+                if (j == 0u) lightValue = whereMask(lanes, value, lightValue);
                 if (!needsRay) return;
                 if (general) {
 #pragma unroll
                     for (int k = 0; k < kLanes; ++k)
                         if (lanes >> k & 1u)
-                            p.shadowFactors[contributionIndex(first + k, lightSlots, j)] = make_float4(at(a, k), at(g1, k), at(g2, k), at(g3, k));
+                            p.shadowFactors[(first + k) * lightSlots + j] = make_float4(at(a, k), at(g1, k), at(g2, k), at(g3, k));
                 }
                 emitShadow(p, group, kLanes == 3 ? lanes : entry & 7u, kind | (j << 2) | (general ? kShadowGeneral : 0u) | (index << 8),
                            offsetSurfaceOrigin(hit, orientedGeometricNormal, direction), direction, traceDistance);
@@ -816,7 +872,7 @@ __global__ void __launch_bounds__((shadeThreads<kLanes, kFull>()), (shadeMinBloc
                             const V value = a * (misWeight / V(lightPdf));
 #pragma unroll
                             for (int k = 0; k < kLanes; ++k)
-                                if (lit >> k & 1u) p.contribution[contributionIndex(first + k, lightSlots, 1u)] = at(value, k);
+                                if (lit >> k & 1u) p.contribution[contributionIndex(first + k, 1u)] = at(value, k);
                             if (!(maxDistance <= 0.001f)) {
                                 emitShadow(p, group, kLanes == 3 ? lit : entry & 7u, kShadowMesh | (1u << 2),
                                            offsetSurfaceOrigin(hit, orientedGeometricNormal, lightDirection), lightDirection, maxDistance);
@@ -831,7 +887,7 @@ __global__ void __launch_bounds__((shadeThreads<kLanes, kFull>()), (shadeMinBloc
             open &= ~lanes;
             }
 
-            if (!kReplay) storeRadiance();
+            storeLight();
             if (lastBounce) continue;  // the same for every thread
             __syncthreads();
 
@@ -1025,8 +1081,7 @@ __global__ void __launch_bounds__((shadeThreads<kLanes, kFull>()), (shadeMinBloc
             }
     }
     if (!misses) return;
-    // The bounce's misses (:1245-1255), at the end of the launch rather than in
-    // one of their own: the environment, looked up once per entry.
+    // The bounce's misses, at the end of the launch rather than in one of their own.
     const uint32_t missCount = p.counters[kCountMisses];
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < missCount; i += gridDim.x * blockDim.x)
         shadeMiss(s, f, p, p.missQueue[i], lightSlots);

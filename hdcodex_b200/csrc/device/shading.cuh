@@ -30,16 +30,16 @@ HDCX_D Spectrum makeSpectrum(float wavelength)
 {
     Spectrum s;
     s.wavelength = wavelength;
-    s.br = gexp(-0.5f * gpow2((wavelength - 620.0f) / 30.0f));
-    s.bg = gexp(-0.5f * gpow2((wavelength - 535.0f) / 25.0f));
-    s.bb = gexp(-0.5f * gpow2((wavelength - 450.0f) / 20.0f));
+    s.br = hdcx_fp_exp(-0.5f * gpow2((wavelength - 620.0f) / 30.0f));
+    s.bg = hdcx_fp_exp(-0.5f * gpow2((wavelength - 535.0f) / 25.0f));
+    s.bb = hdcx_fp_exp(-0.5f * gpow2((wavelength - 450.0f) / 20.0f));
     s.denominator = gmax(s.br + s.bg + s.bb, 1e-5f);
     const float temperature = 6504.0f;
     const float c2 = 1.4387769e7f;
     const float referenceWavelength = 560.0f;
     s.planck = gpow5(referenceWavelength / wavelength) *
-               (gexp(c2 / (referenceWavelength * temperature)) - 1.0f) /
-               gmax(gexp(c2 / (wavelength * temperature)) - 1.0f, 1e-5f);
+               (hdcx_fp_exp(c2 / (referenceWavelength * temperature)) - 1.0f) /
+               gmax(hdcx_fp_exp(c2 / (wavelength * temperature)) - 1.0f, 1e-5f);
     return s;
 }
 
@@ -99,10 +99,10 @@ HDCX_D float3 cieXyz(float wavelength)
     const float ty2 = (wavelength - 530.9f) * (wavelength < 530.9f ? 0.0613f : 0.0322f);
     const float tz1 = (wavelength - 437.0f) * (wavelength < 437.0f ? 0.0845f : 0.0278f);
     const float tz2 = (wavelength - 459.0f) * (wavelength < 459.0f ? 0.0385f : 0.0725f);
-    return f3(0.362f * gexp(-0.5f * tx1 * tx1) + 1.056f * gexp(-0.5f * tx2 * tx2) -
-                  0.065f * gexp(-0.5f * tx3 * tx3),
-              0.821f * gexp(-0.5f * ty1 * ty1) + 0.286f * gexp(-0.5f * ty2 * ty2),
-              1.217f * gexp(-0.5f * tz1 * tz1) + 0.681f * gexp(-0.5f * tz2 * tz2));
+    return f3(0.362f * hdcx_fp_exp(-0.5f * tx1 * tx1) + 1.056f * hdcx_fp_exp(-0.5f * tx2 * tx2) -
+                  0.065f * hdcx_fp_exp(-0.5f * tx3 * tx3),
+              0.821f * hdcx_fp_exp(-0.5f * ty1 * ty1) + 0.286f * hdcx_fp_exp(-0.5f * ty2 * ty2),
+              1.217f * hdcx_fp_exp(-0.5f * tz1 * tz1) + 0.681f * hdcx_fp_exp(-0.5f * tz2 * tz2));
 }
 HDCX_D float3 sensorXyz(float wavelength) { return cieXyz(wavelength) * (400.0f / 106.856895f); }
 HDCX_D float3 spectralSensor(float wavelength)

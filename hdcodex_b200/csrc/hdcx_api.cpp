@@ -115,15 +115,14 @@ struct PathStore {
         p.capacity = n;
         p.wavePaths = n;
         p.shadowPerPath = shadowPerPath;
-        p.wavelength = alloc<float>(n);
-        p.spectrum = alloc<float4>(n);
-        p.throughput = alloc<float>(n);
-        p.radiance = alloc<float>(n);
+        const uint64_t groups = n / 3u + 1u;
+        p.laneLight = alloc<float4>(2 * groups);
+        p.laneState = alloc<float4>(3 * groups);
+        p.laneSpectrum = alloc<float4>(4 * groups);
         p.ray = alloc<float4>(2 * n);
-        p.previousPdf = alloc<float2>(n);
         p.medium = alloc<float4>(n);
         p.hit = alloc<float4>(n);
-        p.contribution = alloc<float>(3 * n);
+        p.contribution = alloc<float>(2 * n);
         p.queue[0] = alloc<uint32_t>(n);
         p.queue[1] = alloc<uint32_t>(n);
         p.groupQueue = alloc<uint32_t>(n / 2 + 1);

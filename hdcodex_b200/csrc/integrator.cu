@@ -50,6 +50,22 @@ struct WaveDesc {
     uint32_t count;        // samples * pixels * 3
 };
 
+// Pixel number `index` of the order in which a wave takes the image: bands of
+// four rows, in blocks of eight columns. The samples of a pixel are neighbours
+// in a wave and the pixels of a block too, so a warp's camera rays and first
+// hits lie close together.
+HDCX_D uint32_t tiledPixel(const FrameConst& f, uint32_t index)
+{
+    const uint32_t band = index / (f.width * 4u);
+    const uint32_t inBand = index - band * f.width * 4u;
+    const uint32_t rows = min(4u, f.height - band * 4u);
+    const uint32_t block = inBand / (8u * rows);
+    const uint32_t inBlock = inBand - block * 8u * rows;
+    const uint32_t columns = min(8u, f.width - block * 8u);
+    const uint32_t row = inBlock / columns;
+    return (band * 4u + row) * f.width + block * 8u + (inBlock - row * columns);
+}
+
 // ---------------------------------------------------------------------------
 // generate: main() prologue (vulkan_path_tracer.cpp:1191-1223), one thread
 // per group: the lanes of a sample share its seed, so its camera ray too.
@@ -63,8 +79,8 @@ __global__ void generateKernel(FrameConst f, WaveDesc w, PathBuffers p)
         *reinterpret_cast<unsigned long long*>(p.counters + kCountQueue0) = lanes | (p.split ? w.count : groups);
     }
     if (group >= groups) return;
-    const uint32_t pixel = w.pixelBase + group % w.pixels;
-    const uint32_t sampleNumber = f.sampleIndex + w.sampleBase + group / w.pixels;
+    const uint32_t pixel = tiledPixel(f, w.pixelBase + group / w.samples);
+    const uint32_t sampleNumber = f.sampleIndex + w.sampleBase + group % w.samples;
     const uint32_t px = pixel % f.width, py = pixel / f.width;
     const uint32_t index = pixel;
     uint32_t rng = hashState(index ^ (sampleNumber * 0x9e3779b9u) ^ 0xa511e9b3u);
@@ -74,17 +90,23 @@ __global__ void generateKernel(FrameConst f, WaveDesc w, PathBuffers p)
     const float u = (u2f(px) + jx) / u2f(f.width);
     const float v = (u2f(py) + jy) / u2f(f.height);
     const float3 direction = normalize(f.lowerLeft + u * f.horizontal + v * f.vertical - f.origin);
+    float wavelengths[3];
+#pragma unroll
+    for (uint32_t lane = 0; lane < 3u; ++lane) {
+        wavelengths[lane] =
+            380.0f + 400.0f * fract(wavelengthShift + (u2f(sampleNumber & 31u) + 0.5f) / 32.0f + u2f(lane) / 3.0f);
+        const Spectrum s = makeSpectrum(wavelengths[lane]);
+        p.laneSpectrum[4u * static_cast<size_t>(group) + lane] = make_float4(s.br, s.bg, s.bb, s.planck);
+    }
+    p.laneSpectrum[4u * static_cast<size_t>(group) + 3u] = make_float4(wavelengths[0], wavelengths[1], wavelengths[2], 0.0f);
+    float4* light = reinterpret_cast<float4*>(lightRecord(p, group));
+    light[0] = light[1] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    float4* record = reinterpret_cast<float4*>(laneRecord(p, group));
+    record[0] = make_float4(1.0f, 1.0f, 1.0f, 0.0f);
+    record[1] = record[2] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     for (uint32_t lane = 0; lane < 3u; ++lane) {
         const uint32_t slot = group * 3u + lane;
-        const float wavelength =
-            380.0f + 400.0f * fract(wavelengthShift + (u2f(sampleNumber & 31u) + 0.5f) / 32.0f + u2f(lane) / 3.0f);
-        const Spectrum s = makeSpectrum(wavelength);
-        p.wavelength[slot] = wavelength;
-        p.spectrum[slot] = make_float4(s.br, s.bg, s.bb, s.planck);
-        p.throughput[slot] = 1.0f;
-        p.radiance[slot] = 0.0f;
-        p.previousPdf[slot] = make_float2(0.0f, 0.0f);
-        for (uint32_t j = 0; j < p.lightSlots; ++j) p.contribution[contributionIndex(slot, p.lightSlots, j)] = 0.0f;
+        for (uint32_t j = 1; j < p.lightSlots; ++j) p.contribution[contributionIndex(slot, j)] = 0.0f;
         uint32_t flags = kFlagEnvironmentOnMiss | kFlagPreviousWasDelta;
         if (p.cache.enabled) {
             // Training paths: a deterministic subset chosen by the path identity.
@@ -179,17 +201,18 @@ HDCX_D void shadowEntry(const DeviceScene& s, const PathBuffers& p, uint32_t i, 
     }
     for (uint32_t lane = 0; lane < 3u; ++lane) {
         if (!(entry >> lane & 1u)) continue;
-        const uint32_t slot = (entry >> 3) * 3u + lane;
-        const uint32_t index = contributionIndex(slot, p.lightSlots, j);
+        const uint32_t group = entry >> 3, slot = group * 3u + lane;
         float value = 0.0f;
         if (general) {
-            const float4 fct = p.shadowFactors[index];
-            const Spectrum spec = spectrumFromBasis(p.wavelength[slot], p.spectrum[slot]);
+            const float4 fct = p.shadowFactors[slot * p.lightSlots + j];
+            const float* spectra = spectrumRecord(p, group);
+            const Spectrum spec = spectrumFromBasis(spectra[12u + lane], reinterpret_cast<const float4*>(spectra)[lane]);
             const float sv = reflectanceSpectrum(visibility, spec);
             const uint32_t kind = info & 3u;
             value = kind == kShadowAnalytic ? fct.x * sv * fct.y * fct.z / fct.w : (kind == kShadowSun ? fct.x * sv : fct.x * sv * fct.y);
         }
-        p.contribution[index] = value;
+        if (j == 0u) lightRecord(p, group)[kLaneLight + lane] = value;
+        else p.contribution[contributionIndex(slot, j)] = value;
     }
 }
 
@@ -273,8 +296,8 @@ __global__ void __launch_bounds__(128, HDCX_TRACE_MIN_BLOCKS)
         if (result == kWalkExits) {
             const uint32_t flags = kFlagEnvironmentOnMiss | kFlagPreviousWasDelta |
                                    (__float_as_uint(p.ray[2u * slot + 1u].w) & (kFlagInsideMedium | kFlagTraining));
-            p.throughput[slot] = state.z * w.attenuation;
-            p.previousPdf[slot] = make_float2(0.0f, p.previousPdf[slot].y);
+            laneRecord(p, slot / 3u)[kLaneThroughput + slot % 3u] = state.z * w.attenuation;
+            laneRecord(p, slot / 3u)[kLaneBsdfPdf + slot % 3u] = 0.0f;
             p.ray[2u * slot] = make_float4(w.origin.x, w.origin.y, w.origin.z, __uint_as_float(w.rng));
             p.ray[2u * slot + 1u] = make_float4(w.direction.x, w.direction.y, w.direction.z, __uint_as_float(flags));
             if (p.cone != nullptr) p.cone[slot] = make_float2(0.0f, -1.0f);
@@ -291,32 +314,77 @@ __global__ void __launch_bounds__(128, HDCX_TRACE_MIN_BLOCKS)
 // ---------------------------------------------------------------------------
 // accumulate: sensor and per-pixel batch sums (vulkan_path_tracer.cpp:1882-1884)
 // ---------------------------------------------------------------------------
-__global__ void accumulateKernel(FrameConst f, WaveDesc w, PathBuffers p, float4* batch, double* batchXyz)
+//
+// A pixel's samples add up in order, but what each adds (fourteen exponentials
+// per sample) does not depend on the others: a thread per sample computes it,
+// then a thread per pixel adds the block's values (thread-per-pixel alone took
+// 1.48 ms for eight samples at 1920x1080).
+constexpr uint32_t kAccumulateThreads = 256;
+
+// What sample `group` adds: sensor RGB (a third of the lanes' sum) and XYZ.
+HDCX_D void sampleValue(const PathBuffers& p, uint32_t group, float3& rgb, double xyz[3])
 {
-    const uint32_t local = blockIdx.x * blockDim.x + threadIdx.x;
-    if (local >= w.pixels) return;
-    const uint32_t pixel = w.pixelBase + local;
-    float4 b = batch[pixel];
-    double bx = batchXyz[3 * pixel + 0], by = batchXyz[3 * pixel + 1], bz = batchXyz[3 * pixel + 2];
-    for (uint32_t sOff = 0; sOff < w.samples; ++sOff) {
-        float3 spectral = f3(0.0f);
-        double sx = 0.0, sy = 0.0, sz = 0.0;
-        for (uint32_t lane = 0; lane < 3u; ++lane) {
-            const uint32_t slot = (sOff * w.pixels + local) * 3u + lane;
-            float radiance = p.radiance[slot];
-            for (uint32_t j = 0; j < p.lightSlots; ++j) radiance += p.contribution[contributionIndex(slot, p.lightSlots, j)];
-            const float wavelength = p.wavelength[slot];
-            spectral = spectral + spectralSensor(wavelength) * radiance;
-            const float3 x = sensorXyz(wavelength);
-            sx = __dadd_rn(sx, __dmul_rn(static_cast<double>(x.x), static_cast<double>(radiance)));
-            sy = __dadd_rn(sy, __dmul_rn(static_cast<double>(x.y), static_cast<double>(radiance)));
-            sz = __dadd_rn(sz, __dmul_rn(static_cast<double>(x.z), static_cast<double>(radiance)));
-        }
-        b = make_float4(b.x + spectral.x / 3.0f, b.y + spectral.y / 3.0f, b.z + spectral.z / 3.0f, 0.0f);
-        bx = __dadd_rn(bx, __ddiv_rn(sx, 3.0));
-        by = __dadd_rn(by, __ddiv_rn(sy, 3.0));
-        bz = __dadd_rn(bz, __ddiv_rn(sz, 3.0));
+    const float4* light = reinterpret_cast<const float4*>(lightRecord(p, group));
+    const float4 la = light[0], lb = light[1], wl = p.laneSpectrum[4u * static_cast<size_t>(group) + 3u];
+    const float radiances[3] = {la.x + la.w, la.y + lb.x, la.z + lb.y}, wavelengths[3] = {wl.x, wl.y, wl.z};
+    float3 spectral = f3(0.0f);
+    double sx = 0.0, sy = 0.0, sz = 0.0;
+#pragma unroll
+    for (uint32_t lane = 0; lane < 3u; ++lane) {
+        float radiance = radiances[lane];
+        for (uint32_t j = 1; j < p.lightSlots; ++j) radiance += p.contribution[contributionIndex(group * 3u + lane, j)];
+        const float wavelength = wavelengths[lane];
+        spectral = spectral + spectralSensor(wavelength) * radiance;
+        const float3 x = sensorXyz(wavelength);
+        sx = __dadd_rn(sx, __dmul_rn(static_cast<double>(x.x), static_cast<double>(radiance)));
+        sy = __dadd_rn(sy, __dmul_rn(static_cast<double>(x.y), static_cast<double>(radiance)));
+        sz = __dadd_rn(sz, __dmul_rn(static_cast<double>(x.z), static_cast<double>(radiance)));
     }
+    rgb = f3(spectral.x / 3.0f, spectral.y / 3.0f, spectral.z / 3.0f);
+    xyz[0] = __ddiv_rn(sx, 3.0);
+    xyz[1] = __ddiv_rn(sy, 3.0);
+    xyz[2] = __ddiv_rn(sz, 3.0);
+}
+
+__global__ void __launch_bounds__(kAccumulateThreads) accumulateKernel(FrameConst f, WaveDesc w, PathBuffers p, float4* batch, double* batchXyz)
+{
+    __shared__ float3 rgbs[kAccumulateThreads];
+    __shared__ double xyzs[3][kAccumulateThreads];
+    // Pixels per block, and samples per pass (a pixel with more than the block
+    // has threads takes several).
+    const uint32_t step = min(w.samples, kAccumulateThreads);
+    const uint32_t pixels = kAccumulateThreads / step;
+    const uint32_t firstLocal = blockIdx.x * pixels;
+    const uint32_t local = firstLocal + threadIdx.x;
+    const bool adds = threadIdx.x < pixels && local < w.pixels;
+    const uint32_t pixel = adds ? tiledPixel(f, w.pixelBase + local) : 0u;
+    float4 b = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    double bx = 0.0, by = 0.0, bz = 0.0;
+    if (adds) {
+        b = batch[pixel];
+        bx = batchXyz[3 * pixel + 0], by = batchXyz[3 * pixel + 1], bz = batchXyz[3 * pixel + 2];
+    }
+    for (uint32_t base = 0; base < w.samples; base += step) {
+        const uint32_t mine = threadIdx.x / step, sample = base + threadIdx.x % step;
+        if (mine < pixels && firstLocal + mine < w.pixels && sample < w.samples) {
+            double xyz[3];
+            sampleValue(p, (firstLocal + mine) * w.samples + sample, rgbs[threadIdx.x], xyz);
+            for (int k = 0; k < 3; ++k) xyzs[k][threadIdx.x] = xyz[k];
+        }
+        __syncthreads();
+        if (adds) {
+            for (uint32_t s = 0; s < min(step, w.samples - base); ++s) {
+                const uint32_t t = threadIdx.x * step + s;
+                const float3 rgb = rgbs[t];
+                b = make_float4(b.x + rgb.x, b.y + rgb.y, b.z + rgb.z, 0.0f);
+                bx = __dadd_rn(bx, xyzs[0][t]);
+                by = __dadd_rn(by, xyzs[1][t]);
+                bz = __dadd_rn(bz, xyzs[2][t]);
+            }
+        }
+        __syncthreads();
+    }
+    if (!adds) return;
     batch[pixel] = b;
     batchXyz[3 * pixel + 0] = bx;
     batchXyz[3 * pixel + 1] = by;
@@ -371,7 +439,7 @@ __global__ void cacheApplyKernel(PathBuffers p)
     const uint32_t n = p.cache.counters[0];
     for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
         const uint32_t slot = p.cache.querySlot[j];
-        p.radiance[slot] += p.throughput[slot] * fmaxf(p.cache.predictions[j], 0.0f);
+        lightRecord(p, slot / 3u)[kLaneRadiance + slot % 3u] += laneRecord(p, slot / 3u)[kLaneThroughput + slot % 3u] * fmaxf(p.cache.predictions[j], 0.0f);
     }
 }
 
@@ -380,8 +448,9 @@ __global__ void cacheTargetsKernel(PathBuffers p)
     const uint32_t n = min(p.cache.counters[1], p.cache.trainCapacity);
     for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
         const uint32_t slot = p.cache.trainSlot[t];
-        float total = p.radiance[slot];
-        for (uint32_t j = 0; j < p.lightSlots; ++j) total += p.contribution[contributionIndex(slot, p.lightSlots, j)];
+        const float* light = lightRecord(p, slot / 3u) + slot % 3u;
+        float total = light[kLaneRadiance] + light[kLaneLight];
+        for (uint32_t j = 1; j < p.lightSlots; ++j) total += p.contribution[contributionIndex(slot, j)];
         const uint32_t vertices = min(p.cache.trainVertices[t], kCacheMaxVertices);
         for (uint32_t b = 0; b < vertices; ++b) {
             const uint32_t r = t * kCacheMaxVertices + b;
@@ -804,7 +873,8 @@ void renderFrame(const DeviceScene& sceneIn, const FrameConst& frame, PathBuffer
             launched += 2;
         }
         launched += 2;
-        accumulateKernel<<<(w.pixels + 255u) / 256u, 256, 0, stream>>>(frame, w, paths, fb.batch, fb.batchXyz);
+        const uint32_t blockPixels = kAccumulateThreads / std::min(w.samples, kAccumulateThreads);
+        accumulateKernel<<<(w.pixels + blockPixels - 1u) / blockPixels, kAccumulateThreads, 0, stream>>>(frame, w, paths, fb.batch, fb.batchXyz);
         CUDA_OK(cudaGetLastError());
     }
     finalizeKernel<<<(pixels + 255u) / 256u, 256, 0, stream>>>(frame, fb);
