@@ -86,17 +86,16 @@ HDCX_D void shadeMiss(const DeviceScene& s, const FrameConst& f, const PathBuffe
     const float4 basis[3] = {spectra[0], spectra[1], spectra[2]}, w = spectra[3];
     // Light samples of the previous bounce, in slot order.
     float radiance[3] = {l0.x + l0.w, l0.y + l1.x, l0.z + l1.y};
+    if (lightSlots > 1u) {
+        const float4 l2 = light[2];
+        radiance[0] = radiance[0] + l1.z + l2.y;
+        radiance[1] = radiance[1] + l1.w + l2.z;
+        radiance[2] = radiance[2] + l2.x + l2.w;
+    }
     const float throughput[3] = {a.x, a.y, a.z}, bsdfPdf[3] = {a.w, b.x, b.y}, lightPdf[3] = {b.z, b.w, c.x};
     const float wavelength[3] = {w.x, w.y, w.z};
 #pragma unroll
     for (uint32_t lane = 0; lane < 3u; ++lane) {
-        if (lightSlots > 1u && (entry >> lane & 1u)) {
-            for (uint32_t j = 1; j < lightSlots; ++j) {
-                float& pending = p.contribution[contributionIndex(group * 3u + lane, j)];
-                radiance[lane] += pending;
-                pending = 0.0f;
-            }
-        }
         if (lit) {
             const Spectrum spec = spectrumFromBasis(wavelength[lane], basis[lane]);
             const float misWeight = (flags & kFlagPreviousWasDelta) != 0u ? 1.0f : powerHeuristic(bsdfPdf[lane], lightPdf[lane]);
@@ -107,13 +106,14 @@ HDCX_D void shadeMiss(const DeviceScene& s, const FrameConst& f, const PathBuffe
     if ((entry & 7u) == 7u) {
         reinterpret_cast<float4*>(out)[0] = make_float4(radiance[0], radiance[1], radiance[2], 0.0f);
         reinterpret_cast<float4*>(out)[1] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (lightSlots > 1u) reinterpret_cast<float4*>(out)[2] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         return;
     }
 #pragma unroll
     for (uint32_t lane = 0; lane < 3u; ++lane) {
         if (!(entry >> lane & 1u)) continue;
         out[kLaneRadiance + lane] = radiance[lane];
-        out[kLaneLight + lane] = 0.0f;
+        for (uint32_t j = 0; j < lightSlots; ++j) out[kLaneLight + 3u * j + lane] = 0.0f;
     }
 }
 
@@ -301,6 +301,10 @@ __global__ void __launch_bounds__((shadeThreads<kLanes, kFull>()), (shadeMinBloc
             const float4* r = reinterpret_cast<const float4*>(record);
             const float4 l0 = l[0], l1 = l[1], a = r[0], b = r[1], c = r[2];
             radiance = Lanes3(l0.x, l0.y, l0.z) + Lanes3(l0.w, l1.x, l1.y);
+            if (!kLit && lightSlots > 1u) {
+                const float4 l2 = l[2];
+                radiance = radiance + Lanes3(l1.z, l1.w, l2.x) + Lanes3(l2.y, l2.z, l2.w);
+            }
             throughput = Lanes3(a.x, a.y, a.z);
             previousBsdfPdf = Lanes3(a.w, b.x, b.y);
             previousEnvironmentLightPdf = Lanes3(b.z, b.w, c.x);
@@ -316,29 +320,17 @@ __global__ void __launch_bounds__((shadeThreads<kLanes, kFull>()), (shadeMinBloc
             throughput = record[kLaneThroughput + onlyLane];
             radiance = lightOf[kLaneRadiance + onlyLane];
             if (!kReplay) radiance += lightOf[kLaneLight + onlyLane];
+            if (!kReplay && !kLit && lightSlots > 1u) {
+                radiance += lightOf[kLaneLight + 3u + onlyLane];
+                radiance += lightOf[kLaneLight + 6u + onlyLane];
+            }
             previousBsdfPdf = record[kLaneBsdfPdf + onlyLane];
             previousEnvironmentLightPdf = record[kLaneLightPdf + onlyLane];
             const float* q = spectrumRecord(p, group);
             spec = spectrumFromBasis(q[12u + onlyLane], reinterpret_cast<const float4*>(q)[onlyLane]);
         }
-        if (!kReplay && !kLit && lightSlots > 1u) {
-            // All loads before the clears, as in shadeMiss.
-            V second = V(0.0f), third = V(0.0f);
-#pragma unroll
-            for (int k = 0; k < kLanes; ++k) {
-                if (!(mask >> k & 1u)) continue;
-                put(second, k, p.contribution[contributionIndex(first + k, 1u)]);
-                if (lightSlots > 2u) put(third, k, p.contribution[contributionIndex(first + k, 2u)]);
-            }
-            radiance = radiance + second;
-            if (lightSlots > 2u) radiance = radiance + third;
-#pragma unroll
-            for (int k = 0; k < kLanes; ++k) {
-                if (at(second, k) != 0.0f) p.contribution[contributionIndex(first + k, 1u)] = 0.0f;
-                if (at(third, k) != 0.0f) p.contribution[contributionIndex(first + k, 2u)] = 0.0f;
-            }
-        }
-        V lightValue = V(0.0f);  // this bounce's light-sample slot 0
+        // This bounce's light-sample slots.
+        V lightValue = V(0.0f), secondValue = V(0.0f), thirdValue = V(0.0f);
         // Ray cone (width, spread) of texture LOD; spread <= 0: level 0.
         const bool lodOn = kFull && f.pixelSpread > 0.0f && p.cone != nullptr;
         const float2 cone = lodOn ? p.cone[slot] : make_float2(0.0f, -1.0f);
@@ -381,7 +373,9 @@ __global__ void __launch_bounds__((shadeThreads<kLanes, kFull>()), (shadeMinBloc
             if (kLanes == 3 && mask == 7u) {
                 float4* l = reinterpret_cast<float4*>(lightOf);
                 l[0] = make_float4(at(radiance, 0), at(radiance, 1), at(radiance, 2), at(lightValue, 0));
-                l[1] = make_float4(at(lightValue, 1), at(lightValue, 2), 0.0f, 0.0f);
+                l[1] = make_float4(at(lightValue, 1), at(lightValue, 2), at(secondValue, 0), at(secondValue, 1));
+                if (!kLit && lightSlots > 1u)
+                    l[2] = make_float4(at(secondValue, 2), at(thirdValue, 0), at(thirdValue, 1), at(thirdValue, 2));
                 return;
             }
 #pragma unroll
@@ -390,6 +384,10 @@ __global__ void __launch_bounds__((shadeThreads<kLanes, kFull>()), (shadeMinBloc
                 const uint32_t lane = kLanes == 3 ? static_cast<uint32_t>(k) : onlyLane;
                 lightOf[kLaneRadiance + lane] = at(radiance, k);
                 lightOf[kLaneLight + lane] = at(lightValue, k);
+                if (!kLit && lightSlots > 1u) {
+                    lightOf[kLaneLight + 3u + lane] = at(secondValue, k);
+                    lightOf[kLaneLight + 6u + lane] = at(thirdValue, k);
+                }
             }
         };
 
@@ -688,10 +686,10 @@ __global__ void __launch_bounds__((shadeThreads<kLanes, kFull>()), (shadeMinBloc
 #pragma unroll
                 for (int k = 0; k < kLanes; ++k) {
                     if (!(lanes >> k & 1u)) continue;
-                    if (j != 0u) p.contribution[contributionIndex(first + k, j)] = at(value, k);
                     general = general || !isfinite(at(value, k));
                 }
-                if (j == 0u) lightValue = whereMask(lanes, value, lightValue);
+                V& slotValue = j == 0u ? lightValue : (j == 1u ? secondValue : thirdValue);
+                slotValue = whereMask(lanes, value, slotValue);
                 if (!needsRay) return;
                 if (general) {
 #pragma unroll
@@ -870,9 +868,7 @@ __global__ void __launch_bounds__((shadeThreads<kLanes, kFull>()), (shadeMinBloc
                             const V a = throughput * direct * spectralLight;
                             const float maxDistance = gmax(lightDistance - 0.003f, 0.001f);
                             const V value = a * (misWeight / V(lightPdf));
-#pragma unroll
-                            for (int k = 0; k < kLanes; ++k)
-                                if (lit >> k & 1u) p.contribution[contributionIndex(first + k, 1u)] = at(value, k);
+                            secondValue = whereMask(lit, value, secondValue);
                             if (!(maxDistance <= 0.001f)) {
                                 emitShadow(p, group, kLanes == 3 ? lit : entry & 7u, kShadowMesh | (1u << 2),
                                            offsetSurfaceOrigin(hit, orientedGeometricNormal, lightDirection), lightDirection, maxDistance);

@@ -105,10 +105,10 @@ HDCX_D float3 cieXyz(float wavelength)
               1.217f * hdcx_fp_exp(-0.5f * tz1 * tz1) + 0.681f * hdcx_fp_exp(-0.5f * tz2 * tz2));
 }
 HDCX_D float3 sensorXyz(float wavelength) { return cieXyz(wavelength) * (400.0f / 106.856895f); }
-HDCX_D float3 spectralSensor(float wavelength)
+// The sensor's RGB of a wavelength, from its sensorXyz.
+HDCX_D float3 spectralSensor(float3 x)
 {
     // :172-179
-    const float3 x = sensorXyz(wavelength);
     return f3(3.2404542f * x.x - 1.5371385f * x.y - 0.4985314f * x.z,
               -0.9692660f * x.x + 1.8760108f * x.y + 0.0415560f * x.z,
               0.0556434f * x.x - 0.2040259f * x.y + 1.0572252f * x.z);

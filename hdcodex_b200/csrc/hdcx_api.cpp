@@ -116,13 +116,12 @@ struct PathStore {
         p.wavePaths = n;
         p.shadowPerPath = shadowPerPath;
         const uint64_t groups = n / 3u + 1u;
-        p.laneLight = alloc<float4>(2 * groups);
+        p.laneLight = alloc<float4>(3 * groups);
         p.laneState = alloc<float4>(3 * groups);
         p.laneSpectrum = alloc<float4>(4 * groups);
         p.ray = alloc<float4>(2 * n);
         p.medium = alloc<float4>(n);
         p.hit = alloc<float4>(n);
-        p.contribution = alloc<float>(2 * n);
         p.queue[0] = alloc<uint32_t>(n);
         p.queue[1] = alloc<uint32_t>(n);
         p.groupQueue = alloc<uint32_t>(n / 2 + 1);

@@ -101,12 +101,12 @@ __global__ void generateKernel(FrameConst f, WaveDesc w, PathBuffers p)
     p.laneSpectrum[4u * static_cast<size_t>(group) + 3u] = make_float4(wavelengths[0], wavelengths[1], wavelengths[2], 0.0f);
     float4* light = reinterpret_cast<float4*>(lightRecord(p, group));
     light[0] = light[1] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (p.lightSlots > 1u) light[2] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     float4* record = reinterpret_cast<float4*>(laneRecord(p, group));
     record[0] = make_float4(1.0f, 1.0f, 1.0f, 0.0f);
     record[1] = record[2] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     for (uint32_t lane = 0; lane < 3u; ++lane) {
         const uint32_t slot = group * 3u + lane;
-        for (uint32_t j = 1; j < p.lightSlots; ++j) p.contribution[contributionIndex(slot, j)] = 0.0f;
         uint32_t flags = kFlagEnvironmentOnMiss | kFlagPreviousWasDelta;
         if (p.cache.enabled) {
             // Training paths: a deterministic subset chosen by the path identity.
@@ -211,8 +211,7 @@ HDCX_D void shadowEntry(const DeviceScene& s, const PathBuffers& p, uint32_t i, 
             const uint32_t kind = info & 3u;
             value = kind == kShadowAnalytic ? fct.x * sv * fct.y * fct.z / fct.w : (kind == kShadowSun ? fct.x * sv : fct.x * sv * fct.y);
         }
-        if (j == 0u) lightRecord(p, group)[kLaneLight + lane] = value;
-        else p.contribution[contributionIndex(slot, j)] = value;
+        lightRecord(p, group)[kLaneLight + 3u * j + lane] = value;
     }
 }
 
@@ -326,16 +325,21 @@ HDCX_D void sampleValue(const PathBuffers& p, uint32_t group, float3& rgb, doubl
 {
     const float4* light = reinterpret_cast<const float4*>(lightRecord(p, group));
     const float4 la = light[0], lb = light[1], wl = p.laneSpectrum[4u * static_cast<size_t>(group) + 3u];
-    const float radiances[3] = {la.x + la.w, la.y + lb.x, la.z + lb.y}, wavelengths[3] = {wl.x, wl.y, wl.z};
+    float radiances[3] = {la.x + la.w, la.y + lb.x, la.z + lb.y};
+    if (p.lightSlots > 1u) {
+        const float4 lc = light[2];
+        radiances[0] = radiances[0] + lb.z + lc.y;
+        radiances[1] = radiances[1] + lb.w + lc.z;
+        radiances[2] = radiances[2] + lc.x + lc.w;
+    }
+    const float wavelengths[3] = {wl.x, wl.y, wl.z};
     float3 spectral = f3(0.0f);
     double sx = 0.0, sy = 0.0, sz = 0.0;
 #pragma unroll
     for (uint32_t lane = 0; lane < 3u; ++lane) {
-        float radiance = radiances[lane];
-        for (uint32_t j = 1; j < p.lightSlots; ++j) radiance += p.contribution[contributionIndex(group * 3u + lane, j)];
-        const float wavelength = wavelengths[lane];
-        spectral = spectral + spectralSensor(wavelength) * radiance;
-        const float3 x = sensorXyz(wavelength);
+        const float radiance = radiances[lane];
+        const float3 x = sensorXyz(wavelengths[lane]);
+        spectral = spectral + spectralSensor(x) * radiance;
         sx = __dadd_rn(sx, __dmul_rn(static_cast<double>(x.x), static_cast<double>(radiance)));
         sy = __dadd_rn(sy, __dmul_rn(static_cast<double>(x.y), static_cast<double>(radiance)));
         sz = __dadd_rn(sz, __dmul_rn(static_cast<double>(x.z), static_cast<double>(radiance)));
@@ -450,7 +454,7 @@ __global__ void cacheTargetsKernel(PathBuffers p)
         const uint32_t slot = p.cache.trainSlot[t];
         const float* light = lightRecord(p, slot / 3u) + slot % 3u;
         float total = light[kLaneRadiance] + light[kLaneLight];
-        for (uint32_t j = 1; j < p.lightSlots; ++j) total += p.contribution[contributionIndex(slot, j)];
+        for (uint32_t j = 1; j < p.lightSlots; ++j) total += light[kLaneLight + 3u * j];
         const uint32_t vertices = min(p.cache.trainVertices[t], kCacheMaxVertices);
         for (uint32_t b = 0; b < vertices; ++b) {
             const uint32_t r = t * kCacheMaxVertices + b;

@@ -69,13 +69,12 @@ struct PathBuffers {
     uint32_t split = 0;             // 1: every lane travels as an entry of its own from the start
     uint32_t merged = 0;            // 1: hitQueue takes every entry, groupQueue none
     uint32_t shadowWord = 0;        // counter of the bounce's shadow queue
-    float4* laneLight = nullptr;    // two per group: kLaneRadiance, kLaneLight of its lanes (device/paths.cuh)
+    float4* laneLight = nullptr;    // two (lightSlots = 1) or three per group: kLaneRadiance, kLaneLight of its lanes (device/paths.cuh)
     float4* laneState = nullptr;    // three per group: kLaneThroughput, kLaneBsdfPdf, kLaneLightPdf of its lanes
     float4* laneSpectrum = nullptr; // four per group: basis r, g, b and Planck factor of each lane, their wavelengths
     float4* ray = nullptr;          // at leaders, two per slot: origin and RNG state, direction and flags
     float4* medium = nullptr;       // absorption, scattering, anisotropy
     float4* hit = nullptr;          // at leaders: t, primitive (bits), b1, b2
-    float* contribution = nullptr;  // 2 * capacity: light-sample slots 1 and 2 of each path slot (slot 0: laneLight)
     uint32_t* queue[2] = {nullptr, nullptr};  // extension entries
     uint32_t* groupQueue = nullptr;     // extend's output: entries of several lanes whose ray hit
     uint32_t* hitQueue = nullptr;       // extend's output: entries of one lane whose ray hit (all of them if merged)

@@ -40,13 +40,12 @@ constexpr uint64_t alignUp(uint64_t v) { return (v + kAlign - 1) / kAlign * kAli
 constexpr uint64_t kN = kStaticWavePaths;
 constexpr uint64_t kShadow = kN * kStaticShadowPerPath;
 constexpr uint64_t kRegionBytes[] = {
-    32 * (kN / 3 + 1),             // laneLight
+    48 * (kN / 3 + 1),             // laneLight
     48 * (kN / 3 + 1),             // laneState
     64 * (kN / 3 + 1),             // laneSpectrum
     32 * kN,                       // ray
     16 * kN,                       // medium
     16 * kN,                       // hit
-    4 * 2 * kN,                    // contribution (light-sample slots 1 and 2)
     4 * kN,                        // queue[0]
     4 * kN,                        // queue[1]
     4 * (kN / 2 + 1),              // groupQueue
@@ -126,24 +125,23 @@ unsigned int renderStatic(const DeviceScene& scene, const FrameConst& frame, flo
     p.ray = reinterpret_cast<float4*>(region[3]);
     p.medium = reinterpret_cast<float4*>(region[4]);
     p.hit = reinterpret_cast<float4*>(region[5]);
-    p.contribution = reinterpret_cast<float*>(region[6]);
-    p.queue[0] = reinterpret_cast<uint32_t*>(region[7]);
-    p.queue[1] = reinterpret_cast<uint32_t*>(region[8]);
-    p.groupQueue = reinterpret_cast<uint32_t*>(region[9]);
-    p.hitQueue = reinterpret_cast<uint32_t*>(region[10]);
-    p.missQueue = reinterpret_cast<uint32_t*>(region[11]);
-    p.shadowRay = reinterpret_cast<float4*>(region[12]);
-    p.shadowFactors = reinterpret_cast<float4*>(region[13]);
-    p.shadowInfo = reinterpret_cast<uint32_t*>(region[14]);
-    p.counters = reinterpret_cast<uint32_t*>(region[15]);
-    p.stats = reinterpret_cast<unsigned long long*>(region[16]);
+    p.queue[0] = reinterpret_cast<uint32_t*>(region[6]);
+    p.queue[1] = reinterpret_cast<uint32_t*>(region[7]);
+    p.groupQueue = reinterpret_cast<uint32_t*>(region[8]);
+    p.hitQueue = reinterpret_cast<uint32_t*>(region[9]);
+    p.missQueue = reinterpret_cast<uint32_t*>(region[10]);
+    p.shadowRay = reinterpret_cast<float4*>(region[11]);
+    p.shadowFactors = reinterpret_cast<float4*>(region[12]);
+    p.shadowInfo = reinterpret_cast<uint32_t*>(region[13]);
+    p.counters = reinterpret_cast<uint32_t*>(region[14]);
+    p.stats = reinterpret_cast<unsigned long long*>(region[15]);
 
     FrameBuffers fb;
     fb.width = frame.width;
     fb.height = frame.height;
     fb.rgba = rgba;
-    fb.batch = reinterpret_cast<float4*>(region[17]);
-    fb.batchXyz = reinterpret_cast<double*>(region[18]);
+    fb.batch = reinterpret_cast<float4*>(region[16]);
+    fb.batchXyz = reinterpret_cast<double*>(region[17]);
     // The frame's FP64 XYZ running sums are not kept by this variant: the
     // finalize pass adds them into the batch sums of the same pixel (each
     // thread reads and writes only its own pixel), which the next call clears.

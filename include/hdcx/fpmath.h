@@ -166,9 +166,13 @@ HDCX_FP float hdcx_fp_cos(float x)
 
 HDCX_FP float hdcx_fp_exp(float x)
 {
+#if !defined(__CUDA_ARCH__)
+    /* On the GPU these cases are picked at the end, so that a warp runs one
+     * sequence without branches. */
     if (!(x == x)) return x;
     if (x > 88.72283935546875f) return hdcx_fp_bits_to_float(0x7f800000u);
     if (x < -103.97208404541015625f) return 0.0f;
+#endif
     const float k = hdcx_fp_round(x * 1.4426950408889634074f);
     float r = HDCX_FP_FMA(k, -0.693145751953125f, x);       /* ln2 high part */
     r = HDCX_FP_FMA(k, -1.428606765330187045e-6f, r);         /* ln2 low part */
@@ -182,9 +186,17 @@ HDCX_FP float hdcx_fp_exp(float x)
     p = HDCX_FP_FMA(p, r, 1.0f);
     p = HDCX_FP_FMA(p, r, 1.0f);
     const int32_t ki = (int32_t)k;
-    /* Scale in two steps so that 2^k never overflows or flushes early. */
+    /* Scale in two steps so that 2^k never overflows or flushes early: k lies
+     * in [-150, 128], so both halves are exponents of normal numbers. */
     const int32_t k1 = ki / 2;
-    return (p * hdcx_fp_pow2i(k1)) * hdcx_fp_pow2i(ki - k1);
+    const float scaled = (p * hdcx_fp_bits_to_float((uint32_t)(k1 + 127) << 23)) *
+                         hdcx_fp_bits_to_float((uint32_t)(ki - k1 + 127) << 23);
+#if defined(__CUDA_ARCH__)
+    if (!(x == x)) return x;
+    if (x > 88.72283935546875f) return hdcx_fp_bits_to_float(0x7f800000u);
+    if (x < -103.97208404541015625f) return 0.0f;
+#endif
+    return scaled;
 }
 
 HDCX_FP float hdcx_fp_log(float x)
