@@ -50,6 +50,7 @@ enum class Accept : int {
     Opaque = 0,      // every candidate is confirmed
     Stochastic = 1,  // confirmed iff anyHitThreshold(rayRng, prim) <= opacity
     Threshold = 2,   // confirmed iff opacity >= 0.5
+    Boundary = 3,    // Opaque; of hits farther than `enough`, any one will do
 };
 
 struct HitRecord {
@@ -191,6 +192,7 @@ struct Traversal {
     float bestT;
     uint32_t bestPrim;
     float bestB1, bestB2;
+    float enough;     // Accept::Boundary only
     uint2 nodeGroup;  // x: base index of the internal children; y: hit bits in 24..31 (by visiting order) | imask
     uint2 triGroup;   // x: first triangle slot; y: bits of the triangles left to test
     uint32_t triMask; // the node's triangle bits (see testNode)
@@ -323,7 +325,7 @@ HDCX_D bool testTriangle(Traversal& st, const DeviceScene& s, uint2* work)
     const uint32_t prim = __float_as_uint(w0.w);
     if (!kAny) {
         if (t > st.bestT) return false;
-        if (t == st.bestT && prim > st.bestPrim) return false;
+        if (kMode != Accept::Boundary && t == st.bestT && prim > st.bestPrim) return false;
     }
     if (kMode == Accept::Stochastic) {
         // The threshold lies in [0, 1]: an opacity of 1 always confirms.
@@ -333,6 +335,14 @@ HDCX_D bool testTriangle(Traversal& st, const DeviceScene& s, uint2* work)
         if (!(leafOpacity(w1.w, s, prim, b1, b2) >= 0.5f)) return false;
     }
     if (kAny) return true;
+    if (kMode == Accept::Boundary) {
+        // Any hit beyond `enough` ends the search beyond it; each hit found
+        // after another is at most as far.
+        st.bestT = fminf(t, st.enough);
+        st.bestB1 = t;
+        st.bestPrim = prim;
+        return false;
+    }
     st.bestT = t;
     st.bestPrim = prim;
     st.bestB1 = b1;
@@ -566,13 +576,14 @@ HDCX_D bool traceInstanced(const DeviceScene& s, float3 o, float3 d, float tmin,
 // into *fault.
 template <Accept kMode, bool kAny, bool kCount = false, int kInst = -1>
 HDCX_D bool traceRay(const DeviceScene& s, float3 o, float3 d, float tmin, float tmax, uint32_t rayRng, HitRecord& hit,
-                     uint32_t& fault, uint2* work = nullptr)
+                     uint32_t& fault, uint2* work = nullptr, float enough = 0.0f)
 {
     if (s.nodeCount == 0u) return false;
     if (kInst == 1 || (kInst == -1 && s.instances != nullptr))
-        return traceInstanced<kMode, kAny, kCount>(s, o, d, tmin, tmax, rayRng, hit, work, fault);
+        return traceInstanced<kMode == Accept::Boundary ? Accept::Opaque : kMode, kAny, kCount>(s, o, d, tmin, tmax, rayRng, hit, work, fault);
     Traversal st;
     beginTraversal(st, s, o, d, tmin, tmax, rayRng);
+    st.enough = enough;
     uint2 stack[kTraversalStack];
     int r;
     while ((r = traversalStep<kMode, kAny, kCount>(st, stack, s, work)) == kStepContinue) {
@@ -580,7 +591,7 @@ HDCX_D bool traceRay(const DeviceScene& s, float3 o, float3 d, float tmin, float
     fault |= st.fault;
     if (kAny) return r == kStepAnyHit;
     if (st.bestPrim == kInvalidPrimitive) return false;
-    hit.t = st.bestT;
+    hit.t = kMode == Accept::Boundary ? st.bestB1 : st.bestT;
     hit.primitive = st.bestPrim;
     hit.b1 = st.bestB1;
     hit.b2 = st.bestB2;

@@ -43,10 +43,16 @@ template <int kInst = -1>
 __device__ __forceinline__ int stepWalk(const DeviceScene& s, SubsurfaceWalk& w, uint32_t& fault)
 {
     HitRecord h;
-    if (!traceRay<Accept::Opaque, false, false, kInst>(s, w.origin, w.direction, 0.001f, 10000.0f, 0u, h, fault)) return kWalkFails;
-    const float boundaryDistance = h.t;
-    const float scatterDistance = -glog(gmax(1.0f - randomFloat(w.rng), 1e-6f)) / w.sigmaS;
+    uint32_t rng = w.rng;
+    const float scatterDistance = -glog(gmax(1.0f - randomFloat(rng), 1e-6f)) / w.sigmaS;
     const bool forceExit = w.step == kWalkSteps - 1;
+    // The boundary's distance counts only up to the scattering event's: beyond
+    // it, that there is a boundary is enough.
+    if (!traceRay<Accept::Boundary, false, false, kInst>(s, w.origin, w.direction, 0.001f, 10000.0f, 0u, h, fault, nullptr,
+                                                        forceExit ? INFINITY : scatterDistance))
+        return kWalkFails;
+    w.rng = rng;
+    const float boundaryDistance = h.t;
     const float travel = forceExit ? boundaryDistance : gmin(scatterDistance, boundaryDistance);
     w.attenuation = w.attenuation * gexp(-w.sigmaA * travel);
     if (forceExit || scatterDistance >= boundaryDistance) {
