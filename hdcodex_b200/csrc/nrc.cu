@@ -299,8 +299,9 @@ __device__ __forceinline__ void issueForward(uint32_t dTmem, const __nv_bfloat16
 // with its own activations, tensor-memory columns and barriers; the weights
 // (35 KB) are shared. A tile is a chain of five dependent GEMMs, each far too
 // small for the tensor pipe, so the kernel runs at tiles in flight per SM:
-// two blocks of four tiles fit (99 KB each) where blocks of one tile (51 KB)
-// fitted four.
+// two blocks of four tiles fit (99 KB each), eight tiles where blocks of one
+// (51 KB) fitted four. Both measured the same, 28.5 and 28.2 us per 2^18
+// queries; four read the weights a quarter as often.
 constexpr uint32_t kQueryGroups = 4;
 constexpr uint32_t kQueryThreads = kQueryGroups * 128u;
 constexpr uint32_t kQuerySmem = kWeightCount * 2u + kQueryGroups * kTile * kWidth * 2u + (kQueryGroups + 1u) * 8u;
@@ -555,42 +556,47 @@ __global__ void __launch_bounds__(128) trainKernel(DeviceParams p, const float* 
 // to the table's FP32 gradients. One thread per record and kEncodeLevels
 // levels, a two-float vector atomic per corner. (Inside trainKernel, with one
 // block of four warps per SM, the scatter waited on its own latency: 228 us a
-// step of 2^16 records for the whole kernel.)
+// step of 2^16 records for the whole kernel.) Records are taken in waves of a
+// tile per SM, as trainKernel takes them: an entry's sum forms nearly in the
+// order of the records, and runs differ no more than that. With all records of
+// a call in flight the same sums came out in any order, and single parameters
+// whose gradients nearly cancel moved by a learning rate three times as often
+// (four steps of 2^16 records: 569 us in any order, 579 us in waves).
 __global__ void __launch_bounds__(256) scatterKernel(DeviceParams p, const float* queries, const float* featureGrad, uint32_t count,
                                                      float* gridGrad)
 {
-    const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= count) return;
-    // Scalar loads: callers' records need no more than float alignment.
-    const float* record = queries + static_cast<size_t>(q) * kQueryFloats;
-    const float3 pos = make_float3(__ldg(record), __ldg(record + 1), __ldg(record + 2));
-    const int firstLevel = static_cast<int>(blockIdx.y) * kEncodeLevels;
-    const float4* row = reinterpret_cast<const float4*>(featureGrad + static_cast<size_t>(q) * kGridFeatures + 2 * firstLevel);
-    float d[2 * kEncodeLevels];
+    for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < count; q += gridDim.x * blockDim.x) {
+        // Scalar loads: callers' records need no more than float alignment.
+        const float* record = queries + static_cast<size_t>(q) * kQueryFloats;
+        const float3 pos = make_float3(__ldg(record), __ldg(record + 1), __ldg(record + 2));
+        const int firstLevel = static_cast<int>(blockIdx.y) * kEncodeLevels;
+        const float4* row = reinterpret_cast<const float4*>(featureGrad + static_cast<size_t>(q) * kGridFeatures + 2 * firstLevel);
+        float d[2 * kEncodeLevels];
 #pragma unroll
-    for (int i = 0; i < kEncodeLevels / 2; ++i) {
-        const float4 v = __ldg(row + i);
-        d[4 * i] = v.x, d[4 * i + 1] = v.y, d[4 * i + 2] = v.z, d[4 * i + 3] = v.w;
-    }
+        for (int i = 0; i < kEncodeLevels / 2; ++i) {
+            const float4 v = __ldg(row + i);
+            d[4 * i] = v.x, d[4 * i + 1] = v.y, d[4 * i + 2] = v.z, d[4 * i + 3] = v.w;
+        }
 #pragma unroll
-    for (int l = 0; l < kEncodeLevels; ++l) {
-        const float d0 = d[2 * l], d1 = d[2 * l + 1];
-        if (d0 == 0.0f && d1 == 0.0f) continue;
-        uint32_t index[8];
-        float weight[8];
-        levelCorners(p, firstLevel + l, pos, index, weight);
-        // Corners that differ in x share an aligned pair of entries when their
-        // indices differ in the lowest bit alone: one four-float atomic.
+        for (int l = 0; l < kEncodeLevels; ++l) {
+            const float d0 = d[2 * l], d1 = d[2 * l + 1];
+            if (d0 == 0.0f && d1 == 0.0f) continue;
+            uint32_t index[8];
+            float weight[8];
+            levelCorners(p, firstLevel + l, pos, index, weight);
+            // Corners that differ in x share an aligned pair of entries when their
+            // indices differ in the lowest bit alone: one four-float atomic.
 #pragma unroll
-        for (int c = 0; c < 8; c += 2) {
-            const float2 a = make_float2(weight[c] * d0, weight[c] * d1), b = make_float2(weight[c + 1] * d0, weight[c + 1] * d1);
-            if ((index[c] ^ index[c + 1]) == 1u) {
-                const bool swapped = (index[c] & 1u) != 0u;
-                atomicAdd(reinterpret_cast<float4*>(gridGrad) + (index[c] >> 1),
-                          swapped ? make_float4(b.x, b.y, a.x, a.y) : make_float4(a.x, a.y, b.x, b.y));
-            } else {
-                atomicAdd(reinterpret_cast<float2*>(gridGrad) + index[c], a);
-                atomicAdd(reinterpret_cast<float2*>(gridGrad) + index[c + 1], b);
+            for (int c = 0; c < 8; c += 2) {
+                const float2 a = make_float2(weight[c] * d0, weight[c] * d1), b = make_float2(weight[c + 1] * d0, weight[c + 1] * d1);
+                if ((index[c] ^ index[c + 1]) == 1u) {
+                    const bool swapped = (index[c] & 1u) != 0u;
+                    atomicAdd(reinterpret_cast<float4*>(gridGrad) + (index[c] >> 1),
+                              swapped ? make_float4(b.x, b.y, a.x, a.y) : make_float4(a.x, a.y, b.x, b.y));
+                } else {
+                    atomicAdd(reinterpret_cast<float2*>(gridGrad) + index[c], a);
+                    atomicAdd(reinterpret_cast<float2*>(gridGrad) + index[c + 1], b);
+                }
             }
         }
     }
@@ -762,7 +768,8 @@ void runTrainKernels(Cache* c, const float* queries, const float* targets, uint3
         const int blocks = static_cast<int>(std::min<uint32_t>((n + kTile - 1) / kTile, static_cast<uint32_t>(c->sms)));
         trainKernel<<<blocks, 128, kTrainSmem, stream>>>(c->params(), records, c->features, targets + begin, n,
                                                          1.0f / static_cast<float>(count), c->mlpGrad, c->featureGrad, c->loss, c->error);
-        scatterKernel<<<encodeGrid(n), 256, 0, stream>>>(c->params(), records, c->featureGrad, n, c->gridGrad);
+        const uint32_t wave = static_cast<uint32_t>(c->sms) * kTile;
+        scatterKernel<<<encodeGrid(std::min(n, wave)), 256, 0, stream>>>(c->params(), records, c->featureGrad, n, c->gridGrad);
         NRC_OK(cudaGetLastError());
     }
 }
