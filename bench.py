@@ -269,9 +269,10 @@ def cpu_baseline(wl, target_seconds, rank0=True):
 def traversal_roofline(tracers_and_workloads, peak, peak_kind):
     """Roofline of the closest-hit traversal kernel over untimed renders of
     the given (tracer, workload) pairs: node visits and triangle tests from a
-    counting render, extension rays and extendKernel time from a stage-timed
-    render; algorithmic bytes (32 B ray + 16 B hit + 80 B per wide node + 36 B
-    per triangle) over the kernel's time, against the HBM copy peak."""
+    counting render, extension rays and the kernel's time from a stage-timed
+    render; algorithmic bytes (80 B per wide node + 36 B per triangle;
+    32 B ray + 16 B hit per traversal, which serves up to three rays, so a
+    third of it per ray) over the kernel's time, against the HBM copy peak."""
     from hdcodex_b200.tracer import PROFILE_COUNT_TRAVERSAL, PROFILE_STAGE_TIMES
     total_bytes, total_ms, rays, nodes, tris = 0.0, 0.0, 0, 0, 0
     for t, wl in tracers_and_workloads:
@@ -283,14 +284,14 @@ def traversal_roofline(tracers_and_workloads, peak, peak_kind):
         st = t.stats()
         t.set_profiling(0)
         r = max(c["extension_rays"], 1)
-        per_ray = 32 + 16 + 80 * c["extension_node_visits"] / r + 36 * c["extension_triangle_tests"] / r
+        per_ray = 16 + 80 * c["extension_node_visits"] / r + 36 * c["extension_triangle_tests"] / r
         total_bytes += per_ray * st["extension_rays"]
         total_ms += st["extend_ms"]
         rays += c["extension_rays"]
         nodes += c["extension_node_visits"]
         tris += c["extension_triangle_tests"]
     achieved = total_bytes / (total_ms / 1000.0) / 1e9 if total_ms > 0 else None
-    return {"kernel": "extendKernel (closest-hit traversal)", "bound": "hbm", "achieved": achieved, "peak": peak,
+    return {"kernel": "traceKernel (closest-hit traversal)", "bound": "hbm", "achieved": achieved, "peak": peak,
             "unit": "GB/s", "frac": (achieved / peak) if achieved else None, "peak_source": peak_kind,
             "traffic": None, "nodes_per_ray": nodes / max(rays, 1), "triangles_per_ray": tris / max(rays, 1),
             "jobs_measured": len(tracers_and_workloads)}
@@ -786,12 +787,12 @@ def run_hdcx(args):
     rays_c = max(counted["extension_rays"], 1)
     nodes_per_ray = counted["extension_node_visits"] / rays_c
     tris_per_ray = counted["extension_triangle_tests"] / rays_c
-    bytes_per_ray = 32 + 16 + 80 * nodes_per_ray + 36 * tris_per_ray
+    bytes_per_ray = 16 + 80 * nodes_per_ray + 36 * tris_per_ray
     achieved_gbs = ext_rays * bytes_per_ray / (extend_ms / 1000.0) / 1e9 if extend_ms > 0 else None
     peak, peak_kind = measured_peaks()
     traffic = traffic_from_profile(args.workload)
     roofline = {
-        "kernel": "extendKernel (closest-hit traversal)",
+        "kernel": "traceKernel (closest-hit traversal)",
         "bound": "hbm", "achieved": achieved_gbs, "peak": peak, "unit": "GB/s",
         "frac": (achieved_gbs / peak) if achieved_gbs else None, "peak_source": peak_kind,
         # ncu DRAM bytes per extension ray (profiles/extend_kernel_traffic_heavy.json,

@@ -80,8 +80,8 @@ enum : uint32_t {
     kLaneLightPdf = 6,    // previousEnvironmentLightPdf
 };
 // A scene whose light samples use one slot takes two float4, others three
-// (with slots 1 and 2 in an array of their own, the shade stage of the mesh-light
-// box took 0.78 ms instead of the figure below).
+// (with slots 1 and 2 in an array of their own, the shade stage of a 301x199
+// 8 spp box with a mesh light took 0.80 ms instead of 0.56).
 HDCX_D float* lightRecord(const PathBuffers& p, uint32_t group)
 {
     return reinterpret_cast<float*>(p.laneLight + (p.lightSlots > 1u ? 3u : 2u) * static_cast<size_t>(group));

@@ -47,7 +47,8 @@ __device__ __forceinline__ int stepWalk(const DeviceScene& s, SubsurfaceWalk& w,
     const float scatterDistance = -glog(gmax(1.0f - randomFloat(rng), 1e-6f)) / w.sigmaS;
     const bool forceExit = w.step == kWalkSteps - 1;
     // The boundary's distance counts only up to the scattering event's: beyond
-    // it, that there is a boundary is enough.
+    // it, that there is a boundary is enough (shading stage of a 1280x720 8 spp
+    // scene with subsurface objects: 23.4 -> 22.6 ms).
     if (!traceRay<Accept::Boundary, false, false, kInst>(s, w.origin, w.direction, 0.001f, 10000.0f, 0u, h, fault, nullptr,
                                                         forceExit ? INFINITY : scatterDistance))
         return kWalkFails;

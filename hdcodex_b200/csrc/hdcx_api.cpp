@@ -143,7 +143,7 @@ struct PathStore {
 // ---------------------------------------------------------------------------
 // Path arenas
 //
-// A render needs the path state of its waves (about 359 bytes per path) only
+// A render needs the path state of its waves (about 352 bytes per path) only
 // while it runs, so path state belongs to a per-device pool of arenas rather
 // than to tracers: hdcx_render and hdcx_autotune check an arena out for the
 // call, hdcx_render_batch one per lane until the batch's work has finished.
@@ -837,7 +837,7 @@ void ensureOutput(hdcx_tracer* t, uint32_t w, uint32_t h)
 constexpr uint64_t kAutomaticWavePaths = 12ull << 20;  // ~12.6M paths per wave
 // Device bytes of path state per path (PathBuffers with three shadow slots
 // and the deferred subsurface-walk records).
-constexpr uint64_t kPathStateBytes = 143 + 48 + 8 + 3 * 56;
+constexpr uint64_t kPathStateBytes = 140 + 48 + 8 + 3 * 52;
 
 // Smallest wave an automatic wave is shrunk to when device memory is short.
 constexpr uint64_t kMinimumAutomaticWave = 1ull << 16;

@@ -4,13 +4,17 @@
 // src/gpu/vulkan_path_tracer.cpp:1189-1891): for every sample and each of the
 // three wavelength lanes it loops over bounces, tracing, shading, sampling
 // lights and the BSDF. Here every (pixel, sample, lane) is a path slot of a
-// wave, and each bounce of a wave is four queue-driven kernels:
-//   generate  - camera ray, RNG seed and wavelength of every slot (:1191-1213);
-//   extend    - closest-hit traversal of the extension queue (:1228-1243);
+// wave, the lanes of a sample travel together while they share their path
+// (device/paths.cuh), and each bounce is a few queue-driven kernels:
+//   generate  - camera ray, RNG seed and wavelengths (:1191-1213);
+//   trace     - closest-hit traversal of the extension queue (:1228-1243) and
+//               any-hit visibility of the shadow queue of the bounce before
+//               (:855-912), in one launch unless stages are timed;
 //   shade     - miss/emission/medium/material/NEE/BSDF/roulette (:1245-1879),
 //               appending surviving paths to the next extension queue and
-//               light-sample rays to the shadow queue;
-//   shadow    - any-hit visibility of the shadow queue (:855-912);
+//               light-sample rays to the shadow queue; one launch for entries
+//               of several lanes and, where lanes part, one for single lanes;
+//   walk      - deferred subsurface walks (scenes that have them);
 // and one accumulate kernel per wave adds the lane radiances through the
 // sensor (:1882-1884). A path's radiance gets its contributions in the
 // megakernel's order: light-sample contributions of bounce b are stored per
@@ -314,10 +318,11 @@ __global__ void __launch_bounds__(128, HDCX_TRACE_MIN_BLOCKS)
 // accumulate: sensor and per-pixel batch sums (vulkan_path_tracer.cpp:1882-1884)
 // ---------------------------------------------------------------------------
 //
-// A pixel's samples add up in order, but what each adds (fourteen exponentials
-// per sample) does not depend on the others: a thread per sample computes it,
-// then a thread per pixel adds the block's values (thread-per-pixel alone took
-// 1.48 ms for eight samples at 1920x1080).
+// A pixel's samples add up in order, but what each adds (seven exponentials per
+// wavelength) does not depend on the others: a thread per sample computes it,
+// then a thread per pixel adds the block's values. Bound by instruction issue:
+// eight samples at 1920x1080 took 1.6 ms with the sensor's RGB and XYZ each
+// evaluating the exponentials and these branching, 0.69 ms with neither.
 constexpr uint32_t kAccumulateThreads = 256;
 
 // What sample `group` adds: sensor RGB (a third of the lanes' sum) and XYZ.
@@ -751,7 +756,7 @@ void renderFrame(const DeviceScene& sceneIn, const FrameConst& frame, PathBuffer
     const std::vector<WaveDesc> waves = planWaves(pixels, std::max(frame.sampleCount, 1u), wavePaths);
     const int traceGrid = gridFor(static_cast<uint32_t>(wavePaths), static_cast<int>(std::max(paths.traceBlocksPerSm, 1u)));
     const int shadeGrid = gridFor(static_cast<uint32_t>(wavePaths), static_cast<int>(std::max(paths.shadeBlocksPerSm, 1u)));
-    const int missGrid = gridFor(static_cast<uint32_t>(wavePaths), 8);
+    const int replayGrid = gridFor(static_cast<uint32_t>(wavePaths), 8);
     const bool sortHits = paths.sortHits != 0u && paths.sortedHits != nullptr && paths.hitBins != nullptr;
     const bool sortRays = paths.sortRays != 0u;
     // Subsurface walks in walkKernel (scenes that can take them).
@@ -842,7 +847,7 @@ void renderFrame(const DeviceScene& sceneIn, const FrameConst& frame, PathBuffer
                     launch.queue = paths.hitQueue;
                     launch.count = counters + kCountReplays;
                     launch.misses = false;
-                    launch.grid = missGrid;
+                    launch.grid = replayGrid;
                     launchShadeReplays(variant, launch);
                     launched += 2;
                 }

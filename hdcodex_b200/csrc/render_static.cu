@@ -14,7 +14,7 @@
 // kStaticMaxPixels pixels; waves of kStaticWavePaths paths (a frame needs more
 // waves than the ordinary render, whose waves hold up to ~12.6M paths, so this
 // variant is slower on large frames). Every GPU that loads the library keeps
-// the array, kStaticScratchBytes (about 62 MB), until the process exits.
+// the array, kStaticScratchBytes (about 61 MB), until the process exits.
 //
 // The array's device address is looked up once per device with
 // cudaGetSymbolAddress, by the first call on that device (with that device

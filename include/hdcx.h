@@ -323,10 +323,13 @@ typedef struct hdcx_render_stats {
     uint32_t waves;                  /* path waves the render was split into */
     uint32_t extend_launches;        /* closest-hit traversal launches */
     uint64_t kernel_launches;        /* kernels the render launched */
-    uint64_t extension_node_visits;  /* wide nodes loaded by closest-hit rays (counting mode) */
-    uint64_t extension_triangle_tests; /* triangle tests of closest-hit rays (counting mode) */
-    uint64_t shadow_node_visits;     /* wide nodes loaded by shadow rays (counting mode) */
-    uint64_t shadow_triangle_tests;  /* triangle tests of shadow rays (counting mode) */
+    /* Counting mode. A sample's wavelength lanes share a traversal while they
+     * share their path: rays are counted per lane, visits and tests per
+     * traversal. */
+    uint64_t extension_node_visits;    /* wide nodes loaded by closest-hit traversals */
+    uint64_t extension_triangle_tests; /* triangle tests of closest-hit traversals */
+    uint64_t shadow_node_visits;       /* wide nodes loaded by shadow traversals */
+    uint64_t shadow_triangle_tests;    /* triangle tests of shadow traversals */
 } hdcx_render_stats;
 
 /* One job of hdcx_render_batch: the arguments of one hdcx_render call and
@@ -504,7 +507,7 @@ HDCX_API int32_t hdcx_get_shading_mode(const hdcx_tracer* tracer);
  * RGBA32F image (width*height*4 floats, row 0 = bottom) is copied into it.
  * With no geometry or a zero size nothing is traced and *written = 0
  * (the reference returns an empty vector, :3235); otherwise *written = 1.
- * Device memory: the path state of a wave (about 359 bytes per path) lives in
+ * Device memory: the path state of a wave (about 352 bytes per path) lives in
  * a per-device pool of arenas, not in the tracer: a call checks out a free
  * arena (at most eight per device; when all are busy it waits for one) and
  * grows it to its wave, and the arenas are freed with the device's last
@@ -691,7 +694,7 @@ HDCX_API hdcx_status hdcx_set_tuning(hdcx_tracer* tracer, const hdcx_tuning* tun
  * size, bounce budget and sample count over wave sizes and traversal/shade
  * grid sizes and the hit sort, one knob at a time from the defaults, keeps the fastest on the
  * tracer and returns it. Wave sizes of 1M to 48M paths are tried, the larger
- * ones while their path state (about 359 bytes per path) fits half of the free
+ * ones while their path state (about 352 bytes per path) fits half of the free
  * device memory; a path arena grown for a candidate larger than the one kept
  * is released before it returns. Results are cached per device and workload shape
  * (triangles, pixels, samples, bounces, shading variant) for the process, so
