@@ -63,7 +63,7 @@ HDCX_D V combineShadow(uint32_t kind, V a, V sv, V g1, V g2, V g3)
 // slot j.
 HDCX_D void emitShadow(PathBuffers& p, uint32_t group, uint32_t lanes, uint32_t info, float3 origin, float3 direction, float tmax)
 {
-    const uint32_t i = appendEntry(reinterpret_cast<unsigned long long*>(p.counters + p.shadowWord), lanes);
+    const uint32_t i = appendEntry(reinterpret_cast<unsigned long long*>(p.counters + kCountShadow), lanes);
     p.shadowRay[2u * i] = make_float4(origin.x, origin.y, origin.z, tmax);
     p.shadowRay[2u * i + 1u] = make_float4(direction.x, direction.y, direction.z, __uint_as_float((group << 3) | lanes));
     p.shadowInfo[i] = info;

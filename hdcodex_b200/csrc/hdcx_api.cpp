@@ -916,6 +916,7 @@ FrameConst makeFrame(const hdcx_tracer* t, const hdcx_camera& c, uint32_t w, uin
     f.height = h;
     f.sampleIndex = sampleIndex;
     f.sampleCount = std::max(sampleCount, 1u);
+    static_assert(HDCX_MAX_PATH_BOUNCES <= kMaxBounces, "every bounce has a set of queue counters");
     f.maxBounces = std::clamp(maxBounces, 1u, HDCX_MAX_PATH_BOUNCES);
     f.zUp = t->fallbackZUp ? 1u : 0u;
     if (t->textureLod) {

@@ -80,7 +80,7 @@ __global__ void generateKernel(FrameConst f, WaveDesc w, PathBuffers p)
     const uint32_t groups = w.count / 3u;
     if (group == 0) {
         const unsigned long long lanes = static_cast<unsigned long long>(w.count) << 32;
-        *reinterpret_cast<unsigned long long*>(p.counters + kCountQueue0) = lanes | (p.split ? w.count : groups);
+        *reinterpret_cast<unsigned long long*>(p.counters + kCountQueue) = lanes | (p.split ? w.count : groups);
     }
     if (group >= groups) return;
     const uint32_t pixel = tiledPixel(f, w.pixelBase + group / w.samples);
@@ -315,7 +315,8 @@ __global__ void __launch_bounds__(128, HDCX_TRACE_MIN_BLOCKS)
 }
 
 // ---------------------------------------------------------------------------
-// accumulate: sensor and per-pixel batch sums (vulkan_path_tracer.cpp:1882-1884)
+// accumulate: sensor and per-pixel batch sums (vulkan_path_tracer.cpp:1882-1884),
+// and the running mean once a pixel's last wave has been added
 // ---------------------------------------------------------------------------
 //
 // A pixel's samples add up in order, but what each adds (seven exponentials per
@@ -355,7 +356,7 @@ HDCX_D void sampleValue(const PathBuffers& p, uint32_t group, float3& rgb, doubl
     xyz[2] = __ddiv_rn(sz, 3.0);
 }
 
-__global__ void __launch_bounds__(kAccumulateThreads) accumulateKernel(FrameConst f, WaveDesc w, PathBuffers p, float4* batch, double* batchXyz)
+__global__ void __launch_bounds__(kAccumulateThreads) accumulateKernel(FrameConst f, WaveDesc w, PathBuffers p, FrameBuffers fb)
 {
     __shared__ float3 rgbs[kAccumulateThreads];
     __shared__ double xyzs[3][kAccumulateThreads];
@@ -369,9 +370,9 @@ __global__ void __launch_bounds__(kAccumulateThreads) accumulateKernel(FrameCons
     const uint32_t pixel = adds ? tiledPixel(f, w.pixelBase + local) : 0u;
     float4 b = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     double bx = 0.0, by = 0.0, bz = 0.0;
-    if (adds) {
-        b = batch[pixel];
-        bx = batchXyz[3 * pixel + 0], by = batchXyz[3 * pixel + 1], bz = batchXyz[3 * pixel + 2];
+    if (adds && w.sampleBase != 0u) {
+        b = fb.batch[pixel];
+        bx = fb.batchXyz[3 * pixel + 0], by = fb.batchXyz[3 * pixel + 1], bz = fb.batchXyz[3 * pixel + 2];
     }
     for (uint32_t base = 0; base < w.samples; base += step) {
         const uint32_t mine = threadIdx.x / step, sample = base + threadIdx.x % step;
@@ -394,31 +395,30 @@ __global__ void __launch_bounds__(kAccumulateThreads) accumulateKernel(FrameCons
         __syncthreads();
     }
     if (!adds) return;
-    batch[pixel] = b;
-    batchXyz[3 * pixel + 0] = bx;
-    batchXyz[3 * pixel + 1] = by;
-    batchXyz[3 * pixel + 2] = bz;
-}
-
-// pixels[index] = vec4((previous * previousWeight + batchRadiance) / totalWeight, 1.0)
-// (vulkan_path_tracer.cpp:1886-1890); the FP64 XYZ sums add the batch.
-__global__ void finalizeKernel(FrameConst f, FrameBuffers fb)
-{
-    const uint32_t pixel = blockIdx.x * blockDim.x + threadIdx.x;
-    if (pixel >= f.width * f.height) return;
-    // A restart (sampleIndex 0) gives the previous mean weight 0; it is not
-    // read, so whatever the output buffer held (NaN included) cannot leak in.
+    if (w.sampleBase + w.samples < f.sampleCount) {
+        fb.batch[pixel] = b;
+        fb.batchXyz[3 * pixel + 0] = bx;
+        fb.batchXyz[3 * pixel + 1] = by;
+        fb.batchXyz[3 * pixel + 2] = bz;
+        return;
+    }
+    // The pixel's last wave: pixels[index] = vec4((previous * previousWeight +
+    // batchRadiance) / totalWeight, 1.0) (vulkan_path_tracer.cpp:1886-1890); the
+    // FP64 XYZ sums add the batch. A restart (sampleIndex 0) gives the previous
+    // mean weight 0; it is not read, so whatever the output buffer held (NaN
+    // included) cannot leak in.
     const float4 prev = f.sampleIndex == 0 ? make_float4(0.0f, 0.0f, 0.0f, 0.0f) : fb.rgba[pixel];
-    const float4 b = fb.batch[pixel];
     const float previousWeight = u2f(f.sampleIndex);
     const float totalWeight = previousWeight + u2f(f.sampleCount);
     fb.rgba[pixel] = make_float4((prev.x * previousWeight + b.x) / totalWeight, (prev.y * previousWeight + b.y) / totalWeight,
                                  (prev.z * previousWeight + b.z) / totalWeight, 1.0f);
+    const double sums[3] = {bx, by, bz};
     for (int k = 0; k < 3; ++k) {
         const double base = f.sampleIndex == 0 ? 0.0 : fb.xyz[3 * pixel + k];
-        fb.xyz[3 * pixel + k] = __dadd_rn(base, fb.batchXyz[3 * pixel + k]);
+        fb.xyz[3 * pixel + k] = __dadd_rn(base, sums[k]);
     }
 }
+
 
 __global__ void primaryKernel(DeviceScene s, FrameConst f, uint32_t sampleNumber, uint32_t* primitives, float* distances)
 {
@@ -750,8 +750,6 @@ void renderFrame(const DeviceScene& sceneIn, const FrameConst& frame, PathBuffer
     if (!cacheMode) paths.cache.enabled = 0u;
     uint64_t launched = 0;
     const uint32_t pixels = frame.width * frame.height;
-    CUDA_OK(cudaMemsetAsync(fb.batch, 0, sizeof(float4) * pixels, stream));
-    CUDA_OK(cudaMemsetAsync(fb.batchXyz, 0, sizeof(double) * 3u * pixels, stream));
     const uint64_t wavePaths = paths.wavePaths ? std::min(paths.wavePaths, paths.capacity) : paths.capacity;
     const std::vector<WaveDesc> waves = planWaves(pixels, std::max(frame.sampleCount, 1u), wavePaths);
     const int traceGrid = gridFor(static_cast<uint32_t>(wavePaths), static_cast<int>(std::max(paths.traceBlocksPerSm, 1u)));
@@ -789,8 +787,8 @@ void renderFrame(const DeviceScene& sceneIn, const FrameConst& frame, PathBuffer
     // Stage times and traversal counts are those of separate launches.
     const bool fused = timing == nullptr && !countTraversal;
     const ShadeVariant variant{scene.fullShading != 0u, lit, cacheMode, deferWalks(paths)};
-    uint32_t* counters = paths.counters;
-    auto counter64 = [&](uint32_t word) { return reinterpret_cast<unsigned long long*>(counters + word); };
+    uint32_t* const allCounters = paths.counters;
+    auto counter64 = [](uint32_t* set, uint32_t word) { return reinterpret_cast<unsigned long long*>(set + word); };
     // Material order of a hit queue (tuning sort_hits).
     auto sortedByMaterial = [&](const uint32_t* hits, const uint32_t* count) {
         if (!sortHits) return hits;
@@ -804,18 +802,19 @@ void renderFrame(const DeviceScene& sceneIn, const FrameConst& frame, PathBuffer
     for (const WaveDesc& w : waves) {
         NvtxRange waveRange("hdcx wave");
         if (cacheMode) CUDA_OK(cudaMemsetAsync(paths.cache.counters, 0, 3 * sizeof(uint32_t), stream));
+        // (A clear before every bounce was a launch in each: 2 us of its latency.)
+        paths.counters = allCounters;
+        CUDA_OK(cudaMemsetAsync(allCounters, 0, kCountEnd * sizeof(uint32_t), stream));
         generateKernel<<<(w.count / 3u + 127u) / 128u, 128, 0, stream>>>(frame, w, paths);
         CUDA_OK(cudaGetLastError());
         for (uint32_t bounce = 0; bounce < frame.maxBounces; ++bounce) {
             uint32_t* inQueue = paths.queue[bounce & 1u];
             uint32_t* outQueue = paths.queue[(bounce + 1u) & 1u];
-            const bool odd = (bounce & 1u) != 0u;
-            unsigned long long* inCount = counter64(odd ? kCountQueue1 : kCountQueue0);
-            unsigned long long* outCount = counter64(odd ? kCountQueue0 : kCountQueue1);
-            const unsigned long long* previousShadows = bounce > 0u ? counter64(odd ? kCountShadow0 : kCountShadow1) : nullptr;
-            paths.shadowWord = odd ? kCountShadow1 : kCountShadow0;
-            const uint32_t clearFrom = odd ? 0u : kCountHits, clearTo = odd ? kCountShadow0 : kCountEnd;
-            CUDA_OK(cudaMemsetAsync(counters + clearFrom, 0, (clearTo - clearFrom) * sizeof(uint32_t), stream));
+            uint32_t* counters = allCounters + bounce * kCountWords;
+            paths.counters = counters;
+            unsigned long long* inCount = counter64(counters, kCountQueue);
+            unsigned long long* outCount = counter64(counters + kCountWords, kCountQueue);
+            const unsigned long long* previousShadows = bounce > 0u ? counter64(counters - kCountWords, kCountShadow) : nullptr;
             if (sortRays && bounce > 0u) {
                 sortRaysKernel<<<sortGrid, 256, 0, stream>>>(paths, inQueue, inCount);
                 launched += 1;
@@ -856,7 +855,7 @@ void renderFrame(const DeviceScene& sceneIn, const FrameConst& frame, PathBuffer
             launched += 1;
             if (!fused || bounce + 1u == frame.maxBounces) {
                 timed(2, [&] {
-                    launchTrace(scene, paths, TraceWork{nullptr, nullptr, counter64(paths.shadowWord)}, countTraversal, traceGrid, stream);
+                    launchTrace(scene, paths, TraceWork{nullptr, nullptr, counter64(counters, kCountShadow)}, countTraversal, traceGrid, stream);
                 });
                 launched += 1;
             }
@@ -883,12 +882,9 @@ void renderFrame(const DeviceScene& sceneIn, const FrameConst& frame, PathBuffer
         }
         launched += 2;
         const uint32_t blockPixels = kAccumulateThreads / std::min(w.samples, kAccumulateThreads);
-        accumulateKernel<<<(w.pixels + blockPixels - 1u) / blockPixels, kAccumulateThreads, 0, stream>>>(frame, w, paths, fb.batch, fb.batchXyz);
+        accumulateKernel<<<(w.pixels + blockPixels - 1u) / blockPixels, kAccumulateThreads, 0, stream>>>(frame, w, paths, fb);
         CUDA_OK(cudaGetLastError());
     }
-    finalizeKernel<<<(pixels + 255u) / 256u, 256, 0, stream>>>(frame, fb);
-    CUDA_OK(cudaGetLastError());
-    launched += 1;
     if (launches) *launches = launched;
     if (timing) {
         CUDA_OK(cudaStreamSynchronize(stream));

@@ -39,25 +39,23 @@ struct CacheDevice {
 // Material bins of the hit sort (material index modulo kHitBins).
 constexpr uint32_t kHitBins = 256;
 
-// Queue counters of a wave (32-bit words of PathBuffers::counters). The
-// extension and shadow queues count entries in a 64-bit counter's low half
-// and lanes in its high half. A bounce reads its extension queue and the
-// shadow queue of the bounce before it and fills the others, which one clear
-// covers: words kCountHits to the end in even bounces (they read kCountQueue0
-// and kCountShadow1), words 0 to kCountShadow0 in odd ones.
+// Queue counters (32-bit words of PathBuffers::counters). The extension and
+// shadow queues count entries in a 64-bit counter's low half and lanes in its
+// high half. Every bounce has a set of its own, and its surviving paths are
+// counted in the next one's, so that one clear serves a whole wave.
 enum : uint32_t {
-    kCountQueue0 = 0,    // 64-bit: extension queue of even bounces
-    kCountShadow1 = 2,   // 64-bit: shadow queue of odd bounces
+    kCountQueue = 0,     // 64-bit: extension queue
+    kCountShadow = 2,    // 64-bit: shadow queue
     kCountHits = 4,      // entries of hitQueue
     kCountGroups = 5,    // entries of groupQueue
     kCountMisses = 6,
     kCountWalks = 7,     // deferred subsurface walks
     kCountReplays = 8,   // failed walks to re-shade
     kCountWalkNext = 9,  // walks taken by walkKernel's threads
-    kCountShadow0 = 10,  // 64-bit: shadow queue of even bounces
-    kCountQueue1 = 12,   // 64-bit: extension queue of odd bounces
-    kCountEnd = 14,
+    kCountWords = 10,    // of one set
 };
+constexpr uint32_t kMaxBounces = 12;
+constexpr uint32_t kCountEnd = (kMaxBounces + 1u) * kCountWords;
 
 // Device buffers of one wave of paths (structure of arrays; slot 3 g + lane,
 // see device/paths.cuh for groups and leaders).
@@ -68,7 +66,6 @@ struct PathBuffers {
     uint32_t lightSlots = 3;        // light-sample slots in use: 1 (analytic), 2 (+ mesh lights) or 3 (fallback sun and sky)
     uint32_t split = 0;             // 1: every lane travels as an entry of its own from the start
     uint32_t merged = 0;            // 1: hitQueue takes every entry, groupQueue none
-    uint32_t shadowWord = 0;        // counter of the bounce's shadow queue
     float4* laneLight = nullptr;    // two (lightSlots = 1) or three per group: kLaneRadiance, kLaneLight of its lanes (device/paths.cuh)
     float4* laneState = nullptr;    // three per group: kLaneThroughput, kLaneBsdfPdf, kLaneLightPdf of its lanes
     float4* laneSpectrum = nullptr; // four per group: basis r, g, b and Planck factor of each lane, their wavelengths
@@ -82,7 +79,7 @@ struct PathBuffers {
     float4* shadowRay = nullptr;        // two per shadow ray: origin and tmax, direction and entry
     float4* shadowFactors = nullptr;    // per path slot and light-sample slot (kShadowGeneral): partial product, f1, f2, f3
     uint32_t* shadowInfo = nullptr;     // kind, light-sample slot, light (device/paths.cuh)
-    uint32_t* counters = nullptr;       // kCountEnd words
+    uint32_t* counters = nullptr;       // kCountEnd words (in a launch: the set of its bounce)
     // extension, shadow, subsurface rays; extension node visits and triangle
     // tests; shadow node visits and triangle tests (counting mode)
     unsigned long long* stats = nullptr;

@@ -143,13 +143,13 @@ unsigned int renderStatic(const DeviceScene& scene, const FrameConst& frame, flo
     fb.batch = reinterpret_cast<float4*>(region[16]);
     fb.batchXyz = reinterpret_cast<double*>(region[17]);
     // The frame's FP64 XYZ running sums are not kept by this variant: the
-    // finalize pass adds them into the batch sums of the same pixel (each
-    // thread reads and writes only its own pixel), which the next call clears.
+    // accumulation adds them into the batch sums of the same pixel (each
+    // thread reads and writes only its own pixel), which the next call's first
+    // wave of the pixel overwrites.
     fb.xyz = fb.batchXyz;
 
-    // The array keeps the previous call's contents: the queue counters and
-    // ray statistics must start at zero (renderFrame clears the batch sums).
-    ok(cudaMemsetAsync(p.counters, 0, kCountEnd * sizeof(uint32_t), stream), "clear counters");
+    // The array keeps the previous call's contents: the ray statistics must
+    // start at zero (renderFrame clears the queue counters).
     ok(cudaMemsetAsync(p.stats, 0, 8 * sizeof(unsigned long long), stream), "clear stats");
     renderFrame(scene, frame, p, fb, stream, nullptr, false, nullptr);
     // The lock covers the GPU work too: the next call may reuse the array.
