@@ -6,8 +6,9 @@
 // state) travel as one queue entry: (g << 3) | lane mask. What they share (ray,
 // random state, flags, hit, ray cone) is kept at the slot of the entry's first
 // lane, its leader; what depends on the wavelength (throughput, radiance,
-// previous pdfs, medium, light samples) at each lane's own slot. Where lanes
-// part, the entry becomes several, each with its own leader.
+// previous pdfs, light samples, spectrum) in records of the group, the medium
+// at each lane's own slot. Where lanes part, the entry becomes several, each
+// with its own leader.
 #pragma once
 
 #include "../integrator.h"
