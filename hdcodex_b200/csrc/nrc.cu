@@ -238,6 +238,31 @@ __global__ void __launch_bounds__(256) encodeKernel(DeviceParams p, const float*
     *reinterpret_cast<uint4*>(features + static_cast<size_t>(q) * kGridFeatures + 2 * firstLevel) = *reinterpret_cast<const uint4*>(out);
 }
 
+// The 64 network inputs of query record q (zeros for a missing query).
+__device__ void encodeQuery(const DeviceParams& p, const float* q, float in[kWidth])
+{
+#pragma unroll
+    for (int i = 0; i < kWidth; ++i) in[i] = 0.0f;
+    if (!q) return;
+    const float3 pos = make_float3(q[0], q[1], q[2]);
+    for (int level = 0; level < kLevels; ++level) {
+        uint32_t index[8];
+        float weight[8];
+        levelCorners(p, level, pos, index, weight);
+        float f0 = 0.0f, f1 = 0.0f;
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+            const float2 v = __half22float2(p.grid[index[c]]);
+            f0 = fmaf(weight[c], v.x, f0);
+            f1 = fmaf(weight[c], v.y, f1);
+        }
+        in[2 * level] = f0;
+        in[2 * level + 1] = f1;
+    }
+#pragma unroll
+    for (int i = 0; i < 9; ++i) in[32 + i] = q[3 + i];
+}
+
 // Writes 64 values of row `row` as BF16 into a tile with `colGroups` column groups.
 __device__ __forceinline__ void storeRow(__nv_bfloat16* tile, uint32_t row, const float* v, uint32_t colGroups, int count)
 {
@@ -388,13 +413,20 @@ __global__ void __launch_bounds__(kQueryThreads, 2) queryKernel(DeviceParams p, 
 
 // Forward and backward of every tile of 128 training records; weight
 // gradients accumulate in tensor memory and are added to `mlpGrad` at the
-// end; the gradients of the encoded features go to `featureGrad`, one row of
-// kGridFeatures per record, from which scatterKernel adds them to the table.
+// end; hash-grid gradients are scattered with atomics into `gridGrad`.
+//
+// Records are encoded and scattered here, tile by tile, and not in kernels of
+// their own: the barriers of a tile order a block's additions (a tile's before
+// those of the block's next), and with them the FP32 rounding of an entry's
+// sum. Adam divides by the gradient's own size, so a parameter whose gradient
+// nearly cancels moves by up to a learning rate with that rounding. With the
+// scatter in a kernel whose warps run on freely, four steps of 2^16 records
+// gave single parameters a third of a learning rate away (1.4e-5 of the table
+// in relative L2, where this order repeats itself to 2.5e-7).
 constexpr uint32_t kTrainSmem = kWeightCount * 2u + 5u * kTile * kWidth * 2u + kTile * 128u * 2u + 16u;
 
-__global__ void __launch_bounds__(128) trainKernel(DeviceParams p, const float* queries, const __nv_bfloat16* features,
-                                                   const float* targets, uint32_t count, float gradientScale, float* mlpGrad,
-                                                   float* featureGrad, float* lossSum,
+__global__ void __launch_bounds__(128) trainKernel(DeviceParams p, const float* queries, const float* targets, uint32_t count,
+                                                   float gradientScale, float* mlpGrad, float* gridGrad, float* lossSum,
                                                    uint32_t* error)
 {
     extern __shared__ __align__(16) uint8_t smem[];
@@ -425,7 +457,8 @@ __global__ void __launch_bounds__(128) trainKernel(DeviceParams p, const float* 
         const bool valid = q < count;
         const float* record = valid ? queries + static_cast<size_t>(q) * kQueryFloats : nullptr;
         float v[kWidth];
-        storeInputRow(xs, row, features + static_cast<size_t>(q) * kGridFeatures, record);
+        encodeQuery(p, record, v);
+        storeRow(xs, row, v, 8u, kWidth);
         float prediction = 0.0f;
         // Forward, keeping X_0 .. X_4.
         for (int layer = 0; layer < kLayers && !failed; ++layer) {
@@ -513,10 +546,20 @@ __global__ void __launch_bounds__(128) trainKernel(DeviceParams p, const float* 
                 }
                 storeRow(g, row, v, 16u, kWidth);
             } else if (valid) {
-                // Gradients of the encoded features: input columns 0..31.
-                float4* dst = reinterpret_cast<float4*>(featureGrad + static_cast<size_t>(q) * kGridFeatures);
+                // Hash-grid gradients: input columns 0..31.
+                const float3 pos = make_float3(record[0], record[1], record[2]);
+                for (int level = 0; level < kLevels; ++level) {
+                    uint32_t index[8];
+                    float weight[8];
+                    levelCorners(p, level, pos, index, weight);
+                    const float d0 = v[2 * level], d1 = v[2 * level + 1];
+                    if (d0 == 0.0f && d1 == 0.0f) continue;
 #pragma unroll
-                for (int c = 0; c < static_cast<int>(kGridFeatures); c += 4) dst[c / 4] = make_float4(v[c], v[c + 1], v[c + 2], v[c + 3]);
+                    for (int c = 0; c < 8; ++c) {
+                        atomicAdd(gridGrad + 2u * index[c], weight[c] * d0);
+                        atomicAdd(gridGrad + 2u * index[c] + 1u, weight[c] * d1);
+                    }
+                }
             }
             fenceBeforeSync();
         }
@@ -539,9 +582,7 @@ __global__ void __launch_bounds__(128) trainKernel(DeviceParams p, const float* 
             for (int c = 0; c < kWidth; c += 16) tmemLoad16(tmem + laneOffset + 64u + 64u * layer + static_cast<uint32_t>(c), d + c);
             if (r < static_cast<uint32_t>(layerRows(layer))) {
                 float* dst = mlpGrad + layerOffset(layer) + r * kWidth;
-#pragma unroll
-                for (int c = 0; c < kWidth; c += 4)
-                    atomicAdd(reinterpret_cast<float4*>(dst + c), make_float4(d[c], d[c + 1], d[c + 2], d[c + 3]));
+                for (int c = 0; c < kWidth; ++c) atomicAdd(dst + c, d[c]);
             }
         }
     }
@@ -550,56 +591,6 @@ __global__ void __launch_bounds__(128) trainKernel(DeviceParams p, const float* 
     __syncthreads();
     fenceAfterSync();
     if (warp == 0) tmemFree(tmem, 512u);
-}
-
-// Hash-grid gradients: every feature gradient times its corner's weight, added
-// to the table's FP32 gradients. One thread per record and kEncodeLevels
-// levels, a two-float vector atomic per corner. (Inside trainKernel, with one
-// block of four warps per SM, the scatter waited on its own latency: 228 us a
-// step of 2^16 records for the whole kernel.) Records are taken in waves of a
-// tile per SM, as trainKernel takes them: an entry's sum forms nearly in the
-// order of the records, and runs differ no more than that. With all records of
-// a call in flight the same sums came out in any order, and single parameters
-// whose gradients nearly cancel moved by a learning rate three times as often
-// (four steps of 2^16 records: 569 us in any order, 579 us in waves).
-__global__ void __launch_bounds__(256) scatterKernel(DeviceParams p, const float* queries, const float* featureGrad, uint32_t count,
-                                                     float* gridGrad)
-{
-    for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < count; q += gridDim.x * blockDim.x) {
-        // Scalar loads: callers' records need no more than float alignment.
-        const float* record = queries + static_cast<size_t>(q) * kQueryFloats;
-        const float3 pos = make_float3(__ldg(record), __ldg(record + 1), __ldg(record + 2));
-        const int firstLevel = static_cast<int>(blockIdx.y) * kEncodeLevels;
-        const float4* row = reinterpret_cast<const float4*>(featureGrad + static_cast<size_t>(q) * kGridFeatures + 2 * firstLevel);
-        float d[2 * kEncodeLevels];
-#pragma unroll
-        for (int i = 0; i < kEncodeLevels / 2; ++i) {
-            const float4 v = __ldg(row + i);
-            d[4 * i] = v.x, d[4 * i + 1] = v.y, d[4 * i + 2] = v.z, d[4 * i + 3] = v.w;
-        }
-#pragma unroll
-        for (int l = 0; l < kEncodeLevels; ++l) {
-            const float d0 = d[2 * l], d1 = d[2 * l + 1];
-            if (d0 == 0.0f && d1 == 0.0f) continue;
-            uint32_t index[8];
-            float weight[8];
-            levelCorners(p, firstLevel + l, pos, index, weight);
-            // Corners that differ in x share an aligned pair of entries when their
-            // indices differ in the lowest bit alone: one four-float atomic.
-#pragma unroll
-            for (int c = 0; c < 8; c += 2) {
-                const float2 a = make_float2(weight[c] * d0, weight[c] * d1), b = make_float2(weight[c + 1] * d0, weight[c + 1] * d1);
-                if ((index[c] ^ index[c + 1]) == 1u) {
-                    const bool swapped = (index[c] & 1u) != 0u;
-                    atomicAdd(reinterpret_cast<float4*>(gridGrad) + (index[c] >> 1),
-                              swapped ? make_float4(b.x, b.y, a.x, a.y) : make_float4(a.x, a.y, b.x, b.y));
-                } else {
-                    atomicAdd(reinterpret_cast<float2*>(gridGrad) + index[c], a);
-                    atomicAdd(reinterpret_cast<float2*>(gridGrad) + index[c + 1], b);
-                }
-            }
-        }
-    }
 }
 
 // The kernels' bounded wait on an mbarrier that nothing arrives at: the wait
@@ -714,13 +705,11 @@ struct Cache {
     __half* gridHalf = nullptr;
     float* loss = nullptr;      // the loss sum, and after it the error word: one copy reads both
     uint32_t* error = nullptr;  // loss + 1
-    // Encoded features and their gradients of one chunk of records. Calls on
-    // one cache share them: each holds `work` until its kernels have finished.
+    // Encoded features of one chunk of records. Queries on one cache share
+    // them: each holds `work` until its kernels have finished.
     std::mutex work;
     __nv_bfloat16* features = nullptr;
-    float* featureGrad = nullptr;
     uint32_t chunk = 0;         // records `features` holds
-    uint32_t trainChunk = 0;    // records `featureGrad` holds
     uint64_t step = 0;
     int sms = 148;
 
@@ -758,20 +747,12 @@ void finish(Cache* c, cudaStream_t stream, float* loss = nullptr)
 
 dim3 encodeGrid(uint32_t count) { return dim3((count + 255u) / 256u, kLevels / kEncodeLevels); }
 
-// Forward and backward of all records, chunk by chunk; gradients and loss add up.
-void runTrainKernels(Cache* c, const float* queries, const float* targets, uint32_t count, cudaStream_t stream)
+void runTrainKernel(Cache* c, const float* queries, const float* targets, uint32_t count, cudaStream_t stream)
 {
-    for (uint32_t begin = 0; begin < count; begin += c->trainChunk) {
-        const uint32_t n = std::min(c->trainChunk, count - begin);
-        const float* records = queries + static_cast<size_t>(begin) * kQueryFloats;
-        encodeKernel<<<encodeGrid(n), 256, 0, stream>>>(c->params(), records, n, c->features);
-        const int blocks = static_cast<int>(std::min<uint32_t>((n + kTile - 1) / kTile, static_cast<uint32_t>(c->sms)));
-        trainKernel<<<blocks, 128, kTrainSmem, stream>>>(c->params(), records, c->features, targets + begin, n,
-                                                         1.0f / static_cast<float>(count), c->mlpGrad, c->featureGrad, c->loss, c->error);
-        const uint32_t wave = static_cast<uint32_t>(c->sms) * kTile;
-        scatterKernel<<<encodeGrid(std::min(n, wave)), 256, 0, stream>>>(c->params(), records, c->featureGrad, n, c->gridGrad);
-        NRC_OK(cudaGetLastError());
-    }
+    const int blocks = static_cast<int>(std::min<uint32_t>((count + kTile - 1) / kTile, static_cast<uint32_t>(c->sms)));
+    trainKernel<<<blocks, 128, kTrainSmem, stream>>>(c->params(), queries, targets, count, 1.0f / static_cast<float>(count),
+                                                     c->mlpGrad, c->gridGrad, c->loss, c->error);
+    NRC_OK(cudaGetLastError());
 }
 
 }  // namespace
@@ -808,16 +789,12 @@ Cache* create(int device, const Config& config)
     c->error = reinterpret_cast<uint32_t*>(c->loss + 1);
     // Chunks of 2^20 records to encode (64 MB of features, which stay in L2
     // between the kernels; chunks of 2^18 cost 0.14 ms of launch gaps in a
-    // query of 10^6) and of 2^18 to train on (32 MB), fewer where memory is short.
+    // query of 10^6), fewer where memory is short.
     for (c->chunk = 1u << 20;; c->chunk >>= 1) {
-        c->trainChunk = std::min(c->chunk, 1u << 18);
         try {
             c->features = deviceAlloc<__nv_bfloat16>(static_cast<size_t>(c->chunk) * kGridFeatures);
-            c->featureGrad = deviceAlloc<float>(static_cast<size_t>(c->trainChunk) * kGridFeatures);
             break;
         } catch (const std::exception&) {
-            deviceFree(c->features);
-            c->features = nullptr;
             if (c->chunk <= kTile) throw;
         }
     }
@@ -847,8 +824,7 @@ void destroy(Cache* c)
     for (void* p : {static_cast<void*>(c->mlp), static_cast<void*>(c->mlpGrad), static_cast<void*>(c->mlpM),
                     static_cast<void*>(c->mlpV), static_cast<void*>(c->mlpTiled), static_cast<void*>(c->grid),
                     static_cast<void*>(c->gridGrad), static_cast<void*>(c->gridM), static_cast<void*>(c->gridV),
-                    static_cast<void*>(c->gridHalf), static_cast<void*>(c->loss), static_cast<void*>(c->features),
-                    static_cast<void*>(c->featureGrad)})
+                    static_cast<void*>(c->gridHalf), static_cast<void*>(c->loss), static_cast<void*>(c->features)})
         deviceFree(p);
     delete c;
 }
@@ -882,7 +858,6 @@ void getParameters(Cache* c, float* mlp, float* grid)
 
 void checkWaitTimeout(Cache* c, uint32_t polls, cudaStream_t stream)
 {
-    std::lock_guard<std::mutex> hold(c->work);
     waitTimeoutKernel<<<1, 128, 0, stream>>>(polls, c->error);
     NRC_OK(cudaGetLastError());
     finish(c, stream);
@@ -910,13 +885,12 @@ void query(Cache* c, const float* queries, uint32_t count, float* out, cudaStrea
 float train(Cache* c, const float* queries, const float* targets, uint32_t count, uint32_t steps, cudaStream_t stream)
 {
     if (count == 0 || steps == 0) return 0.0f;
-    std::lock_guard<std::mutex> hold(c->work);
     const uint32_t gridCount = static_cast<uint32_t>(c->gridCount);
     const uint32_t gridBlocks = std::min((gridCount / 4u + kAdamThreads - 1u) / kAdamThreads, static_cast<uint32_t>(c->sms) * 16u);
     float lossValue = 0.0f;
     for (uint32_t s = 0; s < steps; ++s) {
         NRC_OK(cudaMemsetAsync(c->loss, 0, sizeof(float), stream));
-        runTrainKernels(c, queries, targets, count, stream);
+        runTrainKernel(c, queries, targets, count, stream);
         ++c->step;
         const float b1 = 1.0f - std::pow(c->config.beta1, float(c->step));
         const float b2 = 1.0f - std::pow(c->config.beta2, float(c->step));
@@ -932,11 +906,10 @@ float train(Cache* c, const float* queries, const float* targets, uint32_t count
 void gradients(Cache* c, const float* queries, const float* targets, uint32_t count, float* mlpGrad, float* gridGrad,
                cudaStream_t stream)
 {
-    std::lock_guard<std::mutex> hold(c->work);
     NRC_OK(cudaMemsetAsync(c->mlpGrad, 0, kWeightCount * sizeof(float), stream));
     NRC_OK(cudaMemsetAsync(c->gridGrad, 0, c->gridCount * sizeof(float), stream));
     NRC_OK(cudaMemsetAsync(c->loss, 0, sizeof(float), stream));
-    if (count > 0) runTrainKernels(c, queries, targets, count, stream);
+    if (count > 0) runTrainKernel(c, queries, targets, count, stream);
     finish(c, stream);
     if (mlpGrad) NRC_OK(cudaMemcpy(mlpGrad, c->mlpGrad, kWeightCount * sizeof(float), cudaMemcpyDeviceToHost));
     if (gridGrad) NRC_OK(cudaMemcpy(gridGrad, c->gridGrad, c->gridCount * sizeof(float), cudaMemcpyDeviceToHost));
