@@ -742,10 +742,10 @@ void launchShadeReplays(const ShadeVariant& v, const ShadeLaunch& l)
     else shadeFullReplaysUnlit(v.cache, l);
 }
 
-void renderFrame(const DeviceScene& sceneIn, const FrameConst& frame, PathBuffers& paths, FrameBuffers& fb,
+void renderFrame(const DeviceScene& scene, const FrameConst& frame, const PathBuffers& buffers, FrameBuffers& fb,
                  cudaStream_t stream, StageTimes* timing, bool countTraversal, uint64_t* launches, CacheRun* cacheRun)
 {
-    const DeviceScene& scene = sceneIn;
+    PathBuffers paths = buffers;  // what this call's launches get: its counters move from bounce to bounce
     const bool cacheMode = cacheRun != nullptr && cacheRun->cache != nullptr && paths.cache.enabled != 0u;
     if (!cacheMode) paths.cache.enabled = 0u;
     uint64_t launched = 0;

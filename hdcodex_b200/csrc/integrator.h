@@ -123,10 +123,12 @@ struct StageTimes {
     uint32_t extendLaunches = 0;
 };
 
-// Renders sampleCount samples per pixel into fb (running mean update).
+// Renders sampleCount samples per pixel into fb (running mean update). The
+// caller's `buffers` stay as they are, so that a call whose work did not run
+// (a batch graph that could not be captured) can be made again.
 // `timing` non-null records per-stage device times with CUDA events.
 // countTraversal selects the traversal kernels that count node visits and
-// triangle tests (into paths.stats[3..6]); *launches gets the kernel count.
+// triangle tests (into buffers.stats[3..6]); *launches gets the kernel count.
 namespace nrc {
 struct Cache;
 }
@@ -139,7 +141,7 @@ struct CacheRun {
     uint64_t queries = 0, samples = 0;
 };
 
-void renderFrame(const DeviceScene& scene, const FrameConst& frame, PathBuffers& paths, FrameBuffers& fb,
+void renderFrame(const DeviceScene& scene, const FrameConst& frame, const PathBuffers& buffers, FrameBuffers& fb,
                  cudaStream_t stream, StageTimes* timing, bool countTraversal, uint64_t* launches,
                  CacheRun* cacheRun = nullptr);
 
