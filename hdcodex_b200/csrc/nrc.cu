@@ -344,8 +344,13 @@ __device__ __forceinline__ bool groupSyncOr(uint32_t group, bool value)
     return any != 0u;
 }
 
-__global__ void __launch_bounds__(kQueryThreads, 2) queryKernel(DeviceParams p, const float* queries, const __nv_bfloat16* features,
-                                                                uint32_t count, float* out, uint32_t* error)
+// kEncoded: `features` holds the encoded records. Otherwise they are encoded
+// here (a query that finds the workspace taken by another): the gathers need
+// the registers of one block per SM, and take 870 us per 10^6 queries where
+// both kernels take 376 us; the same bits.
+template <bool kEncoded>
+__global__ void __launch_bounds__(kQueryThreads, kEncoded ? 2 : 1)
+    queryKernel(DeviceParams p, const float* queries, const __nv_bfloat16* features, uint32_t count, float* out, uint32_t* error)
 {
     extern __shared__ __align__(16) uint8_t smem[];
     __nv_bfloat16* w = reinterpret_cast<__nv_bfloat16*>(smem);
@@ -369,8 +374,13 @@ __global__ void __launch_bounds__(kQueryThreads, 2) queryKernel(DeviceParams p, 
     for (uint32_t base = (blockIdx.x * kQueryGroups + group) * kTile; base < count && !failed; base += gridDim.x * kQueryGroups * kTile) {
         const uint32_t q = base + row;
         float v[kWidth];
-        storeInputRow(x, row, features + static_cast<size_t>(q) * kGridFeatures,
-                      q < count ? queries + static_cast<size_t>(q) * kQueryFloats : nullptr);
+        const float* record = q < count ? queries + static_cast<size_t>(q) * kQueryFloats : nullptr;
+        if constexpr (kEncoded) {
+            storeInputRow(x, row, features + static_cast<size_t>(q) * kGridFeatures, record);
+        } else {
+            encodeQuery(p, record, v);
+            storeRow(x, row, v, 8u, kWidth);
+        }
         for (int layer = 0; layer < kLayers; ++layer) {
             fenceProxyAsync();
             fenceBeforeSync();
@@ -705,8 +715,9 @@ struct Cache {
     __half* gridHalf = nullptr;
     float* loss = nullptr;      // the loss sum, and after it the error word: one copy reads both
     uint32_t* error = nullptr;  // loss + 1
-    // Encoded features of one chunk of records. Queries on one cache share
-    // them: each holds `work` until its kernels have finished.
+    // Encoded features of one chunk of records, and who uses them: a query
+    // holds `work` until its kernels have finished. One that finds it held (by
+    // another thread, on another stream) does without, so queries still overlap.
     std::mutex work;
     __nv_bfloat16* features = nullptr;
     uint32_t chunk = 0;         // records `features` holds
@@ -798,7 +809,8 @@ Cache* create(int device, const Config& config)
             if (c->chunk <= kTile) throw;
         }
     }
-    NRC_OK(cudaFuncSetAttribute(queryKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kQuerySmem));
+    NRC_OK(cudaFuncSetAttribute(queryKernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kQuerySmem));
+    NRC_OK(cudaFuncSetAttribute(queryKernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kQuerySmem));
     NRC_OK(cudaFuncSetAttribute(trainKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTrainSmem));
     // Initialisation: weights uniform in +-sqrt(6 / (fan_in + fan_out)), table uniform in +-1e-4.
     std::mt19937 rng(config.seed);
@@ -869,14 +881,21 @@ uint32_t resolution(const Cache* c, int level) { return c->resolution[level]; }
 void query(Cache* c, const float* queries, uint32_t count, float* out, cudaStream_t stream)
 {
     if (count == 0) return;
-    std::lock_guard<std::mutex> hold(c->work);
+    constexpr uint32_t kBlockQueries = kQueryGroups * kTile;
+    std::unique_lock<std::mutex> hold(c->work, std::try_to_lock);
+    if (!hold.owns_lock()) {
+        const int blocks = static_cast<int>(std::min<uint32_t>((count + kBlockQueries - 1) / kBlockQueries, static_cast<uint32_t>(c->sms)));
+        queryKernel<false><<<blocks, kQueryThreads, kQuerySmem, stream>>>(c->params(), queries, nullptr, count, out, c->error);
+        NRC_OK(cudaGetLastError());
+        finish(c, stream);
+        return;
+    }
     for (uint32_t begin = 0; begin < count; begin += c->chunk) {
         const uint32_t n = std::min(c->chunk, count - begin);
         const float* records = queries + static_cast<size_t>(begin) * kQueryFloats;
         encodeKernel<<<encodeGrid(n), 256, 0, stream>>>(c->params(), records, n, c->features);
-        const uint32_t tiles = kQueryGroups * kTile;  // per block
-        const int blocks = static_cast<int>(std::min<uint32_t>((n + tiles - 1) / tiles, static_cast<uint32_t>(c->sms) * 2u));
-        queryKernel<<<blocks, kQueryThreads, kQuerySmem, stream>>>(c->params(), records, c->features, n, out + begin, c->error);
+        const int blocks = static_cast<int>(std::min<uint32_t>((n + kBlockQueries - 1) / kBlockQueries, static_cast<uint32_t>(c->sms) * 2u));
+        queryKernel<true><<<blocks, kQueryThreads, kQuerySmem, stream>>>(c->params(), records, c->features, n, out + begin, c->error);
         NRC_OK(cudaGetLastError());
     }
     finish(c, stream);
