@@ -196,6 +196,7 @@ __device__ __forceinline__ void levelCorners(const DeviceParams& p, int level, f
 // Same products and sums in the same order as corner by corner.
 constexpr int kEncodeLevels = 4;       // levels per thread
 constexpr uint32_t kGridFeatures = kLevels * kFeatures;
+constexpr uint32_t kQueryChunk = 1u << 20;  // records encoded at a time
 
 __device__ __forceinline__ float2 entryOf(const uint4& four, uint32_t index)
 {
@@ -345,9 +346,9 @@ __device__ __forceinline__ bool groupSyncOr(uint32_t group, bool value)
 }
 
 // kEncoded: `features` holds the encoded records. Otherwise they are encoded
-// here (a query that finds the workspace taken by another): the gathers need
-// the registers of one block per SM, and take 870 us per 10^6 queries where
-// both kernels take 376 us; the same bits.
+// here (a query that finds the workspace taken by another, or none): the gathers need
+// the registers of one block per SM, and 10^6 queries take 565 us where the
+// two kernels take 379 us; the same bits.
 template <bool kEncoded>
 __global__ void __launch_bounds__(kQueryThreads, kEncoded ? 2 : 1)
     queryKernel(DeviceParams p, const float* queries, const __nv_bfloat16* features, uint32_t count, float* out, uint32_t* error)
@@ -719,8 +720,7 @@ struct Cache {
     // holds `work` until its kernels have finished. One that finds it held (by
     // another thread, on another stream) does without, so queries still overlap.
     std::mutex work;
-    __nv_bfloat16* features = nullptr;
-    uint32_t chunk = 0;         // records `features` holds
+    __nv_bfloat16* features = nullptr;  // null: no query has it
     uint64_t step = 0;
     int sms = 148;
 
@@ -798,16 +798,12 @@ Cache* create(int device, const Config& config)
     c->gridHalf = deviceAlloc<__half>(c->gridCount);
     c->loss = deviceAlloc<float>(2);
     c->error = reinterpret_cast<uint32_t*>(c->loss + 1);
-    // Chunks of 2^20 records to encode (64 MB of features, which stay in L2
-    // between the kernels; chunks of 2^18 cost 0.14 ms of launch gaps in a
-    // query of 10^6), fewer where memory is short.
-    for (c->chunk = 1u << 20;; c->chunk >>= 1) {
-        try {
-            c->features = deviceAlloc<__nv_bfloat16>(static_cast<size_t>(c->chunk) * kGridFeatures);
-            break;
-        } catch (const std::exception&) {
-            if (c->chunk <= kTile) throw;
-        }
+    // A chunk of 2^20 records to encode: 64 MB of features, which stay in L2
+    // between the kernels (chunks of 2^18 cost 0.14 ms of launch gaps in a
+    // query of 10^6). Where memory is short the cache does without.
+    try {
+        c->features = deviceAlloc<__nv_bfloat16>(static_cast<size_t>(kQueryChunk) * kGridFeatures);
+    } catch (const OutOfDeviceMemory&) {
     }
     NRC_OK(cudaFuncSetAttribute(queryKernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kQuerySmem));
     NRC_OK(cudaFuncSetAttribute(queryKernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kQuerySmem));
@@ -883,15 +879,16 @@ void query(Cache* c, const float* queries, uint32_t count, float* out, cudaStrea
     if (count == 0) return;
     constexpr uint32_t kBlockQueries = kQueryGroups * kTile;
     std::unique_lock<std::mutex> hold(c->work, std::try_to_lock);
-    if (!hold.owns_lock()) {
+    if (!hold.owns_lock() || c->features == nullptr) {
+        hold = {};
         const int blocks = static_cast<int>(std::min<uint32_t>((count + kBlockQueries - 1) / kBlockQueries, static_cast<uint32_t>(c->sms)));
         queryKernel<false><<<blocks, kQueryThreads, kQuerySmem, stream>>>(c->params(), queries, nullptr, count, out, c->error);
         NRC_OK(cudaGetLastError());
         finish(c, stream);
         return;
     }
-    for (uint32_t begin = 0; begin < count; begin += c->chunk) {
-        const uint32_t n = std::min(c->chunk, count - begin);
+    for (uint32_t begin = 0; begin < count; begin += kQueryChunk) {
+        const uint32_t n = std::min(kQueryChunk, count - begin);
         const float* records = queries + static_cast<size_t>(begin) * kQueryFloats;
         encodeKernel<<<encodeGrid(n), 256, 0, stream>>>(c->params(), records, n, c->features);
         const int blocks = static_cast<int>(std::min<uint32_t>((n + kBlockQueries - 1) / kBlockQueries, static_cast<uint32_t>(c->sms) * 2u));

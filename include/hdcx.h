@@ -714,6 +714,10 @@ HDCX_API hdcx_status hdcx_autotune(hdcx_tracer* tracer, const hdcx_camera* camer
  * normalised to [0, 1]), direction (3), shading normal (3), roughness,
  * (wavelength - 380) / 400, 0. Query, target and output pointers of the
  * query/train/gradient calls are device memory.
+ * Device memory: 18 bytes per table parameter and 64 MB for the encoded
+ * records of a query, which one query at a time uses. Queries that run beside
+ * it (threads on other streams) and those of a cache for which the 64 MB were
+ * not to be had take half as long again; their results are the same.
  * ------------------------------------------------------------------------- */
 #define HDCX_NRC_QUERY_FLOATS 12u
 #define HDCX_NRC_WEIGHT_COUNT 17408u /* 4 x 64 x 64 + 16 x 64 FP32 weights, row-major [out][in] per layer */
