@@ -618,8 +618,8 @@ __global__ void waitTimeoutKernel(uint32_t limit, uint32_t* error)
 // Adam on the FP32 parameters of the table and the network in one launch (the
 // network's 17,408 weights in the last blocks); refreshes the FP16 table and
 // the BF16 tiled weights and clears the gradients. Bound by memory: 34 bytes
-// per parameter, four parameters a thread. A parameter without gradient and
-// moments stays as it is and is only read (its step is exactly zero).
+// per parameter, four parameters a thread. Parameters without gradient and
+// moments are only read where that leaves them as they are (AdamStep::restsAtZero).
 struct AdamArrays {
     float* params;
     float* grad;
@@ -628,13 +628,15 @@ struct AdamArrays {
 };
 struct AdamStep {
     float lr, beta1, beta2, epsilon, correction1, correction2;
+    bool restsAtZero;  // zero gradient and moments give zero moments and a step of +0
 };
 
-__device__ __forceinline__ float adamUpdate(const AdamStep& a, float g, float& m, float& v, float param)
+// Updates the moments and returns the step.
+__host__ __device__ __forceinline__ float adamStep(const AdamStep& a, float g, float& m, float& v)
 {
     m = a.beta1 * m + (1.0f - a.beta1) * g;
     v = a.beta2 * v + (1.0f - a.beta2) * g * g;
-    return param - a.lr * (m / a.correction1) / (sqrtf(v / a.correction2) + a.epsilon);
+    return a.lr * (m / a.correction1) / (sqrtf(v / a.correction2) + a.epsilon);
 }
 
 constexpr uint32_t kAdamThreads = 256;
@@ -652,14 +654,14 @@ __global__ void __launch_bounds__(kAdamThreads) adamKernel(AdamArrays grid, uint
     for (uint32_t i = ((network ? blockIdx.x - gridBlocks : blockIdx.x) * kAdamThreads + threadIdx.x) * 4u; i < n; i += stride) {
         const float4 g = *reinterpret_cast<const float4*>(a.grad + i);
         float4 m = *reinterpret_cast<const float4*>(a.m + i), v = *reinterpret_cast<const float4*>(a.v + i);
-        const bool idle = step.epsilon > 0.0f && g.x == 0.0f && g.y == 0.0f && g.z == 0.0f && g.w == 0.0f && m.x == 0.0f && m.y == 0.0f && m.z == 0.0f &&
+        const bool idle = step.restsAtZero && g.x == 0.0f && g.y == 0.0f && g.z == 0.0f && g.w == 0.0f && m.x == 0.0f && m.y == 0.0f && m.z == 0.0f &&
                           m.w == 0.0f && v.x == 0.0f && v.y == 0.0f && v.z == 0.0f && v.w == 0.0f;
         if (idle) continue;
         float4 param = *reinterpret_cast<const float4*>(a.params + i);
-        param.x = adamUpdate(step, g.x, m.x, v.x, param.x);
-        param.y = adamUpdate(step, g.y, m.y, v.y, param.y);
-        param.z = adamUpdate(step, g.z, m.z, v.z, param.z);
-        param.w = adamUpdate(step, g.w, m.w, v.w, param.w);
+        param.x -= adamStep(step, g.x, m.x, v.x);
+        param.y -= adamStep(step, g.y, m.y, v.y);
+        param.z -= adamStep(step, g.z, m.z, v.z);
+        param.w -= adamStep(step, g.w, m.w, v.w);
         *reinterpret_cast<float4*>(a.m + i) = m;
         *reinterpret_cast<float4*>(a.v + i) = v;
         *reinterpret_cast<float4*>(a.params + i) = param;
@@ -910,9 +912,14 @@ float train(Cache* c, const float* queries, const float* targets, uint32_t count
         ++c->step;
         const float b1 = 1.0f - std::pow(c->config.beta1, float(c->step));
         const float b2 = 1.0f - std::pow(c->config.beta2, float(c->step));
+        // (Not so with a decay of one, a rate that is not finite or no epsilon: those give NaN.)
+        AdamStep step{c->config.learningRate, c->config.beta1, c->config.beta2, c->config.epsilon, b1, b2, false};
+        float m = 0.0f, v = 0.0f;
+        const float rest = adamStep(step, 0.0f, m, v);
+        step.restsAtZero = m == 0.0f && v == 0.0f && rest == 0.0f && !std::signbit(rest);
         adamKernel<<<gridBlocks + kAdamMlpBlocks, kAdamThreads, 0, stream>>>(
-            AdamArrays{c->grid, c->gridGrad, c->gridM, c->gridV}, gridCount, AdamArrays{c->mlp, c->mlpGrad, c->mlpM, c->mlpV},
-            AdamStep{c->config.learningRate, c->config.beta1, c->config.beta2, c->config.epsilon, b1, b2}, c->mlpTiled, c->gridHalf);
+            AdamArrays{c->grid, c->gridGrad, c->gridM, c->gridV}, gridCount, AdamArrays{c->mlp, c->mlpGrad, c->mlpM, c->mlpV}, step,
+            c->mlpTiled, c->gridHalf);
         NRC_OK(cudaGetLastError());
     }
     finish(c, stream, &lossValue);
