@@ -101,8 +101,21 @@ struct PathStore {
         b->allocate(count * sizeof(T));
         return b->as<T>();
     }
-    // Replaces the buffers by buffers of `n` paths; the GPU must be done with the old ones.
+    // Replaces the buffers by buffers of `n` paths; the GPU must be done with
+    // the old ones. Where one of them is not to be had the store is empty: a
+    // capacity stands only for buffers that are all there.
     void allocate(uint64_t n, uint32_t shadowPerPath)
+    {
+        try {
+            allocateAll(n, shadowPerPath);
+        } catch (...) {
+            release();
+            throw;
+        }
+    }
+
+private:
+    void allocateAll(uint64_t n, uint32_t shadowPerPath)
     {
         release();
         if (!hostStats &&
