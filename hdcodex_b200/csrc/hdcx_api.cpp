@@ -832,6 +832,7 @@ void ensureOutput(hdcx_tracer* t, uint32_t w, uint32_t h)
     // zero-filled accumulation buffer.
     check(cudaStreamSynchronize(t->stream), "cudaStreamSynchronize");
     const size_t pixels = size_t(w) * h;
+    t->fb = FrameBuffers{};  // set once all of its buffers are there
     t->rgba.allocate(pixels * sizeof(float4));
     t->xyz.allocate(pixels * 3u * sizeof(double));
     t->batch.allocate(pixels * sizeof(float4));
@@ -1500,6 +1501,7 @@ void enqueueAovs(hdcx_tracer* t, const FrameConst& frame)
     const size_t pixels = size_t(frame.width) * frame.height;
     if (t->aovWidth != frame.width || t->aovHeight != frame.height || !t->aovIds.ptr) {
         check(cudaStreamSynchronize(t->stream), "cudaStreamSynchronize");
+        t->aovWidth = t->aovHeight = 0;  // set once both buffers are there
         t->aovIds.allocate(pixels * sizeof(uint32_t));
         t->aovDepth.allocate(pixels * sizeof(float));
         t->aovWidth = frame.width;
