@@ -29,6 +29,7 @@
 #include "nvtx_range.h"
 #include "render_static.h"
 #include "scene_pack.h"
+#include "wave_plan.h"
 
 namespace {
 
@@ -849,24 +850,16 @@ void ensureOutput(hdcx_tracer* t, uint32_t w, uint32_t h)
 }
 
 constexpr uint64_t kAutomaticWavePaths = 12ull << 20;  // ~12.6M paths per wave
-// Device bytes of path state per path (PathBuffers with three shadow slots
-// and the deferred subsurface-walk records).
-constexpr uint64_t kPathStateBytes = 140 + 48 + 8 + 3 * 52;
-
-// Smallest wave an automatic wave is shrunk to when device memory is short.
-constexpr uint64_t kMinimumAutomaticWave = 1ull << 16;
 
 // Sizes the wave of a render of `needed` paths on `store` and grows the store
 // to it; returns the wave. The wave is the tracer's own wave size if it set
 // one, else min(needed, `capOverride` or the automatic wave). A wave the
-// tracer did not set is also bounded by device memory: its path state takes
-// at most three quarters of what is free plus what the store already holds
-// (the wave size does not change the image). Buffers larger than the wave are
+// tracer did not set is also bounded by device memory (boundedWave; the wave
+// size does not change the image). Buffers larger than the wave are
 // kept, but the wave is this call's, since it decides the launch shape.
 // `fixed`: the store is not grown; the wave is bounded by its capacity.
 uint64_t ensureStore(hdcx_tracer* t, PathStore& store, uint64_t needed, uint64_t capOverride, bool fixed)
 {
-    constexpr uint32_t kShadowSlots = 3;
     const uint64_t cap = t->wavePaths ? t->wavePaths : (capOverride ? capOverride : kAutomaticWavePaths);
     uint64_t capacity = std::max<uint64_t>(3, std::min(needed, cap));
     if (fixed) return std::min(capacity, store.paths.capacity);
@@ -875,10 +868,7 @@ uint64_t ensureStore(hdcx_tracer* t, PathStore& store, uint64_t needed, uint64_t
     if (t->wavePaths == 0 && (store.paths.capacity < capacity || store.paths.shadowPerPath < kShadowSlots)) {
         size_t freeBytes = 0, totalBytes = 0;
         check(cudaMemGetInfo(&freeBytes, &totalBytes), "cudaMemGetInfo");
-        const uint64_t held = store.paths.capacity * (143ull + 56ull * store.paths.shadowPerPath);
-        uint64_t fit = (static_cast<uint64_t>(freeBytes) + held) / 4 * 3 / (143ull + 56ull * kShadowSlots);
-        if (store.paths.shadowPerPath >= kShadowSlots) fit = std::max(fit, store.paths.capacity);  // held buffers serve as is
-        capacity = std::min(capacity, std::max(fit, std::min(capacity, kMinimumAutomaticWave)));
+        capacity = boundedWave(capacity, freeBytes, store.paths.capacity);
     }
     if (store.paths.capacity < capacity || store.paths.shadowPerPath < kShadowSlots) {
         check(cudaStreamSynchronize(t->stream), "cudaStreamSynchronize");
