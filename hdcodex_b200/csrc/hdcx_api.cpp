@@ -2450,14 +2450,12 @@ HDCX_API hdcx_status hdcx_set_tuning(hdcx_tracer* t, const hdcx_tuning* in)
 
 namespace {
 
+// The workload shape of a tuning, with everything that decides which kernels a
+// render launches: merged or separate shading of parted lanes, walks, two levels.
 struct TuningKey {
     int device;
-    uint32_t triangles, width, height, samples, bounces, full, lit, opaque;
-    bool operator==(const TuningKey& o) const
-    {
-        return device == o.device && triangles == o.triangles && width == o.width && height == o.height &&
-               samples == o.samples && bounces == o.bounces && full == o.full && lit == o.lit && opaque == o.opaque;
-    }
+    uint32_t triangles, width, height, samples, bounces, full, lit, opaque, partsLanes, subsurface, instanced;
+    bool operator==(const TuningKey&) const = default;
 };
 
 std::mutex gTuningLock;
@@ -2476,7 +2474,8 @@ HDCX_API hdcx_status hdcx_autotune(hdcx_tracer* t, const hdcx_camera* camera, ui
     NvtxRange range("hdcx autotune");
     const TuningKey key{t->device, t->scene.primitiveCount, width, height, std::max(sampleCount, 1u),
                         std::clamp(maxBounces, 1u, HDCX_MAX_PATH_BOUNCES), t->scene.fullShading,
-                        (t->scene.lightCount > 0u && !t->scene.hasMeshLights) ? 1u : 0u, t->scene.opaque};
+                        (t->scene.lightCount > 0u && !t->scene.hasMeshLights) ? 1u : 0u, t->scene.opaque,
+                        t->scene.partsLanes, t->scene.hasSubsurface, t->scene.instances ? 1u : 0u};
     {
         std::lock_guard<std::mutex> lock(gTuningLock);
         for (const auto& entry : gTunings) {

@@ -697,7 +697,7 @@ HDCX_API hdcx_status hdcx_set_tuning(hdcx_tracer* tracer, const hdcx_tuning* tun
  * ones while their path state (about 352 bytes per path) fits half of the free
  * device memory; a path arena grown for a candidate larger than the one kept
  * is released before it returns. Results are cached per device and workload shape
- * (triangles, pixels, samples, bounces, shading variant) for the process, so
+ * (triangles, pixels, samples, bounces, kernel variants) for the process, so
  * a repeated call times nothing. The tuning renders overwrite the tracer's
  * accumulation: render with sample_index 0 afterwards. */
 HDCX_API hdcx_status hdcx_autotune(hdcx_tracer* tracer, const hdcx_camera* camera, uint32_t width, uint32_t height,
