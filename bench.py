@@ -85,6 +85,8 @@ def parse():
                          "not timed)")
     ap.add_argument("--profile", action="store_true",
                     help="render exactly one frame and exit (for ncu launch lists and captures)")
+    ap.add_argument("--stage-times", action="store_true",
+                    help="with --profile: trace extension and shadow rays in launches of their own, as the timed steps do")
     ap.add_argument("--width", type=int, default=0, help="override the workload width (profiling only)")
     ap.add_argument("--height", type=int, default=0, help="override the workload height (profiling only)")
     ap.add_argument("--spp", type=int, default=0, help="override the workload spp (profiling only)")
@@ -720,6 +722,7 @@ def run_hdcx(args):
     elif args.autotune and not args.profile:
         tuning = tracer.autotune(wl.camera, wl.width, wl.height, wl.max_bounces, wl.spp)
     if args.profile:
+        tracer.set_profiling(PROFILE_STAGE_TIMES if args.stage_times else 0)
         tracer.render_device(wl.camera, wl.width, wl.height, 0, wl.max_bounces, wl.spp)
         print(json.dumps({"profile_frame": wl.name, "width": wl.width, "height": wl.height, "spp": wl.spp,
                           "stats": tracer.stats()}), flush=True)
@@ -795,8 +798,9 @@ def run_hdcx(args):
         "kernel": "traceKernel (closest-hit traversal)",
         "bound": "hbm", "achieved": achieved_gbs, "peak": peak, "unit": "GB/s",
         "frac": (achieved_gbs / peak) if achieved_gbs else None, "peak_source": peak_kind,
-        # ncu DRAM bytes per extension ray (profiles/extend_kernel_traffic_heavy.json,
-        # captured on a smaller frame) times this run's rays per launch.
+        # ncu DRAM bytes per extension ray of the extension launches alone
+        # (profiles/extend_kernel_traffic_heavy.json, captured on a smaller
+        # frame) times this run's rays per launch.
         "traffic": (traffic["dram_bytes_per_ray"] * ext_rays / extend_launches
                     if traffic and extend_launches else None),
         "algorithmic_bytes_per_ray": bytes_per_ray, "nodes_per_ray": nodes_per_ray,
