@@ -430,10 +430,13 @@ __global__ void __launch_bounds__(kQueryThreads, kEncoded ? 2 : 1)
 // their own: the barriers of a tile order a block's additions (a tile's before
 // those of the block's next), and with them the FP32 rounding of an entry's
 // sum. Adam divides by the gradient's own size, so a parameter whose gradient
-// nearly cancels moves by up to a learning rate with that rounding. With the
-// scatter in a kernel whose warps run on freely, four steps of 2^16 records
-// gave single parameters a third of a learning rate away (1.4e-5 of the table
-// in relative L2, where this order repeats itself to 2.5e-7).
+// nearly cancels moves by up to a learning rate with that rounding. Blocks
+// still race, so two runs differ (four steps of 2^16 records: one pair of runs
+// in ten by more than 8e-4 of an entry), but with the scatter in a kernel whose
+// warps run on freely single parameters came out where this order does not put
+// them, a third of a learning rate away. A step of 2^16 records takes 0.23 ms
+// (0.14 to 0.16 in kernels of their own), waiting on gathers and atomics with
+// four warps per SM.
 constexpr uint32_t kTrainSmem = kWeightCount * 2u + 5u * kTile * kWidth * 2u + kTile * 128u * 2u + 16u;
 
 __global__ void __launch_bounds__(128) trainKernel(DeviceParams p, const float* queries, const float* targets, uint32_t count,
