@@ -73,6 +73,8 @@ HDCX_D uint32_t maskGreater(float a, float b) { return a > b ? 1u : 0u; }
 HDCX_D uint32_t maskGreater(Lanes3 a, Lanes3 b) { return (a.x > b.x ? 1u : 0u) | (a.y > b.y ? 2u : 0u) | (a.z > b.z ? 4u : 0u); }
 HDCX_D uint32_t maskLess(float a, float b) { return a < b ? 1u : 0u; }
 HDCX_D uint32_t maskLess(Lanes3 a, Lanes3 b) { return maskGreater(b, a); }
+HDCX_D bool allZero(float v) { return v == 0.0f; }
+HDCX_D bool allZero(Lanes3 v) { return v.x == 0.0f && v.y == 0.0f && v.z == 0.0f; }
 HDCX_D float whereMask(uint32_t m, float a, float b) { return (m & 1u) ? a : b; }
 HDCX_D Lanes3 whereMask(uint32_t m, Lanes3 a, Lanes3 b)
 {

@@ -606,8 +606,11 @@ HDCX_D V evaluateDirectSurface(const ShadingFrame& f, const LobeTerms& t, float3
     const V diffuseResponse = mix(reflection, V(wrappedNdotL / kPi), p.subsurface);
     const V diffuse = V(diffuseScale) * (V(1.0f) - baseFresnel) * V(p.diffuseWeight) * V(1.0f - p.translucentWeight) *
                       V(1.0f - p.metalness) * p.diffuseColor * diffuseResponse * V(1.0f - p.transmission);
-    V translucent = V(0.0f);  // a zero weight multiplies finite terms
-    if (p.translucentWeight != 0.0f || !(fabsf(diffuseScale) < INFINITY)) {
+    // A zero weight leaves zero of finite terms. (weightedReflectance has made a
+    // finite colour zero then; one that is not finite may be NaN. The others are
+    // in the diffuse term too.)
+    V translucent = V(0.0f);
+    if (p.translucentWeight != 0.0f || !(fabsf(diffuseScale) < INFINITY) || !allZero(p.translucentColor)) {
         const V viewFresnel = fresnelSchlick(f.nDotV, p.f0);
         translucent = V(diffuseScale) * (V(1.0f) - viewFresnel) * V(p.translucentWeight) * V(1.0f - p.metalness) *
                       p.translucentColor * V(backNdotL / kPi) * V(1.0f - p.transmission);
