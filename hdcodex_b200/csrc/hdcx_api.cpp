@@ -444,6 +444,12 @@ bool needsFullShading(const PackedSceneData& d)
             if (!std::isfinite(v)) return true;
         }
     }
+    // So is a light's diffuse factor.
+    for (uint32_t l = 0; l < d.lightCount && (size_t(l) + 1) * sizeof(GpuLight) <= d.lights.size(); ++l) {
+        GpuLight light;
+        std::memcpy(&light, d.lights.data() + size_t(l) * sizeof(GpuLight), sizeof light);
+        if (!std::isfinite(light.controls.x)) return true;
+    }
     return false;
 }
 

@@ -6,6 +6,7 @@ import pytest
 
 import ref_scenes as R
 from hdcodex_b200 import PathTracer
+from hdcodex_b200.scene import DOME
 from test_gpu_path_groups import check
 
 pytestmark = pytest.mark.gpu
@@ -36,3 +37,15 @@ def test_translucent_colour_without_weight(oracle_lib, color, mesh_light, lights
     for m in s.materials:
         m.translucent_weight, m.translucent_color = 0.0, color
     compare(oracle_lib, s, f"translucent colour {color}")
+
+
+@pytest.mark.parametrize("factor", [INF, -INF, NAN])
+@pytest.mark.parametrize("kind", [1, 2], ids=["analytic", "with dome"])
+def test_diffuse_factor_of_a_light(oracle_lib, factor, kind):
+    """Materials without layered lobes: the specialised closure, if all is finite."""
+    s = R.mesh_light_scene(0.0)
+    s.lights = R.analytic_lights()[:2]
+    if kind == 2:
+        s.lights.append(s.lights[0].copy(id="/dome", type=DOME, color=[0.3, 0.4, 0.5], texture=""))
+    s.lights[1].diffuse = factor
+    compare(oracle_lib, s, f"diffuse factor {factor}")
